@@ -1,5 +1,6 @@
 // api.cu -- the C ABI of include/inductioneq.h: contexts, the name-dispatched reference
 // kernels, the fused/graph-captured time stepping, device-resident CG cleaning and norms.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -9,6 +10,7 @@
 
 #include "ieq_host.h"
 #include "misc_kernels.cuh"
+#include "cg.cuh"
 #include "stage_brick.cuh"
 #include "stage_z.cuh"
 #include "diag.cuh"
@@ -849,7 +851,8 @@ ieq_status ieq_create(ieq_ctx **out, const char *settings, const char *const *pa
   if (st == IEQ_OK) cuda(cudaMemset(c->d_counter, 0, 64 * sizeof(unsigned)), "cudaMemset");
   if (st == IEQ_OK) cuda(cudaMalloc(&c->d_flag, 64 * sizeof(int)), "cudaMalloc");
   if (st == IEQ_OK) cuda(cudaMemset(c->d_flag, 0, 64 * sizeof(int)), "cudaMemset");
-  if (st == IEQ_OK) cuda(cudaMalloc(&c->d_cg, sizeof(CgState)), "cudaMalloc");
+  if (st == IEQ_OK) cuda(cudaMalloc(&c->d_cg, sizeof(CgDevice)), "cudaMalloc");
+  if (st == IEQ_OK) cuda(cudaMemset(c->d_cg, 0, sizeof(CgDevice)), "cudaMemset");
   if (st == IEQ_OK) cuda(cudaEventCreate(&c->ev0), "cudaEventCreate");
   if (st == IEQ_OK) cuda(cudaEventCreate(&c->ev1), "cudaEventCreate");
   if (st == IEQ_OK) {

@@ -143,7 +143,8 @@ struct ieq_ctx {
   double *d_total = nullptr;       // reduction totals
   unsigned *d_counter = nullptr;   // last-block tickets
   int *d_flag = nullptr;
-  void *d_cg = nullptr;            // CgState
+  void *d_cg = nullptr;            // CgDevice (the CG loop's state)
+  int cg_resident = 0;             // resident blocks of the CG loop kernel (0: not asked yet)
   double *d_cg_vec = nullptr;      // FP64 CG vectors: div, phi, r, u, u', lap (6 x n_pad)
   double *d_cg_hist = nullptr;
   double *d_lap_s = nullptr;       // the CG Laplacian's rows divided by DX^2, DY^2, DZ^2

@@ -362,6 +362,9 @@ __global__ void k_axpy_interior(Mesh m, int off, int gx, int gy, int gz, S *x, c
   x[idx] = xpay ? x[idx] + av * y[idx] : av * x[idx] + y[idx];
 }
 
+// tile of x-y columns of one block of the CG loop (cg.cuh)
+constexpr int kCgTX = 32, kCgTY = 8;
+
 // ---- device-resident CG loop (matlab/+induction_eq/clean_div.m:47-73).  The scalars live
 // in CgState; every kernel returns at once when `done` is set, so a fixed-length chunk of
 // iterations can be replayed from a CUDA graph and stops exactly where the host loop would.
@@ -430,8 +433,9 @@ struct LapFastArgs {
   double Li[3][W];
   const double *Ls;   // [3][2nb+1][W]
 };
-// ---- the two passes of one CG iteration inside a graph loop (a conditional WHILE node
-// whose condition the last block of pass B sets; no host round trip per iteration).
+// ---- IEQ_CG_PASS_A=1: the two passes of one CG iteration as kernels of their own inside a
+// graph loop (a conditional WHILE node whose condition the last block of pass B sets; no host
+// round trip per iteration).  The default is the one-launch loop of cg.cuh.
 //
 // Pass A (clean_div.m:50-56): the search direction u = beta*u + r (calc_axpy) is formed at
 // every stencil point as it is loaded -- u and r are read, the new direction is written at the
@@ -508,110 +512,6 @@ __global__ void __launch_bounds__(256) k_cg_pass_a(const LapArgs<double> a, cons
     const int np = gridDim.x * gridDim.y * gridDim.z;
     const double ul = block_sum_partials(a.partials, np);
     if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
-      cs->alpha = cs->rr / ul;
-      *counter = 0u;
-    }
-  }
-}
-
-// Pass A as a 2.5D kernel: a CTA of kCgTX x kCgTY threads owns a tile of x-y columns of the
-// CG interior and marches through a chunk of z planes.  Every thread keeps the direction
-// values of its column at planes z - C0 .. z + C0 in a register queue (the z terms), and the
-// plane z of the tile with its x and y halos (C0 deep) sits in shared memory (the x and y
-// terms), so each direction value is formed (__fma_rn(beta, u, r)) and loaded from global
-// memory about once per node instead of once per stencil point.  Values outside the grid are
-// 0 (their coefficient is 0, where the reference reads the node itself); periodic grids wrap.
-// The terms are summed in the order of laplace_dir_at: per row entry c, ((val + x) + y) + z.
-constexpr int kCgTX = 32, kCgTY = 8;
-
-// the direction value at global node (x, y, z): 0 outside the grid (non-periodic)
-__device__ __forceinline__ double cg_dir_at(const LapArgs<double> &a, const double *uo, const double *r, double beta,
-                                            int x, int y, int z) {
-  const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
-  if (a.periodic) {
-    x += x < 0 ? nx : 0; x -= x >= nx ? nx : 0;
-    y += y < 0 ? ny : 0; y -= y >= ny ? ny : 0;
-    z += z < 0 ? nz : 0; z -= z >= nz ? nz : 0;
-  } else if (x < 0 || x >= nx || y < 0 || y >= ny || z < 0 || z >= nz) {
-    return 0.0;
-  }
-  const long long j = x + (long long)nx * (y + (long long)ny * z);
-  return __fma_rn(beta, __ldg(uo + j), __ldg(r + j));
-}
-
-template <int W>
-__global__ void __launch_bounds__(kCgTX * kCgTY) k_cg_pass_a_z(const LapArgs<double> a, const LapFastArgs<W> f,
-                                                                const double *r, double *u0, double *u1, CgState *cs,
-                                                                unsigned *counter, int tz) {
-  if (cs->done) return;   // (host-driven iterations past convergence)
-  constexpr int C0 = (W - 1) / 2;
-  constexpr int SX = kCgTX + 2 * C0, SY = kCgTY + 2 * C0;
-  __shared__ double pl[SY][SX];
-  const int it = cs->it;
-  const double *uo = (it & 1) ? u1 : u0;
-  double *un = (it & 1) ? u0 : u1;
-  const double beta = cs->rr / cs->old;
-  const int tx = threadIdx.x % kCgTX, ty = threadIdx.x / kCgTX;
-  const int x0 = a.off + blockIdx.x * kCgTX, y0 = a.off + blockIdx.y * kCgTY;
-  const int zb = a.off + blockIdx.z * tz;
-  const int ze = min(zb + tz, a.off + a.gz);
-  const int ix = x0 + tx, iy = y0 + ty;
-  const bool mine = ix < a.off + a.gx && iy < a.off + a.gy;
-  const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
-  const int rows = 2 * a.nb + 1;
-  const int rx = a.periodic ? a.nb : sbp_row(ix, nx, a.nb);
-  const int ry = a.periodic ? a.nb : sbp_row(iy, ny, a.nb);
-  const double *lx = f.Ls + ((long long)0 * rows + rx) * W;
-  const double *ly = f.Ls + ((long long)1 * rows + ry) * W;
-  double q[W];
-#pragma unroll
-  for (int k = 0; k < W - 1; ++k) q[k + 1] = mine ? cg_dir_at(a, uo, r, beta, ix, iy, zb - C0 + k) : 0.0;
-  double prod = 0.0;
-  for (int z = zb; z < ze; ++z) {
-#pragma unroll
-    for (int k = 0; k < W - 1; ++k) q[k] = q[k + 1];
-    q[W - 1] = mine ? cg_dir_at(a, uo, r, beta, ix, iy, z + C0) : 0.0;
-    // the tile of plane z (own column: the queue centre) and its x / y halos
-    // (a thread past the interior holds the value of its own grid position: 0 on a box, the
-    // wrapped value on a periodic grid)
-    pl[ty + C0][tx + C0] = mine ? q[C0] : cg_dir_at(a, uo, r, beta, ix, iy, z);
-    for (int h = threadIdx.x; h < 2 * C0 * kCgTY + 2 * C0 * kCgTX; h += kCgTX * kCgTY) {
-      int px, py;
-      if (h < 2 * C0 * kCgTY) {   // x halo: C0 columns on each side of every tile row
-        const int side = h / (C0 * kCgTY), rem = h % (C0 * kCgTY);
-        py = C0 + rem / C0;
-        px = side ? kCgTX + C0 + rem % C0 : rem % C0;
-      } else {                     // y halo: C0 rows above and below the tile's columns
-        const int g = h - 2 * C0 * kCgTY;
-        const int side = g / (C0 * kCgTX), rem = g % (C0 * kCgTX);
-        px = C0 + rem % kCgTX;
-        py = side ? kCgTY + C0 + rem / kCgTX : rem / kCgTX;
-      }
-      pl[py][px] = cg_dir_at(a, uo, r, beta, x0 - C0 + px, y0 - C0 + py, z);
-    }
-    __syncthreads();
-    if (mine) {
-      const int rz = a.periodic ? a.nb : sbp_row(z, nz, a.nb);
-      const double *lz = f.Ls + ((long long)2 * rows + rz) * W;
-      double val = 0.0;
-#pragma unroll
-      for (int c = 0; c < W; ++c) {
-        const double t0 = pl[ty + C0][tx + c] * lx[c];
-        const double t1 = pl[ty + c][tx + C0] * ly[c];
-        const double t2 = q[c] * lz[c];
-        val = ((val + t0) + t1) + t2;
-      }
-      const long long idx = ix + (long long)nx * (iy + (long long)ny * z);
-      un[idx] = q[C0];
-      a.out[idx] = val;
-      prod += q[C0] * val;
-    }
-    __syncthreads();
-  }
-  if (block_partial_and_ticket(prod, a.partials, counter)) {
-    const int np = gridDim.x * gridDim.y * gridDim.z;
-    const double ul = block_sum_partials(a.partials, np);
-    if (threadIdx.x == 0) {
       cs->alpha = cs->rr / ul;
       *counter = 0u;
     }
