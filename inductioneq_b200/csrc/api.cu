@@ -113,6 +113,28 @@ ieq_status upload_tables(ieq_ctx *c) {
         t.H[r][s + i + WH - 1] += term;
       }
   }
+  // the same rows as lists of their non-zero entries
+  const int c0 = (op.sw - 1) / 2, reach = std::max(c0, WH - 1);
+  for (int r = 0; r < rows; ++r) {
+    int nd = 0, nu = 0;
+    for (int o = -reach; o <= reach; ++o) {
+      const R cD = o >= -c0 && o <= c0 ? t.D[r][o + c0] : (R)0;
+      const R cH = o >= -(WH - 1) && o <= WH - 1 ? t.H[r][o + WH - 1] : (R)0;
+      // row r < nb is that of node r, row r > nb that of the node 2 nb - r from the end
+      const bool outside = (r < op.nb && r + o < 0) || (r > op.nb && o > 2 * op.nb - r);
+      if (cD != (R)0) {
+        if (nd == MAX_ND) return fail(c, IEQ_ERR_SETTINGS, "derivative row with too many entries");
+        t.nd[r][nd] = cD;
+        t.nd_off[r][nd++] = outside ? 0 : o;
+      }
+      if (cD != (R)0 || cH != (R)0) {
+        if (nu == MAX_NU) return fail(c, IEQ_ERR_SETTINGS, "dissipation row with too many entries");
+        t.ud[r][nu] = cD;
+        t.uh[r][nu] = cH;
+        t.ud_off[r][nu++] = outside ? 0 : o;
+      }
+    }
+  }
   IEQ_CUDA(c, cudaMalloc(&c->d_tables, sizeof(Tables<R>)));
   IEQ_CUDA(c, cudaMemcpy(c->d_tables, &t, sizeof(t), cudaMemcpyHostToDevice));
   // flat D / Dadj rows for the generic operators, in R and FP64

@@ -56,18 +56,22 @@ __device__ __forceinline__ void st3(R4<R> *p, V3<R> v) {
 // Operator ids: 0..2 classical order 2/4/6, 3..5 extended order 2/4/6.
 // NB = boundary rows per side, SW = derivative stencil width, WH = width of the
 // dissipation factor D_HO, RI = interior radius (ORDER/2) of both D and D_HO^T D_HO.
+// ND = most non-zero entries of a derivative row, NU = of a derivative and dissipation row
+// together; QX = reach of a pair's derivative rows along x, in pairs, boundary rows included.
 template <int OP>
 struct Op;
-template <> struct Op<0> { static constexpr int NB = 1, SW = 3, WH = 2, RI = 1, ORDER = 2; };
-template <> struct Op<1> { static constexpr int NB = 4, SW = 7, WH = 3, RI = 2, ORDER = 4; };
-template <> struct Op<2> { static constexpr int NB = 6, SW = 11, WH = 4, RI = 3, ORDER = 6; };
-template <> struct Op<3> { static constexpr int NB = 3, SW = 5, WH = 2, RI = 1, ORDER = 2; };
-template <> struct Op<4> { static constexpr int NB = 6, SW = 11, WH = 3, RI = 2, ORDER = 4; };
-template <> struct Op<5> { static constexpr int NB = 8, SW = 15, WH = 4, RI = 3, ORDER = 6; };
+template <> struct Op<0> { static constexpr int NB = 1, SW = 3, WH = 2, RI = 1, ORDER = 2, ND = 2, NU = 3, QX = 1; };
+template <> struct Op<1> { static constexpr int NB = 4, SW = 7, WH = 3, RI = 2, ORDER = 4, ND = 4, NU = 6, QX = 1; };
+template <> struct Op<2> { static constexpr int NB = 6, SW = 11, WH = 4, RI = 3, ORDER = 6, ND = 8, NU = 9, QX = 2; };
+template <> struct Op<3> { static constexpr int NB = 3, SW = 5, WH = 2, RI = 1, ORDER = 2, ND = 3, NU = 4, QX = 1; };
+template <> struct Op<4> { static constexpr int NB = 6, SW = 11, WH = 3, RI = 2, ORDER = 4, ND = 7, NU = 8, QX = 2; };
+template <> struct Op<5> { static constexpr int NB = 8, SW = 15, WH = 4, RI = 3, ORDER = 6, ND = 10, NU = 11, QX = 3; };
 
 constexpr int MAX_ROWS = 17;   // 2*NB+1 of the widest operator (6th extended)
 constexpr int MAX_SW = 15;
 constexpr int MAX_HW = 7;      // 2*WH-1
+constexpr int MAX_ND = 10;     // non-zero entries of a derivative row ...
+constexpr int MAX_NU = 11;     // ... and of a derivative and dissipation row together
 constexpr int MAX_LROWS = 23;  // Laplacian rows (6th extended, wide stencil)
 constexpr int MAX_LW = 21;
 
@@ -79,7 +83,21 @@ struct Tables {
   R H[MAX_ROWS][MAX_HW];        // dissipation rows sum_s,i M^-1 D_HO[r][s] D_HO[c][i] (-1)^(p/2+1)
   R DHO[MAX_ROWS][4];           // raw D_HO rows (first-order/adaptive dissipation)
   R Minv[MAX_ROWS];
+  // the rows as lists of their non-zero entries in ascending order (padded with zeros): a
+  // 4th-order boundary row has at most the 4 entries of the interior row, spread over 7
+  // columns.  An offset that leaves the box is 0 (the node itself, include/utils.h:142-168).
+  R nd[MAX_ROWS][MAX_ND];       // derivative rows
+  R ud[MAX_ROWS][MAX_NU];       // entries of the derivative or the dissipation row: D ...
+  R uh[MAX_ROWS][MAX_NU];       // ... and H
+  int nd_off[MAX_ROWS][MAX_ND];
+  int ud_off[MAX_ROWS][MAX_NU];
 };
+
+// whether every active lane of the warp sits on the interior row
+__device__ __forceinline__ bool warp_on_row(int row, int nb) {
+  const unsigned m = __activemask();
+  return __all_sync(m, row == nb) != 0;
+}
 
 // Laplacian rows for divergence cleaning in the CG precision S.
 template <typename S>
@@ -134,10 +152,14 @@ __device__ __forceinline__ void coords(const Mesh &m, int ix, int iy, int iz, R 
   z = (R)m.xmin[2] + (R)gz * (R)m.d[2];
 }
 
+__device__ __forceinline__ void sincos_any(double t, double *s, double *c) { sincos(t, s, c); }
+__device__ __forceinline__ void sincos_any(float t, float *s, float *c) { sincosf(t, s, c); }
+
 // include/rotation_2D.h:7-25
 template <typename R>
 __device__ V3<R> tc_rotation_2d_b(R x, R y, R t) {
-  R s = sin(t), c = cos(t);
+  R s, c;
+  sincos_any(t, &s, &c);
   R xx = c * x + s * y, yy = -s * x + c * y;
   R fac = exp((R)-20 * ((xx - (R)0.5) * (xx - (R)0.5) + yy * yy));
   R bx0 = (R)-4 * yy * fac, by0 = ((R)4 * xx - (R)2) * fac;
@@ -148,7 +170,8 @@ __device__ V3<R> tc_rotation_2d_b(R x, R y, R t) {
 template <typename R>
 __device__ V3<R> tc_rotation_3d_b(R x, R y, R z, R t) {
   const R sqrt3 = (R)1.7320508075688772;
-  R s = sin(t), c = cos(t);
+  R s, c;
+  sincos_any(t, &s, &c);
   R xx = ((1 + 2 * c) * x + (1 - c + sqrt3 * s) * y + (1 - c - sqrt3 * s) * z) / (R)3.0;
   R yy = ((1 - c - sqrt3 * s) * x + (1 + 2 * c) * y + (1 - c + sqrt3 * s) * z) / (R)3.0;
   R zz = ((1 - c + sqrt3 * s) * x + (1 - c - sqrt3 * s) * y + (1 + 2 * c) * z) / (R)3.0;
@@ -219,7 +242,8 @@ __device__ V3<R> tc_rotation_gaussian_b(R x, R y, R t, R om) {
   const R w2 = (R)0.01;
   const R amp = (R)(0.1 * 1.6487212707001282 / 1.4142135623730951);
   R th = om * t;
-  R s = sin(th), c = cos(th);
+  R s, c;
+  sincos_any(th, &s, &c);
   R xr = c * x + s * y - (R)0.5, yr = -s * x + c * y;
   R g = amp * exp(-(xr * xr + yr * yr) / w2);
   R b0x = -(R)2 * yr / w2 * g, b0y = (R)2 * xr / w2 * g;

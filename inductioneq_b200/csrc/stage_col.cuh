@@ -28,8 +28,10 @@ namespace ieq {
 #ifndef IEQ_COL_MIN_BLOCKS
 #define IEQ_COL_MIN_BLOCKS 8
 #endif
+// (convection: rotation 97^3, 6th order, run-time mask, its boundary rows unrolled: 8 blocks
+// spilled 400 bytes and took 3.02 ms for 30 stages, 6 blocks of <= 80 registers 2.52, 5 2.57)
 #ifndef IEQ_COL_CONV_MIN_BLOCKS
-#define IEQ_COL_CONV_MIN_BLOCKS 8
+#define IEQ_COL_CONV_MIN_BLOCKS 6
 #endif
 #ifndef IEQ_CURL_NODES
 #define IEQ_CURL_NODES 1
@@ -132,13 +134,13 @@ __device__ __forceinline__ void col_acc(ColSums<R> &s, int ax, int need, R cD, R
 }
 
 template <typename R, bool HALL, bool HOD, int CONV, typename F = SoA<R>>
-__device__ __forceinline__ void col_load(const StageArgs<R, F> &a, int ax, long long j, V3<R> &B, V3<R> &U,
+__device__ __forceinline__ void col_load(const StageArgs<R, F> &a, int ax, int j, V3<R> &B, V3<R> &U,
                                          R &e1, R &e2) {
   if (CONV || HOD) B = ldf(a.bk, j);
   if (CONV) U = ldf(a.u, j);
   if (HALL) {
-    e1 = __ldg(a.E.p + j + e_comp1(ax) * a.E.s);
-    e2 = __ldg(a.E.p + j + e_comp2(ax) * a.E.s);
+    e1 = __ldg(a.E.p + e_comp1(ax) * a.E.s + j);
+    e2 = __ldg(a.E.p + e_comp2(ax) * a.E.s + j);
   }
 }
 
@@ -148,14 +150,13 @@ __device__ __forceinline__ void col_load(const StageArgs<R, F> &a, int ax, long 
 template <typename R, int OP, bool PER, bool HALL, bool HOD, int CONV, typename F = SoA<R>, int NEED = -1,
           bool FOF = false>
 __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a, int ax, int i, int n,
-                                         long long idx, long long st, const V3<R> &Bm,
+                                         int idx, int st, const V3<R> &Bm,
                                          const V3<R> *Um = nullptr) {
   const int need = NEED >= 0 ? NEED : a.need;
-  constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, WH = Op<OP>::WH, RI = Op<OP>::RI;
-  constexpr int RB = (C0 > WH - 1) ? C0 : WH - 1;
+  constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
   const V3<R> zero = {0, 0, 0};
   const int row = PER ? NB : sbp_row(i, n, NB);
-  if (row == NB) {
+  if (PER || warp_on_row(row, NB)) {
     const bool wrap = PER && (i < RI || i >= n - RI);
 #pragma unroll
     for (int o = -RI; o <= RI; ++o) {
@@ -164,7 +165,7 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
         if (HOD) col_acc<R, false, HOD, 0>(s, ax, 0, (R)0, a.Hint[RI], false, true, Bm, zero, (R)0, (R)0);
         continue;
       }
-      const long long j = wrap ? idx + (long long)(nbr<true>(i, o, n) - i) * st : idx + (long long)o * st;
+      const int j = wrap ? idx + (nbr<true>(i, o, n) - i) * st : idx + o * st;
       V3<R> B = zero, U = zero;
       R e1 = 0, e2 = 0;
       col_load<R, HALL, HOD, CONV, F>(a, ax, j, B, U, e1, e2);
@@ -172,38 +173,46 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
       if (FOF) fo_acc(s, a.Dint[o + RI], B, U, Bm, *Um);
     }
   } else {
-    for (int o = -RB; o <= RB; ++o) {
-      const R cD = (o >= -C0 && o <= C0) ? a.tab->D[row][o + C0] : (R)0;
-      const R cH = (HOD && o >= -(WH - 1) && o <= WH - 1) ? a.tab->H[row][o + WH - 1] : (R)0;
-      if (cD == (R)0 && cH == (R)0) continue;
-      const long long j = idx + (long long)(nbr<PER>(i, o, n) - i) * st;
+    // boundary rows, and every row of a warp that holds one: the row's non-zero entries, all
+    // loads free to issue before the first sum (as a run-time loop over the columns with a
+    // test per column the loads came one at a time).  Padding entries load nothing, add zeros
+    constexpr int NT = HOD ? Op<OP>::NU : Op<OP>::ND;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const R cD = HOD ? __ldg(&a.tab->ud[row][t]) : __ldg(&a.tab->nd[row][t]);
+      const R cH = HOD ? __ldg(&a.tab->uh[row][t]) : (R)0;
+      const int o = HOD ? __ldg(&a.tab->ud_off[row][t]) : __ldg(&a.tab->nd_off[row][t]);
       V3<R> B = zero, U = zero;
       R e1 = 0, e2 = 0;
-      col_load<R, HALL, HOD, CONV, F>(a, ax, j, B, U, e1, e2);
-      col_acc<R, HALL, HOD, CONV>(s, ax, need, cD, cH, cD != (R)0, cH != (R)0, B, U, e1, e2);
+      if (cD != (R)0 || (HOD && cH != (R)0)) col_load<R, HALL, HOD, CONV, F>(a, ax, idx + o * st, B, U, e1, e2);
+      col_acc<R, HALL, HOD, CONV>(s, ax, need, cD, cH, !HOD || cD != (R)0, cH != (R)0, B, U, e1, e2);
       if (FOF) fo_acc(s, cD, B, U, Bm, *Um);
     }
   }
 }
 
-// add one axis' sums into DB (volume and Hall terms) and the dissipation sum
-template <typename R, bool HALL, bool HOD, int CONV, typename F = SoA<R>>
+// add one axis' sums into DB (volume and Hall terms) and the dissipation sum; with the mask at
+// compile time the terms of the sums that are not formed (their weights are zero) drop out
+template <typename R, bool HALL, bool HOD, int CONV, typename F = SoA<R>, int NEED = -1>
 __device__ __forceinline__ void col_combine(const StageArgs<R, F> &a, int ax, const ColSums<R> &s,
                                             const V3<R> &Bm, const V3<R> &um, V3<R> &db, V3<R> &hod) {
   if (CONV) {
     const R Ba = cmp(Bm, ax), Ua = cmp(um, ax);
     const R SBa = cmp(s.SB, ax), SUa = cmp(s.SU, ax);
     const R *w = a.w;
-    V3<R> vol;
-    vol.x = w[0] * s.SuiBa.x + w[1] * Ba * s.SU.x + w[2] * um.x * SBa -
-            (w[3] * s.SuaB.x + w[4] * Ua * s.SB.x + w[5] * Bm.x * SUa);
-    vol.y = w[0] * s.SuiBa.y + w[1] * Ba * s.SU.y + w[2] * um.y * SBa -
-            (w[3] * s.SuaB.y + w[4] * Ua * s.SB.y + w[5] * Bm.y * SUa);
-    vol.z = w[0] * s.SuiBa.z + w[1] * Ba * s.SU.z + w[2] * um.z * SBa -
-            (w[3] * s.SuaB.z + w[4] * Ua * s.SB.z + w[5] * Bm.z * SUa);
-    db.x += a.two_inv_d[ax] * vol.x;
-    db.y += a.two_inv_d[ax] * vol.y;
-    db.z += a.two_inv_d[ax] * vol.z;
+    auto term = [&](R SuiBa, R SU, R SB, R SuaB, R B, R U) -> R {
+      R p = 0, m = 0;
+      if (NEED & 1) p = w[0] * SuiBa;
+      if (NEED & 2) p = p + w[1] * Ba * SU;
+      if (NEED & 4) p = p + w[2] * U * SBa;
+      if (NEED & 8) m = w[3] * SuaB;
+      if (NEED & 4) m = m + w[4] * Ua * SB;
+      if (NEED & 2) m = m + w[5] * B * SUa;
+      return p - m;
+    };
+    db.x += a.two_inv_d[ax] * term(s.SuiBa.x, s.SU.x, s.SB.x, s.SuaB.x, Bm.x, um.x);
+    db.y += a.two_inv_d[ax] * term(s.SuiBa.y, s.SU.y, s.SB.y, s.SuaB.y, Bm.y, um.y);
+    db.z += a.two_inv_d[ax] * term(s.SuiBa.z, s.SU.z, s.SB.z, s.SuaB.z, Bm.z, um.z);
   }
   if (HALL) {
     const R f1 = a.inv_d[ax] * s.h1, f2 = a.inv_d[ax] * s.h2;
@@ -237,8 +246,8 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
   const int iz0 = (blockIdx.z * blockDim.z + threadIdx.z) * NZ;
   if (ix < nx && iy < ny && iz0 < nz) {
     const int cnt = nz - iz0 < NZ ? nz - iz0 : NZ;
-    const long long sz = (long long)nx * ny;
-    const long long base = ix + (long long)nx * iy;
+    const int sz = nx * ny;
+    const int base = ix + nx * iy;
     const V3<R> zero = {0, 0, 0};
     V3<R> Bm[NZ], um[NZ], db[NZ], hod[NZ];
 #pragma unroll
@@ -248,7 +257,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
       Bm[k] = zero;
       um[k] = zero;
       if (k < cnt) {
-        const long long idx = base + (long long)(iz0 + k) * sz;
+        const int idx = base + (iz0 + k) * sz;
         Bm[k] = ldf(a.bk, idx);
         if (CONV) um[k] = ldf(a.u, idx);
       }
@@ -257,7 +266,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
 #pragma unroll
     for (int k = 0; k < NZ; ++k) {
       if (k < cnt) {
-        const long long idx = base + (long long)(iz0 + k) * sz;
+        const int idx = base + (iz0 + k) * sz;
 #pragma unroll
         for (int ax = 0; ax < 2; ++ax) {
           ColSums<R> s{};
@@ -280,15 +289,15 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
           zz += zz < 0 ? nz : 0;
           zz -= zz >= nz ? nz : 0;
         }
-        const long long j = base + (long long)zz * sz;
+        const int j = base + zz * sz;
         V3<R> B = zero, U = zero;
         R e1 = 0, e2 = 0;
         if (p >= 0 && p < NZ) {
           B = Bm[p];
           U = um[p];
           if (HALL) {
-            e1 = __ldg(a.E.p + j + e_comp1(2) * a.E.s);
-            e2 = __ldg(a.E.p + j + e_comp2(2) * a.E.s);
+            e1 = __ldg(a.E.p + e_comp1(2) * a.E.s + j);
+            e2 = __ldg(a.E.p + e_comp2(2) * a.E.s + j);
           }
         } else {
           col_load<R, HALL, HOD, CONV>(a, 2, j, B, U, e1, e2);
@@ -310,7 +319,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
 #pragma unroll
       for (int k = 0; k < NZ; ++k) {
         if (k < cnt) {
-          const long long idx = base + (long long)(iz0 + k) * sz;
+          const int idx = base + (iz0 + k) * sz;
           ColSums<R> s{};
           col_axis<R, OP, PER, HALL, HOD, CONV, SoA<R>, NEED>(s, a, 2, iz0 + k, nz, idx, sz, Bm[k]);
           col_combine<R, HALL, HOD, CONV>(a, 2, s, Bm[k], um[k], db[k], hod[k]);
@@ -322,7 +331,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
       if (k < cnt) {
         const int ii[3] = {ix, iy, iz0 + k};
         const int nn[3] = {nx, ny, nz};
-        const long long idx = base + (long long)(iz0 + k) * sz;
+        const int idx = base + (iz0 + k) * sz;
         V3<R> d = db[k];
         if (!PER) stage_sat<R, SoA<R>, HALL>(a, ii, nn, idx, Bm[k], um[k], CONV, d);
         if (HOD_) {
@@ -332,7 +341,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
           d.z += a.hod_factor * hv.z;
         }
         if (FOAD) {
-          const long long st[3] = {1, nx, sz};
+          const int st[3] = {1, nx, sz};
           const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, PER>(a, ii, nn, st, idx, Bm[k], um[k]);
           d.x += ds.x; d.y += ds.y; d.z += ds.z;
         }
@@ -343,10 +352,75 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
   stage_time_post(a);
 }
 
+// one axis of the curl at one node: the derivatives v1, v2 of the two components of B
+// orthogonal to the axis and, with HODS, the dissipation-row sum ho of all three (interior
+// row, periodic wrap or SBP boundary rows; each sum term by term in stencil order)
+template <typename R, int OP, bool PER, bool HODS>
+__device__ __forceinline__ void curl_axis_node(const CurlArgs<R, SoA<R>> &a, int ax, int i, int n, int idx,
+                                               int st, const V3<R> &Bm, R &v1, R &v2, V3<R> &ho) {
+  constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
+  const int c1 = (ax + 1) % 3, c2 = (ax + 2) % 3;
+  v1 = 0;
+  v2 = 0;
+  ho = {0, 0, 0};
+  const int row = PER ? NB : sbp_row(i, n, NB);
+  if (PER || warp_on_row(row, NB)) {
+    const bool wrap = PER && (i < RI || i >= n - RI);
+#pragma unroll
+    for (int o = -RI; o <= RI; ++o) {
+      const R cH = a.Hint[o + RI];
+      if (o == 0) {
+        if (HODS) {
+          ho.x += cH * Bm.x; ho.y += cH * Bm.y; ho.z += cH * Bm.z;
+        }
+        continue;
+      }
+      const int j = wrap ? idx + (nbr<true>(i, o, n) - i) * st : idx + o * st;
+      const R c = a.Dint[o + RI];
+      if (HODS) {
+        const V3<R> B = ldf(a.b, j);
+        v1 += c * cmp(B, c1);
+        v2 += c * cmp(B, c2);
+        ho.x += cH * B.x; ho.y += cH * B.y; ho.z += cH * B.z;
+      } else {
+        v1 += c * __ldg(a.b.p + c1 * a.b.s + j);
+        v2 += c * __ldg(a.b.p + c2 * a.b.s + j);
+      }
+    }
+  } else {
+    constexpr int NT = HODS ? Op<OP>::NU : Op<OP>::ND;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const R cD = HODS ? __ldg(&a.tab->ud[row][t]) : __ldg(&a.tab->nd[row][t]);
+      const R cH = HODS ? __ldg(&a.tab->uh[row][t]) : (R)0;
+      const int j = idx + (HODS ? __ldg(&a.tab->ud_off[row][t]) : __ldg(&a.tab->nd_off[row][t])) * st;
+      if (HODS) {
+        V3<R> B = {0, 0, 0};
+        if (cD != (R)0 || cH != (R)0) B = ldf(a.b, j);
+        if (cD != (R)0) {
+          v1 += cD * cmp(B, c1);
+          v2 += cD * cmp(B, c2);
+        }
+        if (cH != (R)0) {
+          ho.x += cH * B.x; ho.y += cH * B.y; ho.z += cH * B.z;
+        }
+      } else {
+        R p1 = 0, p2 = 0;
+        if (cD != (R)0) {
+          p1 = __ldg(a.b.p + c1 * a.b.s + j);
+          p2 = __ldg(a.b.p + c2 * a.b.s + j);
+        }
+        v1 += cD * p1;
+        v2 += cD * p2;
+      }
+    }
+  }
+}
+
 // J = curl(B)/rho and E = J x B, two nodes per thread along z (see the file comment)
 template <typename R, int OP, bool PER>
 __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ CurlArgs<R, SoA<R>> a) {
-  constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, RI = Op<OP>::RI;
+  constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
   pdl_enter();
   constexpr int NZ = kCurlNodes;
   const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
@@ -355,41 +429,20 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ 
   const int iz0 = (blockIdx.z * blockDim.z + threadIdx.z) * NZ;
   if (ix >= nx || iy >= ny || iz0 >= nz) return;
   const int cnt = nz - iz0 < NZ ? nz - iz0 : NZ;
-  const long long sz = (long long)nx * ny;
-  const long long base = ix + (long long)nx * iy;
+  const int sz = nx * ny;
+  const int base = ix + nx * iy;
   const int nn[3] = {nx, ny, nz};
-  const long long st[3] = {1, nx, sz};
+  const int st[3] = {1, nx, sz};
   R g[NZ][3][3];   // g[node][axis][component]
   // one axis at one node: the derivatives of the two components orthogonal to it
-  auto axis = [&](int ax, int i, long long idx, R &v1, R &v2) {
-    const int c1 = (ax + 1) % 3, c2 = (ax + 2) % 3;
-    v1 = 0;
-    v2 = 0;
-    const int row = PER ? NB : sbp_row(i, nn[ax], NB);
-    if (row == NB) {
-      const bool wrap = PER && (i < RI || i >= nn[ax] - RI);
-#pragma unroll
-      for (int o = -RI; o <= RI; ++o) {
-        if (o == 0) continue;
-        const R c = a.Dint[o + RI];
-        const long long j = wrap ? idx + (long long)(nbr<true>(i, o, nn[ax]) - i) * st[ax] : idx + (long long)o * st[ax];
-        v1 += c * __ldg(a.b.p + j + c1 * a.b.s);
-        v2 += c * __ldg(a.b.p + j + c2 * a.b.s);
-      }
-    } else {
-      for (int o = -C0; o <= C0; ++o) {
-        const R c = a.tab->D[row][o + C0];
-        if (c == (R)0) continue;
-        const long long j = idx + (long long)(nbr<PER>(i, o, nn[ax]) - i) * st[ax];
-        v1 += c * __ldg(a.b.p + j + c1 * a.b.s);
-        v2 += c * __ldg(a.b.p + j + c2 * a.b.s);
-      }
-    }
+  auto axis = [&](int ax, int i, int idx, R &v1, R &v2) {
+    V3<R> ho;
+    curl_axis_node<R, OP, PER, false>(a, ax, i, nn[ax], idx, st[ax], V3<R>{0, 0, 0}, v1, v2, ho);
   };
 #pragma unroll
   for (int k = 0; k < NZ; ++k) {
     if (k < cnt) {
-      const long long idx = base + (long long)(iz0 + k) * sz;
+      const int idx = base + (iz0 + k) * sz;
 #pragma unroll
       for (int ax = 0; ax < 2; ++ax) {
         R v1, v2;
@@ -416,7 +469,7 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ 
         zz += zz < 0 ? nz : 0;
         zz -= zz >= nz ? nz : 0;
       }
-      const long long j = base + (long long)zz * sz;
+      const int j = base + zz * sz;
       const R bx = __ldg(a.b.p + j), by = __ldg(a.b.p + j + a.b.s);
 #pragma unroll
       for (int k = 0; k < NZ; ++k) {
@@ -436,7 +489,7 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ 
     for (int k = 0; k < NZ; ++k) {
       if (k < cnt) {
         R v1, v2;
-        axis(2, iz0 + k, base + (long long)(iz0 + k) * sz, v1, v2);
+        axis(2, iz0 + k, base + (iz0 + k) * sz, v1, v2);
         g[k][2][0] = v1 * a.inv_d[2];
         g[k][2][1] = v2 * a.inv_d[2];
       }
@@ -446,7 +499,7 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ 
   for (int k = 0; k < NZ; ++k) {
     if (k < cnt) {
       const int iz = iz0 + k;
-      const long long idx = base + (long long)iz * sz;
+      const int idx = base + iz * sz;
       V3<R> J = {g[k][1][2] - g[k][2][1], g[k][2][0] - g[k][0][2], g[k][0][1] - g[k][1][0]};
       if (a.rho) {
         const R r = (R)1 / a.rho[idx];
@@ -456,65 +509,6 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ 
       stf(a.out, idx, V3<R>{J.x * B.y - J.y * B.x, J.x * B.z - J.z * B.x, J.y * B.z - J.z * B.y});
       if (!PER && (ix == 0 || iy == 0 || iz == 0 || ix == nx - 1 || iy == ny - 1 || iz == nz - 1))
         stf(a.jface, idx, J);
-    }
-  }
-}
-
-// one axis of the curl at one node: the derivatives v1, v2 of the two components of B
-// orthogonal to the axis and, with HODS, the dissipation-row sum ho of all three (interior
-// row, periodic wrap or SBP boundary rows; each sum term by term in stencil order)
-template <typename R, int OP, bool PER, bool HODS>
-__device__ __forceinline__ void curl_axis_node(const CurlArgs<R, SoA<R>> &a, int ax, int i, int n, long long idx,
-                                               long long st, const V3<R> &Bm, R &v1, R &v2, V3<R> &ho) {
-  constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, WH = Op<OP>::WH, RI = Op<OP>::RI;
-  constexpr int RB = HODS ? ((C0 > WH - 1) ? C0 : WH - 1) : C0;
-  const int c1 = (ax + 1) % 3, c2 = (ax + 2) % 3;
-  v1 = 0;
-  v2 = 0;
-  ho = {0, 0, 0};
-  const int row = PER ? NB : sbp_row(i, n, NB);
-  if (row == NB) {
-    const bool wrap = PER && (i < RI || i >= n - RI);
-#pragma unroll
-    for (int o = -RI; o <= RI; ++o) {
-      const R cH = a.Hint[o + RI];
-      if (o == 0) {
-        if (HODS) {
-          ho.x += cH * Bm.x; ho.y += cH * Bm.y; ho.z += cH * Bm.z;
-        }
-        continue;
-      }
-      const long long j = wrap ? idx + (long long)(nbr<true>(i, o, n) - i) * st : idx + (long long)o * st;
-      const R c = a.Dint[o + RI];
-      if (HODS) {
-        const V3<R> B = ldf(a.b, j);
-        v1 += c * cmp(B, c1);
-        v2 += c * cmp(B, c2);
-        ho.x += cH * B.x; ho.y += cH * B.y; ho.z += cH * B.z;
-      } else {
-        v1 += c * __ldg(a.b.p + j + c1 * a.b.s);
-        v2 += c * __ldg(a.b.p + j + c2 * a.b.s);
-      }
-    }
-  } else {
-    for (int o = -RB; o <= RB; ++o) {
-      const R cD = (o >= -C0 && o <= C0) ? a.tab->D[row][o + C0] : (R)0;
-      const R cH = (HODS && o >= -(WH - 1) && o <= WH - 1) ? a.tab->H[row][o + WH - 1] : (R)0;
-      if (cD == (R)0 && cH == (R)0) continue;
-      const long long j = idx + (long long)(nbr<PER>(i, o, n) - i) * st;
-      if (HODS) {
-        const V3<R> B = ldf(a.b, j);
-        if (cD != (R)0) {
-          v1 += cD * cmp(B, c1);
-          v2 += cD * cmp(B, c2);
-        }
-        if (cH != (R)0) {
-          ho.x += cH * B.x; ho.y += cH * B.y; ho.z += cH * B.z;
-        }
-      } else {
-        v1 += cD * __ldg(a.b.p + j + c1 * a.b.s);
-        v2 += cD * __ldg(a.b.p + j + c2 * a.b.s);
-      }
     }
   }
 }
@@ -538,10 +532,10 @@ __global__ void __launch_bounds__(kColThreads, IEQ_CURL_MIN_BLOCKS * 128 / kColT
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= nx || iy >= ny || iz >= nz) return;
-  const long long idx = ix + (long long)nx * (iy + (long long)ny * iz);
+  const int idx = ix + nx * (iy + ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {nx, ny, nz};
-  const long long st[3] = {1, nx, (long long)nx * ny};
+  const int st[3] = {1, nx, nx * ny};
   const V3<R> Bm = ldf(a.b, idx);
   R g[3][3];
   V3<R> hod = {0, 0, 0};

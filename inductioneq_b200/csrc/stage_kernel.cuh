@@ -64,23 +64,25 @@ __device__ __forceinline__ void stf(const SoAcg<R> &f, long long j, V3<R> v) {
   f.p[j + f.s] = v.y;
   f.p[j + 2 * f.s] = v.z;
 }
+// (offsets of the fused path's nodes are 32-bit: a state of 2^31 nodes does not fit 180 GB; the
+// component bases are uniform, so a load's address is one multiply-add)
 template <typename R>
-__device__ __forceinline__ V3<R> ldf(const SoA<R> &f, long long j) {
-  return {__ldg(f.p + j), __ldg(f.p + j + f.s), __ldg(f.p + j + 2 * f.s)};
+__device__ __forceinline__ V3<R> ldf(const SoA<R> &f, int j) {
+  return {__ldg(f.p + j), __ldg(f.p + f.s + j), __ldg(f.p + 2 * f.s + j)};
 }
 template <typename R>
 __device__ __forceinline__ V3<R> ldf_plain(const AoS<R> &f, long long j) { return ld3_plain(f.p + j); }
 template <typename R>
-__device__ __forceinline__ V3<R> ldf_plain(const SoA<R> &f, long long j) {
-  return {f.p[j], f.p[j + f.s], f.p[j + 2 * f.s]};
+__device__ __forceinline__ V3<R> ldf_plain(const SoA<R> &f, int j) {
+  return {f.p[j], (f.p + f.s)[j], (f.p + 2 * f.s)[j]};
 }
 template <typename R>
 __device__ __forceinline__ void stf(const AoS<R> &f, long long j, V3<R> v) { st3(f.p + j, v); }
 template <typename R>
-__device__ __forceinline__ void stf(const SoA<R> &f, long long j, V3<R> v) {
+__device__ __forceinline__ void stf(const SoA<R> &f, int j, V3<R> v) {
   f.p[j] = v.x;
-  f.p[j + f.s] = v.y;
-  f.p[j + 2 * f.s] = v.z;
+  (f.p + f.s)[j] = v.y;
+  (f.p + 2 * f.s)[j] = v.z;
 }
 
 enum EpilogueMode : int {
@@ -157,7 +159,7 @@ struct AxisSums {
 // this with compile-time knowledge instead (only the centre derivative coefficient is zero)
 template <typename R, typename F, bool HALL, bool HOD, bool CHK>
 __device__ __forceinline__ void accumulate(AxisSums<R> &s, const StageArgs<R, F> &a, int conv, int axis, R cD, R cH,
-                                           long long j) {
+                                           int j) {
   const V3<R> B = ldf(a.bk, j);
   if (conv && (!CHK || cD != (R)0)) {
     const V3<R> U = ldf(a.u, j);
@@ -190,7 +192,7 @@ __device__ __forceinline__ void accumulate(AxisSums<R> &s, const StageArgs<R, F>
 // the reference per stencil point; used only by the DISS_FO_OR_AD instantiation.
 template <typename R, typename F, int OP, bool PER>
 __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], const int nn[3],
-                                   const long long st[3], long long idx, V3<R> Bm, V3<R> um) {
+                                   const int st[3], int idx, V3<R> Bm, V3<R> um) {
   constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, WH = Op<OP>::WH;
   V3<R> acc = {0, 0, 0};
   const bool adaptive = a.diss_form == 3;
@@ -212,7 +214,7 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
       const int o = c - C0;
       const R cd = fabs(a.tab->D[row][c]);
       if (cd == (R)0) continue;   // a zero coefficient adds a zero term: skip its loads
-      const long long j = idx + (long long)(nbr<PER>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
+      const int j = idx + (nbr<PER>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
       const V3<R> Bk = ldf(a.bk, j);
       const V3<R> uk = ldf(a.u, j);
       V3<R> sg = {fmax(fabs(uk.x), fabs(um.x)), fmax(fabs(uk.y), fabs(um.y)), fmax(fabs(uk.z), fabs(um.z))};
@@ -234,15 +236,15 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
     for (int term = -WH + 1; term <= 0; ++term) {
       for (int ax = 0; ax < 3; ++ax) {
         const int row = PER ? NB : sbp_row(ii[ax], nn[ax], NB);
-        const long long j1 = idx + (long long)(nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
-        const long long j2 = idx + (long long)(nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
+        const int j1 = idx + (nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
+        const int j2 = idx + (nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
         const V3<R> b1 = ldf(a.bk, j1), b2 = ldf(a.bk, j2), u1 = ldf(a.u, j1), u2 = ldf(a.u, j2);
         // diff_HOD (artificial_dissipation.h:58-101) for this start offset
         const R sgn = (Op<OP>::ORDER / 2 + 1) % 2 ? (R)-1 : (R)1;
         V3<R> hod = {0, 0, 0};
         for (int i = 0; i < WH; ++i) {
           const R coef = ((a.tab->Minv[row] * a.tab->DHO[row][term + WH - 1]) * a.tab->DHO[NB][i]) * sgn;
-          const long long j = idx + (long long)(nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
+          const int j = idx + (nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
           const V3<R> Bk = ldf(a.bk, j);
           hod.x += coef * Bk.x; hod.y += coef * Bk.y; hod.z += coef * Bk.z;
         }
@@ -255,9 +257,33 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
   return acc;
 }
 
+// the inflow factors of a face node (induction_Eq_surface.cl:7-33, upwind against
+// b_boundary(t)): f[ax] = sat_s c u_ax on an inflow face of the axis, else 0; whether any is set
+template <typename R, typename F>
+__device__ __forceinline__ bool sat_inflow(const StageArgs<R, F> &a, const int ii[3], const int nn[3],
+                                           const V3<R> &um, R (&f)[3]) {
+  bool any = false;
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    const R ua = ax == 0 ? um.x : (ax == 1 ? um.y : um.z);
+    const R c = (ii[ax] == 0 && ua > (R)0 ? (R)-1 : (R)0) + (ii[ax] == nn[ax] - 1 && ua < (R)0 ? (R)1 : (R)0);
+    f[ax] = c == (R)0 ? (R)0 : (a.sat_s[ax] * c) * ua;
+    any = any || c != (R)0;
+  }
+  return any;
+}
+template <typename R>
+__device__ __forceinline__ void sat_inflow_add(const R (&f)[3], const V3<R> &df, V3<R> &db) {
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    if (f[ax] == (R)0) continue;
+    db.x += f[ax] * df.x; db.y += f[ax] * df.y; db.z += f[ax] * df.z;
+  }
+}
+
 // SAT surface terms on the faces of a non-periodic box (added into db)
 template <typename R, typename F, bool HALL>
-__device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii[3], const int nn[3], long long idx,
+__device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii[3], const int nn[3], int idx,
                                           const V3<R> &Bm, const V3<R> &um, int conv, V3<R> &db) {
   const int ix = ii[0], iy = ii[1], iz = ii[2], nx = nn[0], ny = nn[1], nz = nn[2];
   const bool face = ix == 0 || iy == 0 || iz == 0 || ix == nx - 1 || iy == ny - 1 || iz == nz - 1;
@@ -279,19 +305,44 @@ __device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii
         db.z += a.sat_s[ax] * (f1 * Bm.z + f2 * Jm.z);
       }
     } else if (conv) {
-      // induction_Eq_surface.cl:7-33 (upwind inflow against b_boundary(t))
-      const R t = a.time[1];
-      const V3<R> bb = b_boundary<R>(a.tc, a.m, ix, iy, iz, t);
-      const V3<R> df = {Bm.x - bb.x, Bm.y - bb.y, Bm.z - bb.z};
-      for (int ax = 0; ax < 3; ++ax) {
-        const bool l = ii[ax] == 0, r = ii[ax] == nn[ax] - 1;
-        const R ua = ax == 0 ? um.x : (ax == 1 ? um.y : um.z);
-        const R c = (l && ua > (R)0 ? (R)-1 : (R)0) + (r && ua < (R)0 ? (R)1 : (R)0);
-        if (c == (R)0) continue;
-        const R f = (a.sat_s[ax] * c) * ua;
-        db.x += f * df.x; db.y += f * df.y; db.z += f * df.z;
+      R f[3];
+      if (sat_inflow(a, ii, nn, um, f)) {
+        const V3<R> bb = b_boundary<R>(a.tc, a.m, ix, iy, iz, a.time[1]);
+        sat_inflow_add(f, V3<R>{Bm.x - bb.x, Bm.y - bb.y, Bm.z - bb.z}, db);
       }
     }
+  }
+}
+
+// stage_sat of the inflow terms at two x-adjacent nodes (ix even).  b_boundary costs more than
+// the rest of a face node (its exponential and trigonometric functions), and a warp that holds
+// the ends of a row has one node at x = 0 in one lane and one at x = nx - 1 in another: every
+// lane takes its inflow node, whichever of the two it is, in the same pass, and a second pass
+// runs only where both nodes of a lane have one (y and z faces).
+template <typename R, typename F>
+__device__ __forceinline__ void stage_sat_pair(const StageArgs<R, F> &a, int ix, int iy, int iz, const int nn[3],
+                                               const V3<R> (&Bm)[2], const V3<R> (&um)[2], V3<R> (&db)[2]) {
+  const int i0[3] = {ix, iy, iz}, i1[3] = {ix + 1, iy, iz};
+  if (ix != 0 && iy != 0 && iz != 0 && ix + 1 != nn[0] - 1 && iy != nn[1] - 1 && iz != nn[2] - 1) return;
+  R f0[3], f1[3];
+  const bool need0 = sat_inflow(a, i0, nn, um[0], f0), need1 = sat_inflow(a, i1, nn, um[1], f1);
+  if (!need0 && !need1) return;
+  const R t = a.time[1];
+  int k = need0 ? 0 : 1;
+#pragma unroll 1
+  for (;;) {
+    const V3<R> bb = b_boundary<R>(a.tc, a.m, ix + k, iy, iz, t);
+    const V3<R> B = k ? Bm[1] : Bm[0];
+    V3<R> d = k ? db[1] : db[0];
+    const R f[3] = {k ? f1[0] : f0[0], k ? f1[1] : f0[1], k ? f1[2] : f0[2]};
+    sat_inflow_add(f, V3<R>{B.x - bb.x, B.y - bb.y, B.z - bb.z}, d);
+    if (k) {
+      db[1] = d;
+      break;
+    }
+    db[0] = d;
+    if (!need1) break;
+    k = 1;
   }
 }
 
@@ -304,7 +355,7 @@ struct EpIn {
 };
 
 template <typename R, typename F>
-__device__ __forceinline__ EpIn<R> epilogue_load(const StageArgs<R, F> &a, long long idx) {
+__device__ __forceinline__ EpIn<R> epilogue_load(const StageArgs<R, F> &a, int idx) {
   EpIn<R> e = {{0, 0, 0}, {0, 0, 0}};
   switch (a.mode) {
     case EP_X_PLUS_HF:
@@ -379,7 +430,7 @@ __device__ __forceinline__ EpOut<R> epilogue_values(const StageArgs<R, F> &a, co
 }
 
 template <typename R, typename F>
-__device__ __forceinline__ void epilogue_store(const StageArgs<R, F> &a, long long idx, const V3<R> &db,
+__device__ __forceinline__ void epilogue_store(const StageArgs<R, F> &a, int idx, const V3<R> &db,
                                                const EpIn<R> &e) {
   const EpOut<R> r = epilogue_values(a, db, e);
   stf(a.out, idx, r.o1);
@@ -388,23 +439,21 @@ __device__ __forceinline__ void epilogue_store(const StageArgs<R, F> &a, long lo
 }
 
 template <typename R, typename F>
-__device__ __forceinline__ void stage_epilogue(const StageArgs<R, F> &a, long long idx, const V3<R> &db) {
+__device__ __forceinline__ void stage_epilogue(const StageArgs<R, F> &a, int idx, const V3<R> &db) {
   epilogue_store(a, idx, db, epilogue_load(a, idx));
 }
 
 // DB and the stage update at one node (ix, iy, iz) inside the grid.
 template <typename R, typename F, int OP, bool PER, bool HALL, int DISS, int CONV>
 __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int iy, int iz) {
-  constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, WH = Op<OP>::WH;
-  constexpr int RI = Op<OP>::RI;
-  constexpr int RB = (C0 > WH - 1) ? C0 : WH - 1;
+  constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
   constexpr bool HOD = DISS == DISS_HO;
   const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
   {
-    const long long idx = ix + (long long)nx * (iy + (long long)ny * iz);
+    const int idx = ix + nx * (iy + ny * iz);
     const int ii[3] = {ix, iy, iz};
     const int nn[3] = {nx, ny, nz};
-    const long long st[3] = {1, nx, (long long)nx * ny};
+    const int st[3] = {1, nx, nx * ny};
     const int conv = CONV >= 0 ? CONV : (a.conv_flag ? *a.conv_flag : a.conv);
     const V3<R> Bm = ldf(a.bk, idx);
     V3<R> um = {0, 0, 0};
@@ -415,17 +464,17 @@ __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int
     for (int ax = 0; ax < 3; ++ax) {
       AxisSums<R> s{};
       const int row = PER ? NB : sbp_row(ii[ax], nn[ax], NB);
-      if (row == NB) {
+      if (PER || warp_on_row(row, NB)) {
         // periodic neighbours wrap only within RI of the ends of the axis
         const bool wrap = PER && (ii[ax] < RI || ii[ax] >= nn[ax] - RI);
 #pragma unroll
         for (int o = -RI; o <= RI; ++o) {
           const R cD = a.Dint[o + RI];
           const R cH = a.Hint[o + RI];
-          long long j = idx;
+          int j = idx;
           if (o != 0) {
-            if (wrap) j = idx + (long long)(nbr<true>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
-            else j = idx + (long long)o * st[ax];
+            if (wrap) j = idx + (nbr<true>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
+            else j = idx + o * st[ax];
             accumulate<R, F, HALL, HOD, false>(s, a, conv, ax, cD, cH, j);
           } else if (HOD) {
             // the interior derivative rows have a zero centre
@@ -433,12 +482,14 @@ __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int
           }
         }
       } else {
-        for (int o = -RB; o <= RB; ++o) {
-          const R cD = (o >= -C0 && o <= C0) ? a.tab->D[row][o + C0] : (R)0;
-          const R cH = (HOD && o >= -(WH - 1) && o <= WH - 1) ? a.tab->H[row][o + WH - 1] : (R)0;
+        constexpr int NT = HOD ? Op<OP>::NU : Op<OP>::ND;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const R cD = HOD ? __ldg(&a.tab->ud[row][t]) : __ldg(&a.tab->nd[row][t]);
+          const R cH = HOD ? __ldg(&a.tab->uh[row][t]) : (R)0;
+          const int o = HOD ? __ldg(&a.tab->ud_off[row][t]) : __ldg(&a.tab->nd_off[row][t]);
           if (cD == (R)0 && cH == (R)0) continue;
-          const long long j = idx + (long long)(nbr<PER>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
-          accumulate<R, F, HALL, HOD, true>(s, a, conv, ax, cD, cH, j);
+          accumulate<R, F, HALL, HOD, true>(s, a, conv, ax, cD, cH, idx + o * st[ax]);
         }
       }
       if (conv) {
@@ -533,21 +584,21 @@ struct CurlArgs {
 };
 
 template <typename R, typename F>
-__device__ __forceinline__ R ldc(const F &f, long long j, int comp);
+__device__ __forceinline__ R ldc(const F &f, int j, int comp);
 template <>
-__device__ __forceinline__ double ldc<double, SoA<double>>(const SoA<double> &f, long long j, int comp) {
-  return __ldg(f.p + j + comp * f.s);
+__device__ __forceinline__ double ldc<double, SoA<double>>(const SoA<double> &f, int j, int comp) {
+  return __ldg(f.p + comp * f.s + j);
 }
 template <>
-__device__ __forceinline__ float ldc<float, SoA<float>>(const SoA<float> &f, long long j, int comp) {
-  return __ldg(f.p + j + comp * f.s);
+__device__ __forceinline__ float ldc<float, SoA<float>>(const SoA<float> &f, int j, int comp) {
+  return __ldg(f.p + comp * f.s + j);
 }
 template <>
-__device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f, long long j, int comp) {
+__device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f, int j, int comp) {
   return __ldg(reinterpret_cast<const double *>(f.p + j) + comp);
 }
 template <>
-__device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, long long j, int comp) {
+__device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, int j, int comp) {
   return __ldg(reinterpret_cast<const float *>(f.p + j) + comp);
 }
 
@@ -556,40 +607,45 @@ __device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, lon
 // rounding of the reference's divisions).
 template <typename R, typename F, int OP, bool PER>
 __global__ void __launch_bounds__(256) k_curl_rho(const __grid_constant__ CurlArgs<R, F> a) {
-  constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, RI = Op<OP>::RI;
+  constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= a.m.nx || iy >= a.m.ny || iz >= a.m.nz) return;
-  const long long idx = ix + (long long)a.m.nx * (iy + (long long)a.m.ny * iz);
+  const int idx = ix + a.m.nx * (iy + a.m.ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {a.m.nx, a.m.ny, a.m.nz};
-  const long long st[3] = {1, a.m.nx, (long long)a.m.nx * a.m.ny};
+  const int st[3] = {1, a.m.nx, a.m.nx * a.m.ny};
   R g[3][3];   // g[axis][component]
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
     const int c1 = (ax + 1) % 3, c2 = (ax + 2) % 3;
     R v1 = 0, v2 = 0;
     const int row = PER ? NB : sbp_row(ii[ax], nn[ax], NB);
-    if (row == NB) {
+    if (PER || warp_on_row(row, NB)) {
       const bool wrap = PER && (ii[ax] < RI || ii[ax] >= nn[ax] - RI);
 #pragma unroll
       for (int o = -RI; o <= RI; ++o) {
         if (o == 0) continue;   // the interior row has a zero centre
         const R c = a.Dint[o + RI];
-        long long j;
-        if (wrap) j = idx + (long long)(nbr<true>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
-        else j = idx + (long long)o * st[ax];
+        int j;
+        if (wrap) j = idx + (nbr<true>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
+        else j = idx + o * st[ax];
         v1 += c * ldc<R, F>(a.b, j, c1);
         v2 += c * ldc<R, F>(a.b, j, c2);
       }
     } else {
-      for (int o = -C0; o <= C0; ++o) {
-        const R c = a.tab->D[row][o + C0];
-        if (c == (R)0) continue;
-        const long long j = idx + (long long)(nbr<PER>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
-        v1 += c * ldc<R, F>(a.b, j, c1);
-        v2 += c * ldc<R, F>(a.b, j, c2);
+#pragma unroll
+      for (int t = 0; t < Op<OP>::ND; ++t) {
+        const R c = __ldg(&a.tab->nd[row][t]);
+        const int j = idx + __ldg(&a.tab->nd_off[row][t]) * st[ax];
+        R p1 = 0, p2 = 0;
+        if (c != (R)0) {
+          p1 = ldc<R, F>(a.b, j, c1);
+          p2 = ldc<R, F>(a.b, j, c2);
+        }
+        v1 += c * p1;
+        v2 += c * p2;
       }
     }
     g[ax][c1] = v1 * a.inv_d[ax];
