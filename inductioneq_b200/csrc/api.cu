@@ -71,6 +71,7 @@ ieq_status fail(ieq_ctx *ctx, ieq_status st, const std::string &msg) {
 Mesh mesh_of(const ieq_ctx *c) {
   Mesh m;
   m.nx = c->s.nodes[0];
+  m.px = c->s.nodes[0];
   m.ny = c->s.nodes[1];
   m.nz = c->s.nodes[2];
   for (int a = 0; a < 3; ++a) {
@@ -80,6 +81,23 @@ Mesh mesh_of(const ieq_ctx *c) {
   m.omega = c->s.omega;
   m.zoff = c->s.zoff;
   m.nzg = c->s.nzg;
+  return m;
+}
+
+// the mesh of fields of layout F: the caller's arrays, or the fused state with its row pitch
+template <typename F>
+struct IsSoA {
+  static constexpr bool value = false;
+};
+template <typename R>
+struct IsSoA<SoA<R>> {
+  static constexpr bool value = true;
+};
+inline int soa_pitch(const ieq_ctx *c) { return c->s.nodes[0] + (!c->s.periodic && c->s.nodes[0] % 2 ? 1 : 0); }
+template <typename F>
+Mesh mesh_for(const ieq_ctx *c) {
+  Mesh m = mesh_of(c);
+  if (IsSoA<F>::value) m.px = c->px;
   return m;
 }
 
@@ -212,7 +230,7 @@ template <typename R, typename F = AoS<R>>
 StageArgs<R, F> stage_base(ieq_ctx *c, bool conv) {
   StageArgs<R, F> a;
   std::memset(&a, 0, sizeof(a));
-  a.m = mesh_of(c);
+  a.m = mesh_for<F>(c);
   a.tab = tables<R>(c);
   const SbpOperator &op = c->op;
   const int RI = op.order / 2, C0 = (op.sw - 1) / 2, WH = op.w_hod;
@@ -390,7 +408,7 @@ template <typename R, typename F>
 CurlArgs<R, F> curl_args(ieq_ctx *c, F b, const R *rho, F out) {
   CurlArgs<R, F> a;
   std::memset(&a, 0, sizeof(a));
-  a.m = mesh_of(c);
+  a.m = mesh_for<F>(c);
   a.b = b;
   a.rho = rho;
   a.out = out;
@@ -851,6 +869,11 @@ ieq_status ieq_create(ieq_ctx **out, const char *settings, const char *const *pa
   c->n = (size_t)c->s.nodes[0] * c->s.nodes[1] * c->s.nodes[2];
   c->n_pad = (c->n + c->s.w_size - 1) / c->s.w_size * c->s.w_size;   // initialize.m:43-44
   c->n_groups = c->n_pad / c->s.w_size;
+  // the fused state of a box with odd rows has one more element per row, so that node pairs
+  // load whole 16-byte vectors in every row (a periodic row's pairs would wrap misaligned)
+  c->px = soa_pitch(c);
+  c->soa_n = std::max(c->n_pad, (size_t)c->px * c->s.nodes[1] * c->s.nodes[2]);
+  c->soa_n = (c->soa_n + 3) / 4 * 4;
   ieq_status st = IEQ_OK;
   auto cuda = [&](cudaError_t e, const char *what) {
     if (e != cudaSuccess && st == IEQ_OK) {

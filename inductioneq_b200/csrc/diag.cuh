@@ -37,12 +37,13 @@ __device__ __forceinline__ void diag_terms(const DiagArgs<R, F> &a, long long i,
   const int iy = (int)(r % a.m.ny);
   const int iz = (int)(r / a.m.ny);
   const R fac = (a.wx[ix] * a.wy[iy]) * a.wz[iz];
-  const V3<R> B = ldf(a.b, i);
+  const long long ib = ix + (long long)a.m.px * r;   // the node in the field's layout
+  const V3<R> B = ldf(a.b, ib);
   e += (double)(fac * ((B.x * B.x + B.y * B.y) + B.z * B.z));
   // calc_div (kernel_operator.cl:145): sum over the axes of d/d(axis) of that component
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {a.m.nx, a.m.ny, a.m.nz};
-  const long long st[3] = {1, a.m.nx, (long long)a.m.nx * a.m.ny};
+  const long long st[3] = {1, a.m.px, (long long)a.m.px * a.m.ny};
   const int c0 = (a.sw - 1) / 2;
   R d[3];
 #pragma unroll
@@ -52,7 +53,7 @@ __device__ __forceinline__ void diag_terms(const DiagArgs<R, F> &a, long long i,
     for (int c = 0; c < a.sw; ++c) {
       const R cf = a.D[row * a.sw + c];
       if (cf == (R)0) continue;
-      const long long j = i + (long long)(nbr_rt<R>(ii[ax], c - c0, nn[ax], a.periodic) - ii[ax]) * st[ax];
+      const long long j = ib + (long long)(nbr_rt<R>(ii[ax], c - c0, nn[ax], a.periodic) - ii[ax]) * st[ax];
       v += cf * ldc<R, F>(a.b, j, ax);
     }
     d[ax] = v / a.dS[ax];

@@ -36,10 +36,10 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e_diag(const __grid_consta
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   double acc[3] = {0.0, 0.0, 0.0};
   if (ix < nx && iy < ny && iz < nz) {
-    const long long idx = ix + (long long)nx * (iy + (long long)ny * iz);
+    const int idx = ix + a.m.px * (iy + ny * iz);
     const int ii[3] = {ix, iy, iz};
     const int nn[3] = {nx, ny, nz};
-    const long long st[3] = {1, nx, (long long)nx * ny};
+    const int st[3] = {1, a.m.px, a.m.px * ny};
     const V3<R> Bm = ldf(a.b, idx);
     R g[3][3];
     V3<R> hod = {0, 0, 0};
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e_diag(const __grid_consta
     if (HODS) stf(a.hout, idx, hod);
     if (!PER && (ix == 0 || iy == 0 || iz == 0 || ix == nx - 1 || iy == ny - 1 || iz == nz - 1))
       stf(a.jface, idx, J);
-    diag_terms(d, idx, acc[0], acc[1], acc[2]);
+    diag_terms(d, ix + (long long)nx * (iy + (long long)ny * iz), acc[0], acc[1], acc[2]);
   }
   // block partials (whole warps: the launcher gives 128-thread blocks), then the last block
   // adds them in a fixed order

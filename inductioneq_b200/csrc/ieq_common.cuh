@@ -131,6 +131,8 @@ enum Testcase : int {
 
 struct Mesh {
   int nx, ny, nz;
+  int px;            // elements from one x row of a field to the next: nx, or one more in the
+                     // fused state of a box with odd rows, whose rows then start 16-byte aligned
   double xmin[3];
   double d[3];       // DX, DY, DZ
   double omega;      // rotation rate of TC_ROTATION_GAUSSIAN

@@ -128,6 +128,8 @@ struct ieq_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   size_t n = 0, n_pad = 0, n_groups = 0;
+  int px = 0;                      // row pitch of the fused state (nx, or nx + 1: boxes with odd rows)
+  size_t soa_n = 0;                // elements of one component plane of the fused state
   int op_id = 0;
   // device tables
   void *d_tables = nullptr;        // Tables<REAL>

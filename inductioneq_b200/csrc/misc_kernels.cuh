@@ -46,7 +46,7 @@ __device__ void hall_periodic_u_block(const Mesh &m, R *vout, long long vstride,
   __syncthreads();
   const int ix = base[0] + threadIdx.x, iy = base[1] + threadIdx.y, iz = base[2] + threadIdx.z;
   if (ix >= m.nx || iy >= m.ny || iz >= m.nz) return;
-  const long long idx = ix + (long long)m.nx * (iy + (long long)m.ny * iz);
+  const long long idx = ix + (long long)m.px * (iy + (long long)m.ny * iz);
   const int x = threadIdx.x, y = threadIdx.y, z = threadIdx.z;
   st_any(vout, vstride, idx, V3<R>{tc[1][y] + ts[2][z], tc[2][z] + ts[0][x], tc[0][x] + ts[1][y]});
 }
@@ -62,7 +62,7 @@ __global__ void k_init(Mesh m, int tc, int kind, R *vout, long long vstride, R *
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= m.nx || iy >= m.ny || iz >= m.nz) return;
-  const long long idx = ix + (long long)m.nx * (iy + (long long)m.ny * iz);
+  const long long idx = ix + (long long)m.px * (iy + (long long)m.ny * iz);
   switch (kind) {
     case INIT_B: st_any(vout, vstride, idx, b_analytical<R>(tc, m, ix, iy, iz, (R)0)); break;
     case INIT_U: st_any(vout, vstride, idx, u_analytical<R>(tc, m, ix, iy, iz, (R)0)); break;

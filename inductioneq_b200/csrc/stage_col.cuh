@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
   const int iz0 = (blockIdx.z * blockDim.z + threadIdx.z) * NZ;
   if (ix < nx && iy < ny && iz0 < nz) {
     const int cnt = nz - iz0 < NZ ? nz - iz0 : NZ;
-    const int sz = nx * ny;
-    const int base = ix + nx * iy;
+    const int sz = a.m.px * ny;
+    const int base = ix + a.m.px * iy;
     const V3<R> zero = {0, 0, 0};
     V3<R> Bm[NZ], um[NZ], db[NZ], hod[NZ];
 #pragma unroll
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
         for (int ax = 0; ax < 2; ++ax) {
           ColSums<R> s{};
           col_axis<R, OP, PER, HALL, HOD, CONV, SoA<R>, NEED>(s, a, ax, ax == 0 ? ix : iy, ax == 0 ? nx : ny, idx,
-                                                             ax == 0 ? 1 : nx, Bm[k]);
+                                                             ax == 0 ? 1 : a.m.px, Bm[k]);
           col_combine<R, HALL, HOD, CONV>(a, ax, s, Bm[k], um[k], db[k], hod[k]);
         }
       }
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
           d.z += a.hod_factor * hv.z;
         }
         if (FOAD) {
-          const int st[3] = {1, nx, sz};
+          const int st[3] = {1, a.m.px, sz};
           const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, PER>(a, ii, nn, st, idx, Bm[k], um[k]);
           d.x += ds.x; d.y += ds.y; d.z += ds.z;
         }
@@ -429,10 +429,10 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e(const __grid_constant__ 
   const int iz0 = (blockIdx.z * blockDim.z + threadIdx.z) * NZ;
   if (ix >= nx || iy >= ny || iz0 >= nz) return;
   const int cnt = nz - iz0 < NZ ? nz - iz0 : NZ;
-  const int sz = nx * ny;
-  const int base = ix + nx * iy;
+  const int sz = a.m.px * ny;
+  const int base = ix + a.m.px * iy;
   const int nn[3] = {nx, ny, nz};
-  const int st[3] = {1, nx, sz};
+  const int st[3] = {1, a.m.px, sz};
   R g[NZ][3][3];   // g[node][axis][component]
   // one axis at one node: the derivatives of the two components orthogonal to it
   auto axis = [&](int ax, int i, int idx, R &v1, R &v2) {
@@ -532,10 +532,10 @@ __global__ void __launch_bounds__(kColThreads, IEQ_CURL_MIN_BLOCKS * 128 / kColT
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= nx || iy >= ny || iz >= nz) return;
-  const int idx = ix + nx * (iy + ny * iz);
+  const int idx = ix + a.m.px * (iy + ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {nx, ny, nz};
-  const int st[3] = {1, nx, nx * ny};
+  const int st[3] = {1, a.m.px, a.m.px * ny};
   const V3<R> Bm = ldf(a.b, idx);
   R g[3][3];
   V3<R> hod = {0, 0, 0};

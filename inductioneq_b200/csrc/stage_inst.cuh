@@ -119,8 +119,9 @@ static void launch_stage_hall_k(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per,
   if constexpr (K == 4 && sizeof(IEQ_R) != 4) {
     return;   // (quads are FP32 only; the caller never asks for them in FP64)
   } else {
-    const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx, K);
-    const dim3 g = col_grid(ps, a.m.nx / K, a.m.ny, a.m.nz, 1), b = col_block(ps);
+    const int np = (a.m.nx + K - 1) / K;
+    const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, K * np, K);
+    const dim3 g = col_grid(ps, np, a.m.ny, a.m.nz, 1), b = col_block(ps);
     if (per) {
       if (hodp) launch_pdl(k_stage_hall_x2<IEQ_R, IEQ_OP, true, true, K>, g, b, s, sh.pdl, a);
       else launch_pdl(k_stage_hall_x2<IEQ_R, IEQ_OP, true, false, K>, g, b, s, sh.pdl, a);
@@ -161,8 +162,9 @@ static void launch_hall_conv_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool p
                     k_stage_xband<IEQ_R, IEQ_OP, true, false, 1, N, false, false>, a, sh, s);
     return;
   }
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx);
-  const dim3 g2 = col_grid(ps, a.m.nx / 2, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
+  const int np = (a.m.nx + 1) / 2;
+  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const dim3 g2 = col_grid(ps, np, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
   if (per) {
     if (hodp) launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, true, true, 1, true, false, N>, g2, b2, s, sh.pdl, a);
     else launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, true, false, 1, false, false, N>, g2, b2, s, sh.pdl, a);
@@ -180,8 +182,9 @@ static void launch_conv_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, C
                   k_stage_xband<IEQ_R, IEQ_OP, false, false, 1, N, false, false>, a, sh, s);
     return;
   }
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx);
-  const dim3 g2 = col_grid(ps, a.m.nx / 2, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
+  const int np = (a.m.nx + 1) / 2;
+  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const dim3 g2 = col_grid(ps, np, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
   if (per) launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, false, false, 1, false, false, N>, g2, b2, s, sh.pdl, a);
   else launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, false, false, false, 1, false, false, N>, g2, b2, s, sh.pdl, a);
 }
@@ -194,8 +197,9 @@ static void launch_fo_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, Col
                   k_stage_xband<IEQ_R, IEQ_OP, H, false, 1, 10, false, false, true>, a, sh, s);
     return;
   }
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx);
-  const dim3 g2 = col_grid(ps, a.m.nx / 2, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
+  const int np = (a.m.nx + 1) / 2;
+  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const dim3 g2 = col_grid(ps, np, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
   if (per) launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, H, false, 1, false, false, 10, false, true>, g2, b2, s, sh.pdl, a);
   else launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, false, H, false, 1, false, false, 10, false, true>, g2, b2, s, sh.pdl, a);
 }
@@ -207,7 +211,7 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
   const dim3 g = col_grid(s1, a.m.nx, a.m.ny, a.m.nz, col_nodes(conv)), b = col_block(s1);
   // the precomputed dissipation sum comes with the Hall curl kernel only
   hodp = hodp && hall && hod && !foad;
-  if (sh.pairs && hall && !conv && !foad && (hodp || !hod) && a.m.nx % 2 == 0 && pair_ok(a.E) &&
+  if (sh.pairs && hall && !conv && !foad && (hodp || !hod) && pair_rows(a.m, per) && pair_ok(a.E) &&
       pair_ok(a.Hpre) && pair_ok(a.X) && pair_ok(a.Y) && pair_ok(a.Z) && pair_ok(a.out) && pair_ok(a.out2) &&
       pair_ok(a.out3)) {
     // FP32: four nodes per thread (float4) where the fields allow it
@@ -235,7 +239,7 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
   // second time (measured on B200, CK2N54, 64^3, Hall: periodic with variable u 4th / 6th order
   // 2.21e10 / 1.83e10 DOF/s against 1.12e10 / 8.2e9, confined box 1.80e10 / 1.30e10 against
   // 1.17e10 / 7.4e9)
-  if (sh.pairs && conv && foad && a.diss_form == 2 && a.need == 10 && a.m.nx % 2 == 0 && pair_ok(a.bk) &&
+  if (sh.pairs && conv && foad && a.diss_form == 2 && a.need == 10 && pair_rows(a.m, per) && pair_ok(a.bk) &&
       pair_ok(a.u) && pair_ok(a.E) && pair_ok(a.X) && pair_ok(a.Y) && pair_ok(a.Z) && pair_ok(a.out) &&
       pair_ok(a.out2) && pair_ok(a.out3)) {
     if (hall) launch_fo_pairs<true>(a, per, sh, s);
@@ -250,7 +254,7 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
   if (sh.pairs && hall && conv && !foad && (hodp || !hod) &&
       (a.need == 10 || a.need == 9 || a.need == 6 || a.need == 7 || a.need == 13 || a.need == 14 ||
        a.need == 15) &&
-      a.m.nx % 2 == 0 && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.E) && pair_ok(a.Hpre) && pair_ok(a.X) &&
+      pair_rows(a.m, per) && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.E) && pair_ok(a.Hpre) && pair_ok(a.X) &&
       pair_ok(a.Y) && pair_ok(a.Z) && pair_ok(a.out) && pair_ok(a.out2) && pair_ok(a.out3)) {
     switch (a.need) {
       case 9: launch_hall_conv_pairs<9>(a, per, hodp, sh, s); break;
@@ -269,7 +273,7 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
   // 64^3 whistler 1.68e10 against 1.53e10 DOF/s).  On boxes and without the Hall term the
   // one-node kernels measured faster (the x boundary rows run per node, and the
   // convection sums of two nodes exceed the registers).
-  if (sh.pairs && per && hall && !foad && a.m.nx % 2 == 0 && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.E) &&
+  if (sh.pairs && per && hall && !foad && pair_rows(a.m, per) && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.E) &&
       pair_ok(a.Hpre) && pair_ok(a.X) && pair_ok(a.Y) && pair_ok(a.Z) && pair_ok(a.out) && pair_ok(a.out2) &&
       pair_ok(a.out3)) {
     const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx);
@@ -288,7 +292,7 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
   if (sh.pairs && !hall && conv && !hod && !foad &&
       (a.need == 10 || a.need == 9 || a.need == 6 || a.need == 7 || a.need == 13 || a.need == 14 ||
        a.need == 15) &&
-      a.m.nx % 2 == 0 && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.X) && pair_ok(a.Y) && pair_ok(a.Z) &&
+      pair_rows(a.m, per) && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.X) && pair_ok(a.Y) && pair_ok(a.Z) &&
       pair_ok(a.out) && pair_ok(a.out2) && pair_ok(a.out3)) {
     switch (a.need) {
       case 9: launch_conv_pairs<9>(a, per, sh, s); break;

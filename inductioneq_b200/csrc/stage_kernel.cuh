@@ -323,9 +323,10 @@ template <typename R, typename F>
 __device__ __forceinline__ void stage_sat_pair(const StageArgs<R, F> &a, int ix, int iy, int iz, const int nn[3],
                                                const V3<R> (&Bm)[2], const V3<R> (&um)[2], V3<R> (&db)[2]) {
   const int i0[3] = {ix, iy, iz}, i1[3] = {ix + 1, iy, iz};
-  if (ix != 0 && iy != 0 && iz != 0 && ix + 1 != nn[0] - 1 && iy != nn[1] - 1 && iz != nn[2] - 1) return;
+  if (ix != 0 && iy != 0 && iz != 0 && ix + 1 < nn[0] - 1 && iy != nn[1] - 1 && iz != nn[2] - 1) return;
   R f0[3], f1[3];
-  const bool need0 = sat_inflow(a, i0, nn, um[0], f0), need1 = sat_inflow(a, i1, nn, um[1], f1);
+  // (the last pair of an odd row has one node)
+  const bool need0 = sat_inflow(a, i0, nn, um[0], f0), need1 = ix + 1 < nn[0] && sat_inflow(a, i1, nn, um[1], f1);
   if (!need0 && !need1) return;
   const R t = a.time[1];
   int k = need0 ? 0 : 1;
@@ -450,10 +451,10 @@ __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int
   constexpr bool HOD = DISS == DISS_HO;
   const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
   {
-    const int idx = ix + nx * (iy + ny * iz);
+    const int idx = ix + a.m.px * (iy + ny * iz);
     const int ii[3] = {ix, iy, iz};
     const int nn[3] = {nx, ny, nz};
-    const int st[3] = {1, nx, nx * ny};
+    const int st[3] = {1, a.m.px, a.m.px * ny};
     const int conv = CONV >= 0 ? CONV : (a.conv_flag ? *a.conv_flag : a.conv);
     const V3<R> Bm = ldf(a.bk, idx);
     V3<R> um = {0, 0, 0};
@@ -612,10 +613,10 @@ __global__ void __launch_bounds__(256) k_curl_rho(const __grid_constant__ CurlAr
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= a.m.nx || iy >= a.m.ny || iz >= a.m.nz) return;
-  const int idx = ix + a.m.nx * (iy + a.m.ny * iz);
+  const int idx = ix + a.m.px * (iy + a.m.ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {a.m.nx, a.m.ny, a.m.nz};
-  const int st[3] = {1, a.m.nx, a.m.nx * a.m.ny};
+  const int st[3] = {1, a.m.px, a.m.px * a.m.ny};
   R g[3][3];   // g[axis][component]
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
@@ -669,19 +670,21 @@ void launch_curl(const CurlArgs<R, F> &a, bool per, dim3 grid, dim3 block, cudaS
 
 // layout conversion of a vector field between REAL4 AoS and SoA (fused path entry/exit)
 template <typename R>
-__global__ void k_aos_to_soa(long long n, const R4<R> *in, R *out, long long s) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void k_aos_to_soa(unsigned n, unsigned nx, unsigned px, const R4<R> *in, R *out, long long s) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const V3<R> v = ld3_plain(in + i);
-  out[i] = v.x;
-  out[i + s] = v.y;
-  out[i + 2 * s] = v.z;
+  const unsigned j = px == nx ? i : i + i / nx * (px - nx);
+  out[j] = v.x;
+  (out + s)[j] = v.y;
+  (out + 2 * s)[j] = v.z;
 }
 template <typename R>
-__global__ void k_soa_to_aos(long long n, const R *in, long long s, R4<R> *out) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void k_soa_to_aos(unsigned n, unsigned nx, unsigned px, const R *in, long long s, R4<R> *out) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  st3(out + i, V3<R>{in[i], in[i + s], in[i + 2 * s]});
+  const unsigned j = px == nx ? i : i + i / nx * (px - nx);
+  st3(out + i, V3<R>{in[j], (in + s)[j], (in + 2 * s)[j]});
 }
 
 }  // namespace ieq

@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kColThreads, HODS ? (K == 4 ? IEQ_CURL_X4_MIN_
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= nx - X0 || iy >= ny || iz >= nz) return;
-  const int row0 = nx * (iy + ny * iz);
+  const int row0 = a.m.px * (iy + ny * iz);
   const int idx = row0 + ix;
   const long long cs = a.b.s;
   const V3<R> zero = {0, 0, 0};
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kColThreads, HODS ? (K == 4 ? IEQ_CURL_X4_MIN_
   // y and z: all K nodes on the same row of the axis
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {nx, ny, nz};
-  const int st[3] = {1, nx, nx * ny};
+  const int st[3] = {1, a.m.px, a.m.px * ny};
 #pragma unroll
   for (int ax = 1; ax < 3; ++ax) {
     const int c1 = (ax + 1) % 3, c2 = (ax + 2) % 3;
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kColThreads, K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS 
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix < nx - X0 && iy < ny && iz < nz) {
-    const int row0 = nx * (iy + ny * iz);
+    const int row0 = a.m.px * (iy + ny * iz);
     const int idx = row0 + ix;
     const long long es = a.E.s;
     const V3<R> zero = {0, 0, 0};
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kColThreads, K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS 
       } else {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          col_axis<R, OP, PER, true, false, 0>(s[k], a, 0, ix + k, nx, idx + k, 1, zero);
+          if (ix + k < nx) col_axis<R, OP, PER, true, false, 0>(s[k], a, 0, ix + k, nx, idx + k, 1, zero);
       }
 #pragma unroll
       for (int k = 0; k < K; ++k) col_combine<R, true, false, 0>(a, 0, s[k], zero, zero, db[k], db[k]);
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(kColThreads, K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS 
     // y and z
     const int ii[3] = {ix, iy, iz};
     const int nn[3] = {nx, ny, nz};
-    const int st[3] = {1, nx, nx * ny};
+    const int st[3] = {1, a.m.px, a.m.px * ny};
 #pragma unroll
     for (int ax = 1; ax < 3; ++ax) {
       const int i = ii[ax], n = nn[ax];
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kColThreads, K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS 
     if (HODP) ldf_k<R, K>(a.Hpre, idx, hv);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      if (!PER) {
+      if (!PER && ix + k < nx) {
         const int iik[3] = {ix + k, iy, iz};
         stage_sat<R, SoA<R>, true>(a, iik, nn, idx + k, ldf(a.bk, idx + k), zero, 0, db[k]);
       }
@@ -660,12 +660,17 @@ __device__ __forceinline__ void col_x_pair_rows(ColSums<R> (&s)[2], const StageA
   constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, QX = Op<OP>::QX;
   const int need = NEED >= 0 ? NEED : a.need;
   const V3<R> zero = {0, 0, 0};
-  const R *rows[2] = {a.tab->D[sbp_row(ix, nx, NB)], a.tab->D[sbp_row(ix + 1, nx, NB)]};
+  // the last pair of an odd row has one node (its second values are never used), and the pairs
+  // of the right end then sit one node off: their rows reach a pair further
+  const int r0 = sbp_row(ix, nx, NB), r1 = sbp_row(min(ix + 1, nx - 1), nx, NB);
+  const R *rows[2] = {a.tab->D[r0], a.tab->D[r1]};
+  const bool far = (nx & 1) && (r0 != NB || r1 != NB);
 #pragma unroll
-  for (int q = -QX; q <= QX; ++q) {
+  for (int q = -QX - 1; q <= QX + 1; ++q) {
     const int xx = ix + 2 * q;
     V3<R> B[2] = {zero, zero}, U[2] = {zero, zero};
     R e1[2] = {0, 0}, e2[2] = {0, 0};
+    if ((q < -QX || q > QX) && !far) continue;
     if (xx >= 0 && xx < nx) col_load_pair<R, HALL, false, CONV>(a, 0, row0 + xx, B, U, e1, e2);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -778,7 +783,7 @@ __global__ void __launch_bounds__(kColThreads, FOF ? fo_min_blocks<OP, PER>()
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix < nx - X0 && iy < ny && iz < nz) {
-    const int row0 = nx * (iy + ny * iz);
+    const int row0 = a.m.px * (iy + ny * iz);
     const int idx = row0 + ix;
     const V3<R> zero = {0, 0, 0};
     V3<R> Bm[2], um[2] = {zero, zero}, db[2] = {zero, zero}, hod[2] = {zero, zero}, fo[2] = {zero, zero};
@@ -800,7 +805,7 @@ __global__ void __launch_bounds__(kColThreads, FOF ? fo_min_blocks<OP, PER>()
       }
     }
     const int nn[3] = {nx, ny, nz};
-    const int st[3] = {1, nx, nx * ny};
+    const int st[3] = {1, a.m.px, a.m.px * ny};
 #pragma unroll
     for (int ax = 1; ax < 3; ++ax) {
       ColSums<R> s[2] = {ColSums<R>{}, ColSums<R>{}};
@@ -817,7 +822,7 @@ __global__ void __launch_bounds__(kColThreads, FOF ? fo_min_blocks<OP, PER>()
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int ii[3] = {ix + k, iy, iz};
-      if (!PER && HALL) stage_sat<R, SoA<R>, HALL>(a, ii, nn, idx + k, Bm[k], um[k], CONV, db[k]);
+      if (!PER && HALL && ix + k < nx) stage_sat<R, SoA<R>, HALL>(a, ii, nn, idx + k, Bm[k], um[k], CONV, db[k]);
       if (HOD_) {
         db[k].x += a.hod_factor * hv[k].x;
         db[k].y += a.hod_factor * hv[k].y;
@@ -841,10 +846,10 @@ template <typename R, int OP, bool HALL, bool HOD_, int CONV, int NEED, bool HOD
 __device__ __forceinline__ void col_stage_node(const StageArgs<R, SoA<R>> &a, int ix, int iy, int iz) {
   constexpr bool HOD = HOD_ && !HODP;
   const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
-  const int idx = ix + nx * (iy + ny * iz);
+  const int idx = ix + a.m.px * (iy + ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {nx, ny, nz};
-  const int st[3] = {1, nx, nx * ny};
+  const int st[3] = {1, a.m.px, a.m.px * ny};
   const V3<R> zero = {0, 0, 0};
   const V3<R> Bm = ldf(a.bk, idx);
   const V3<R> um = CONV ? ldf(a.u, idx) : zero;
@@ -902,10 +907,10 @@ __global__ void __launch_bounds__(kColThreads) k_curl_xband(const __grid_constan
   const int slot = (int)(i % (2 * XB));
   const long long row = i / (2 * XB);
   const int ix = slot < XB ? slot : nx - 2 * XB + slot, iy = (int)(row % ny), iz = (int)(row / ny);
-  const int idx = ix + nx * (iy + ny * iz);
+  const int idx = ix + a.m.px * (iy + ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {nx, ny, nz};
-  const int st[3] = {1, nx, nx * ny};
+  const int st[3] = {1, a.m.px, a.m.px * ny};
   const V3<R> Bm = ldf(a.b, idx);
   R g[3][3];
   V3<R> hod = {0, 0, 0};
@@ -937,7 +942,12 @@ inline bool group_ok(const SoA<R> &f) {
   return f.p == nullptr || ((reinterpret_cast<uintptr_t>(f.p) % (K * sizeof(R))) == 0 && f.s % K == 0);
 }
 
-// whether a launch may use the pair kernels: nx even and every pair load or store aligned
+// whether rows hold whole node pairs: an even number of nodes, or (boxes) a pitch of one more,
+// whose last pair then has one node (rotation 97^3, 6th order, 30 stages: 2.34 ms against 2.52
+// with one node per thread on the unpadded rows; 12 batched solves, 3 of them odd, 14.0 / 15.0)
+inline bool pair_rows(const Mesh &m, bool per) { return m.nx % 2 == 0 || (!per && m.px > m.nx); }
+
+// whether a launch may use the pair kernels: whole pairs and every pair load or store aligned
 template <typename R>
 inline bool pair_ok(const SoA<R> &f) {
   return f.p == nullptr || ((reinterpret_cast<uintptr_t>(f.p) % (2 * sizeof(R))) == 0 && f.s % 2 == 0);
