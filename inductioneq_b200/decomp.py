@@ -539,8 +539,11 @@ def _device_scalar(solve):
     import torch
     dt = torch.float32 if solve.ctx.real == np.float32 else torch.float64
 
-    def make(_eng, v):
-        return torch.tensor([v], dtype=dt, device=torch.device("cuda", solve.device))
+    def make(eng, v):
+        # on the stream of the kernel that reads it: freed and handed out again on another
+        # stream, the next value would overwrite it before that kernel has run
+        with torch.cuda.stream(torch.cuda.ExternalStream(eng.stream, device=solve.device)):
+            return torch.tensor([v], dtype=dt, device=torch.device("cuda", solve.device))
     return make
 
 
