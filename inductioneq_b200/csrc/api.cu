@@ -131,6 +131,16 @@ ieq_status upload_tables(ieq_ctx *c) {
         t.H[r][s + i + WH - 1] += term;
       }
   }
+  for (int ax = 0; ax < 3; ++ax)
+    for (int k = 0; k < 4; ++k) {
+      const int k1 = k == 0 ? 1 : k;
+      const double kk = (double)(k1 * k1), dx = (double)(R)c->s.d[ax];
+      t.ad_lo[ax][k] = ((kk * c->s.mp2min) * c->s.cmin) * dx;
+      t.ad_hi[ax][k] = ((kk * c->s.mp2max) * c->s.cmax) * dx;
+      t.ad_thr[ax][k] = t.ad_hi[ax][k] > t.ad_lo[ax][k] ? (R)t.ad_lo[ax][k] : (R)-1;
+      if ((double)t.ad_thr[ax][k] > t.ad_lo[ax][k]) t.ad_thr[ax][k] = std::nextafter(t.ad_thr[ax][k], (R)-1);
+      t.ad_inv[ax][k] = 1.0 / std::fabs(t.ad_hi[ax][k] - t.ad_lo[ax][k]);
+    }
   // the same rows as lists of their non-zero entries
   const int c0 = (op.sw - 1) / 2, reach = std::max(c0, WH - 1);
   for (int r = 0; r < rows; ++r) {

@@ -91,6 +91,10 @@ struct Tables {
   R uh[MAX_ROWS][MAX_NU];       // ... and H
   int nd_off[MAX_ROWS][MAX_ND];
   int ud_off[MAX_ROWS][MAX_NU];
+  // adaptive dissipation on interior rows: the thresholds of kappa per axis and distance k (in
+  // the reference's order, include/artificial_dissipation.h:23-45) and 1 / |hi - lo|
+  double ad_lo[3][4], ad_hi[3][4], ad_inv[3][4];
+  R ad_thr[3][4];               // kappa is zero up to here (-1: thresholds out of order)
 };
 
 // whether every active lane of the warp sits on the interior row

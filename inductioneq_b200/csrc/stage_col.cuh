@@ -33,6 +33,12 @@ namespace ieq {
 #ifndef IEQ_COL_CONV_MIN_BLOCKS
 #define IEQ_COL_CONV_MIN_BLOCKS 6
 #endif
+// first-order / adaptive dissipation: Hall periodic 64^3, adaptive, 4th order, 20 stages: 788 us
+// with 5 blocks (<= 96 registers), 818 with 4; radius 3 holds more points and keeps 4
+template <int OP>
+__host__ __device__ constexpr int foad_min_blocks() {
+  return Op<OP>::RI >= 3 ? 4 : 5;
+}
 #ifndef IEQ_CURL_NODES
 #define IEQ_CURL_NODES 1
 #endif
@@ -147,22 +153,29 @@ __device__ __forceinline__ void col_load(const StageArgs<R, F> &a, int ax, int j
 // the sums of one axis at one node (interior row, periodic wrap or SBP boundary row);
 // NEED >= 0 fixes the flux-form mask (StageArgs::need) at compile time
 // FOF: also the first-order dissipation terms of the axis (*Um: u at the node)
+// AD: adaptive dissipation -- on the interior row, where every kappa of the warp's nodes is
+// zero, it is the high-order row, summed here (*quiet = true); else the caller adds the axis
 template <typename R, int OP, bool PER, bool HALL, bool HOD, int CONV, typename F = SoA<R>, int NEED = -1,
-          bool FOF = false>
+          bool FOF = false, bool AD = false>
 __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a, int ax, int i, int n,
                                          int idx, int st, const V3<R> &Bm,
-                                         const V3<R> *Um = nullptr) {
+                                         const V3<R> *Um = nullptr, bool *quiet = nullptr) {
   const int need = NEED >= 0 ? NEED : a.need;
   constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
   const V3<R> zero = {0, 0, 0};
   const int row = PER ? NB : sbp_row(i, n, NB);
   if (PER || warp_on_row(row, NB)) {
     const bool wrap = PER && (i < RI || i >= n - RI);
+    V3<R> Bp = Bm, Up = AD ? *Um : zero;   // the point before (AD: the pairs beyond the node's own)
+    bool loud = false;
 #pragma unroll
     for (int o = -RI; o <= RI; ++o) {
       if (o == 0) {
         // the interior derivative rows have a zero centre
         if (HOD) col_acc<R, false, HOD, 0>(s, ax, 0, (R)0, a.Hint[RI], false, true, Bm, zero, (R)0, (R)0);
+        if (AD) {
+          s.SHo.x += a.Hint[RI] * Bm.x; s.SHo.y += a.Hint[RI] * Bm.y; s.SHo.z += a.Hint[RI] * Bm.z;
+        }
         continue;
       }
       const int j = wrap ? idx + (nbr<true>(i, o, n) - i) * st : idx + o * st;
@@ -171,8 +184,20 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
       col_load<R, HALL, HOD, CONV, F>(a, ax, j, B, U, e1, e2);
       col_acc<R, HALL, HOD, CONV>(s, ax, need, a.Dint[o + RI], a.Hint[o + RI], true, true, B, U, e1, e2);
       if (FOF) fo_acc(s, a.Dint[o + RI], B, U, Bm, *Um);
+      if (AD) {
+        const R cH = a.Hint[o + RI];
+        s.SHo.x += cH * B.x; s.SHo.y += cH * B.y; s.SHo.z += cH * B.z;
+        loud = ad_test(B, U, Bm, *Um, __ldg(&a.tab->ad_thr[ax][o < 0 ? -o : o])) || loud;
+        if (o > 1) loud = ad_test(B, U, Bp, Up, __ldg(&a.tab->ad_thr[ax][1])) || loud;
+        if (o > 0) {
+          Bp = B;
+          Up = U;
+        }
+      }
     }
+    if (AD) *quiet = !__any_sync(__activemask(), loud);
   } else {
+    if (AD) *quiet = false;
     // boundary rows, and every row of a warp that holds one: the row's non-zero entries, all
     // loads free to issue before the first sum (as a run-time loop over the columns with a
     // test per column the loads came one at a time).  Padding entries load nothing, add zeros
@@ -231,10 +256,13 @@ __device__ __forceinline__ void col_combine(const StageArgs<R, F> &a, int ax, co
 
 // HODP: the dissipation sum comes precomputed (a.Hpre, written by k_curl_e_hod in the
 // same order of operations) instead of being gathered here
-// FOAD: first-order or adaptive dissipation (fo_ad_dissipation, after the SAT terms)
+// FOAD: 1 first-order dissipation, its terms summed in the gathers of the volume terms (fo_acc),
+// 2 adaptive (the axes whose kappas are all zero summed there, fo_ad_dissipation for the others;
+// without convection also first order); both added after the SAT terms
 template <typename R, int OP, bool PER, bool HALL, bool HOD_, int CONV, int NEED = -1, bool HODP = false,
-          bool FOAD = false>
-__global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS : IEQ_COL_MIN_BLOCKS) * 128 / kColThreads) k_stage_col(const __grid_constant__ StageArgs<R, SoA<R>> a) {
+          int FOAD = 0>
+__global__ void __launch_bounds__(kColThreads, (FOAD ? foad_min_blocks<OP>() : CONV ? IEQ_COL_CONV_MIN_BLOCKS : IEQ_COL_MIN_BLOCKS) * 128 / kColThreads)
+    k_stage_col(const __grid_constant__ StageArgs<R, SoA<R>> a) {
   constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI;
   pdl_enter();
   constexpr bool HOD = HOD_ && !HODP;   // the dissipation rows gathered in this kernel
@@ -249,6 +277,17 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
     const int sz = a.m.px * ny;
     const int base = ix + a.m.px * iy;
     const V3<R> zero = {0, 0, 0};
+    constexpr bool ADC = FOAD == 2 && CONV && NZ == 1;   // adaptive dissipation tested in the gathers
+    constexpr bool FOF = FOAD == 1 && CONV && NZ == 1;
+    static_assert(FOAD != 1 || FOF, "first-order dissipation needs the convection loads");
+    V3<R> fo = zero;
+    V3<R> quiet_sum = zero;
+    int quiet_axes = 0;
+    auto quiet_axis = [&](int ax, const ColSums<R> &s, bool quiet) {
+      if (!quiet) return;
+      quiet_axes |= 1 << ax;
+      quiet_sum.x += s.SHo.x; quiet_sum.y += s.SHo.y; quiet_sum.z += s.SHo.z;
+    };
     V3<R> Bm[NZ], um[NZ], db[NZ], hod[NZ];
 #pragma unroll
     for (int k = 0; k < NZ; ++k) {
@@ -270,14 +309,18 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
 #pragma unroll
         for (int ax = 0; ax < 2; ++ax) {
           ColSums<R> s{};
-          col_axis<R, OP, PER, HALL, HOD, CONV, SoA<R>, NEED>(s, a, ax, ax == 0 ? ix : iy, ax == 0 ? nx : ny, idx,
-                                                             ax == 0 ? 1 : a.m.px, Bm[k]);
-          col_combine<R, HALL, HOD, CONV>(a, ax, s, Bm[k], um[k], db[k], hod[k]);
+          bool quiet = false;
+          col_axis<R, OP, PER, HALL, HOD, CONV, SoA<R>, NEED, FOF, ADC>(
+              s, a, ax, ax == 0 ? ix : iy, ax == 0 ? nx : ny, idx, ax == 0 ? 1 : a.m.px, Bm[k], &um[k], &quiet);
+          if (ADC) quiet_axis(ax, s, quiet);
+          if (FOF) fo_combine(a.dR, ax, s, fo);
+          col_combine<R, HALL, HOD, CONV, SoA<R>, NEED>(a, ax, s, Bm[k], um[k], db[k], hod[k]);
         }
       }
     }
     // z: shared stencil planes when the whole column uses the interior row
-    const bool stream = cnt == NZ && (PER || (sbp_row(iz0, nz, NB) == NB && sbp_row(iz0 + NZ - 1, nz, NB) == NB));
+    const bool stream =
+        !ADC && !FOF && cnt == NZ && (PER || (sbp_row(iz0, nz, NB) == NB && sbp_row(iz0 + NZ - 1, nz, NB) == NB));
     if (stream) {
       ColSums<R> s[NZ];
 #pragma unroll
@@ -314,15 +357,19 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
         }
       }
 #pragma unroll
-      for (int k = 0; k < NZ; ++k) col_combine<R, HALL, HOD, CONV>(a, 2, s[k], Bm[k], um[k], db[k], hod[k]);
+      for (int k = 0; k < NZ; ++k) col_combine<R, HALL, HOD, CONV, SoA<R>, NEED>(a, 2, s[k], Bm[k], um[k], db[k], hod[k]);
     } else {
 #pragma unroll
       for (int k = 0; k < NZ; ++k) {
         if (k < cnt) {
           const int idx = base + (iz0 + k) * sz;
           ColSums<R> s{};
-          col_axis<R, OP, PER, HALL, HOD, CONV, SoA<R>, NEED>(s, a, 2, iz0 + k, nz, idx, sz, Bm[k]);
-          col_combine<R, HALL, HOD, CONV>(a, 2, s, Bm[k], um[k], db[k], hod[k]);
+          bool quiet = false;
+          col_axis<R, OP, PER, HALL, HOD, CONV, SoA<R>, NEED, FOF, ADC>(s, a, 2, iz0 + k, nz, idx, sz, Bm[k], &um[k],
+                                                                         &quiet);
+          if (ADC) quiet_axis(2, s, quiet);
+          if (FOF) fo_combine(a.dR, 2, s, fo);
+          col_combine<R, HALL, HOD, CONV, SoA<R>, NEED>(a, 2, s, Bm[k], um[k], db[k], hod[k]);
         }
       }
     }
@@ -340,10 +387,17 @@ __global__ void __launch_bounds__(kColThreads, (CONV ? IEQ_COL_CONV_MIN_BLOCKS :
           d.y += a.hod_factor * hv.y;
           d.z += a.hod_factor * hv.z;
         }
-        if (FOAD) {
+        if (FOF) {
+          d.x += fo.x; d.y += fo.y; d.z += fo.z;
+        } else if (FOAD) {
           const int st[3] = {1, a.m.px, sz};
-          const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, PER>(a, ii, nn, st, idx, Bm[k], um[k]);
-          d.x += ds.x; d.y += ds.y; d.z += ds.z;
+          if (quiet_axes != 7) {
+            const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, PER>(a, ii, nn, st, idx, Bm[k], um[k], quiet_axes);
+            d.x += ds.x; d.y += ds.y; d.z += ds.z;
+          }
+          d.x += a.hod_factor * quiet_sum.x;
+          d.y += a.hod_factor * quiet_sum.y;
+          d.z += a.hod_factor * quiet_sum.z;
         }
         stage_epilogue<R, SoA<R>>(a, idx, d);
       }

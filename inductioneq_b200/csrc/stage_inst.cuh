@@ -71,8 +71,11 @@ static void launch_col_ph(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool hod, int c
   // (a flux-form mask compiled in for the default forms measured 3-10 % slower for orders
   // 4 and 6 on B200: the mask stays a run-time value)
   if (foad) {
-    if (conv) launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 1, -1, false, true>, g, b, s, pdl, a);
-    else launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 0, -1, false, true>, g, b, s, pdl, a);
+    if (!conv) launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 0, -1, false, 2>, g, b, s, pdl, a);
+    else if (a.diss_form == 2 && a.need == 10) launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 1, 10, false, 1>, g, b, s, pdl, a);
+    else if (a.diss_form == 2) launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 1, -1, false, 1>, g, b, s, pdl, a);
+    else if (a.need == 10) launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 1, 10, false, 2>, g, b, s, pdl, a);
+    else launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, false, 1, -1, false, 2>, g, b, s, pdl, a);
   } else if (hod && hodp) {
     if (conv) launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, true, 1, -1, true>, g, b, s, pdl, a);
     else launch_pdl(k_stage_col<IEQ_R, IEQ_OP, P, H, true, 0, -1, true>, g, b, s, pdl, a);

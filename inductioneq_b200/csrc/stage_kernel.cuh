@@ -188,27 +188,129 @@ __device__ __forceinline__ void accumulate(AxisSums<R> &s, const StageArgs<R, F>
   }
 }
 
+template <typename R, typename F>
+__device__ __forceinline__ R ldc(const F &f, int j, int comp);
+template <>
+__device__ __forceinline__ double ldc<double, SoA<double>>(const SoA<double> &f, int j, int comp) {
+  return __ldg(f.p + comp * f.s + j);
+}
+template <>
+__device__ __forceinline__ float ldc<float, SoA<float>>(const SoA<float> &f, int j, int comp) {
+  return __ldg(f.p + comp * f.s + j);
+}
+template <>
+__device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f, int j, int comp) {
+  return __ldg(reinterpret_cast<const double *>(f.p + j) + comp);
+}
+template <>
+__device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, int j, int comp) {
+  return __ldg(reinterpret_cast<const float *>(f.p + j) + comp);
+}
+
+// kappa of adaptive dissipation for one pair (include/artificial_dissipation.h:23-45): s =
+// max(|u1|, |u2|) (b1 - b2)^2 against the thresholds of the distance.  The square root runs only
+// between them.  (0 * s carries a NaN, as there.)
+__device__ __forceinline__ double ad_kappa(double s, double lo, double hi, double inv) {
+  if (s >= hi) return 1.0 + 0.0 * s;
+  if (s > lo) return sqrt((s - lo) * inv);
+  return 0.0 * s;
+}
+
+// adaptive dissipation (artificial_dissipation.cl:83-160) of one axis at a node on the interior
+// row, one component at a time (the loop is not unrolled: a warp comes here only where some
+// kappa is not zero, and 60 inlined kappas would crowd out the rest of the kernel's code).  The
+// 2 RI + 1 points serve the first-order part and the high-order part, whose pairs lie within
+// them; the two pairs at the node are in both.
+template <typename R, typename F, int OP, bool PER>
+__device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, int i, int n, int idx, int st) {
+  constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI, WH = Op<OP>::WH;
+  static_assert(WH == RI + 1, "the dissipation pairs lie within the derivative's points");
+  const bool wrap = PER && (i < RI || i >= n - RI);
+  constexpr R sgn = (Op<OP>::ORDER / 2 + 1) % 2 ? (R)-1 : (R)1;
+  const double lo1 = __ldg(&a.tab->ad_lo[ax][1]), hi1 = __ldg(&a.tab->ad_hi[ax][1]), inv1 = __ldg(&a.tab->ad_inv[ax][1]);
+  V3<R> out = {0, 0, 0};
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    R b[2 * RI + 1], u[2 * RI + 1], kf[2 * RI + 1];
+#pragma unroll
+    for (int o = -RI; o <= RI; ++o) {
+      const int j = wrap ? idx + (nbr<true>(i, o, n) - i) * st : idx + o * st;
+      b[o + RI] = ldc<R, F>(a.bk, j, c);
+      u[o + RI] = fabs(ldc<R, F>(a.u, j, c));
+    }
+    // first-order part: sum_k |c_k| kappa max(|u_k|, |u|) (B_k - B) / DX
+    R fo = 0, ho = 0;
+#pragma unroll
+    for (int o = -RI; o <= RI; ++o) {
+      if (o == 0) continue;
+      const int k = o < 0 ? -o : o;
+      const R sg = fmax(u[o + RI], u[RI]), d = b[o + RI] - b[RI];
+      kf[o + RI] = (R)ad_kappa((double)((sg * d) * d), __ldg(&a.tab->ad_lo[ax][k]), __ldg(&a.tab->ad_hi[ax][k]),
+                               __ldg(&a.tab->ad_inv[ax][k]));
+      fo += ((fabs(a.Dint[o + RI]) * kf[o + RI]) * sg) * d;
+    }
+    // high-order part: (1 - kappa) of the pair (e, e - 1) weights the difference that starts
+    // at e - RI (interior row: M_INV = 1, D_HO integer)
+#pragma unroll
+    for (int e = 0; e <= RI; ++e) {
+      R h = 0;
+#pragma unroll
+      for (int k = 0; k < WH; ++k) h += __ldg(&a.tab->DHO[NB][k]) * b[e + k];
+      R kap;
+      if (e == 0) kap = kf[RI - 1];
+      else if (e == 1) kap = kf[RI + 1];
+      else {
+        const R sg = fmax(u[RI + e], u[RI + e - 1]), d = b[RI + e] - b[RI + e - 1];
+        kap = (R)ad_kappa((double)((sg * d) * d), lo1, hi1, inv1);
+      }
+      ho += (((R)1 - kap) * a.hod_factor) * ((__ldg(&a.tab->DHO[NB][e]) * sgn) * h);
+    }
+    const R v = fo / a.dR[ax] + ho;
+    if (c == 0) out.x = v;
+    else if (c == 1) out.y = v;
+    else out.z = v;
+  }
+  return out;
+}
+
+// whether kappa of a pair of points at distance k may differ from zero in any component
+template <typename R>
+__device__ __forceinline__ bool ad_test(const V3<R> &b1, const V3<R> &u1, const V3<R> &b2, const V3<R> &u2, R thr) {
+  const R dx = b1.x - b2.x, dy = b1.y - b2.y, dz = b1.z - b2.z;
+  const R sx = fmax(fabs(u1.x), fabs(u2.x)), sy = fmax(fabs(u1.y), fabs(u2.y)), sz = fmax(fabs(u1.z), fabs(u2.z));
+  return (sx * dx) * dx > thr || (sy * dy) * dy > thr || (sz * dz) * dz > thr;
+}
+
 // first-order / adaptive dissipation (artificial_dissipation.cl:36-160), evaluated as in
-// the reference per stencil point; used only by the DISS_FO_OR_AD instantiation.
+// the reference per stencil point; used only by the DISS_FO_OR_AD instantiation.  Axes in `skip`
+// are left out; adaptive axes on which the whole warp sits on the interior row take ad_axis_full.
+// (Hall periodic 64^3 with a current sheet, adaptive, 4th order, 20 stages: 2.37 ms with every
+// kappa evaluated from the table rows, 0.92 with the interior points loaded once and thresholds
+// from the host, 0.79 with the axes whose kappas are all zero summed in col_axis.)
 template <typename R, typename F, int OP, bool PER>
 __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], const int nn[3],
-                                   const int st[3], int idx, V3<R> Bm, V3<R> um) {
+                                   const int st[3], int idx, V3<R> Bm, V3<R> um, int skip = 0) {
   constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, WH = Op<OP>::WH;
   V3<R> acc = {0, 0, 0};
   const bool adaptive = a.diss_form == 3;
   auto kap = [&](unsigned k, R dx, R b1, R b2, R u1, R u2) -> R {
-    // include/artificial_dissipation.h:23-45 (k*k of the unsigned argument)
-    R s = (fmax(fabs(u1), fabs(u2)) * (b1 - b2)) * (b1 - b2);
+    const R s = (fmax(fabs(u1), fabs(u2)) * (b1 - b2)) * (b1 - b2);
     k = k + (k == 0);
-    double kk = (double)(k * k);
-    double lo = ((kk * a.mp2min) * a.cmin) * (double)dx;
-    double hi = ((kk * a.mp2max) * a.cmax) * (double)dx;
-    double sd = (double)s;
-    double v = ((lo < sd) && (sd < hi)) * sqrt(fabs(sd - lo) / fabs(hi - lo)) + (double)(sd >= hi);
-    return (R)v;
+    const double kk = (double)(k * k);
+    const double lo = ((kk * a.mp2min) * a.cmin) * (double)dx;
+    const double hi = ((kk * a.mp2max) * a.cmax) * (double)dx;
+    const double sd = (double)s;
+    return (R)(((lo < sd) && (sd < hi)) * sqrt(fabs(sd - lo) / fabs(hi - lo)) + (double)(sd >= hi));
   };
+#pragma unroll 1
   for (int ax = 0; ax < 3; ++ax) {
+    if (skip >> ax & 1) continue;
     const int row = PER ? NB : sbp_row(ii[ax], nn[ax], NB);
+    if (adaptive && (PER || warp_on_row(row, NB))) {
+      const V3<R> v = ad_axis_full<R, F, OP, PER>(a, ax, ii[ax], nn[ax], idx, st[ax]);
+      acc.x += v.x; acc.y += v.y; acc.z += v.z;
+      continue;
+    }
     V3<R> tmp = {0, 0, 0};
     for (int c = 0; c < SW; ++c) {
       const int o = c - C0;
@@ -230,28 +332,24 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
       }
     }
     acc.x += tmp.x / a.dR[ax]; acc.y += tmp.y / a.dR[ax]; acc.z += tmp.z / a.dR[ax];
-  }
-  if (adaptive) {
+    if (!adaptive) continue;
     // high-order part weighted by (1 - kappa) of the neighbouring pair
     for (int term = -WH + 1; term <= 0; ++term) {
-      for (int ax = 0; ax < 3; ++ax) {
-        const int row = PER ? NB : sbp_row(ii[ax], nn[ax], NB);
-        const int j1 = idx + (nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
-        const int j2 = idx + (nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
-        const V3<R> b1 = ldf(a.bk, j1), b2 = ldf(a.bk, j2), u1 = ldf(a.u, j1), u2 = ldf(a.u, j2);
-        // diff_HOD (artificial_dissipation.h:58-101) for this start offset
-        const R sgn = (Op<OP>::ORDER / 2 + 1) % 2 ? (R)-1 : (R)1;
-        V3<R> hod = {0, 0, 0};
-        for (int i = 0; i < WH; ++i) {
-          const R coef = ((a.tab->Minv[row] * a.tab->DHO[row][term + WH - 1]) * a.tab->DHO[NB][i]) * sgn;
-          const int j = idx + (nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
-          const V3<R> Bk = ldf(a.bk, j);
-          hod.x += coef * Bk.x; hod.y += coef * Bk.y; hod.z += coef * Bk.z;
-        }
-        acc.x += (((R)1 - kap(1, a.dR[ax], b1.x, b2.x, u1.x, u2.x)) * a.hod_factor) * hod.x;
-        acc.y += (((R)1 - kap(1, a.dR[ax], b1.y, b2.y, u1.y, u2.y)) * a.hod_factor) * hod.y;
-        acc.z += (((R)1 - kap(1, a.dR[ax], b1.z, b2.z, u1.z, u2.z)) * a.hod_factor) * hod.z;
+      const int j1 = idx + (nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
+      const int j2 = idx + (nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
+      const V3<R> b1 = ldf(a.bk, j1), b2 = ldf(a.bk, j2), u1 = ldf(a.u, j1), u2 = ldf(a.u, j2);
+      // diff_HOD (artificial_dissipation.h:58-101) for this start offset
+      const R sgn = (Op<OP>::ORDER / 2 + 1) % 2 ? (R)-1 : (R)1;
+      V3<R> hod = {0, 0, 0};
+      for (int i = 0; i < WH; ++i) {
+        const R coef = ((a.tab->Minv[row] * a.tab->DHO[row][term + WH - 1]) * a.tab->DHO[NB][i]) * sgn;
+        const int j = idx + (nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
+        const V3<R> Bk = ldf(a.bk, j);
+        hod.x += coef * Bk.x; hod.y += coef * Bk.y; hod.z += coef * Bk.z;
       }
+      acc.x += (((R)1 - kap(1, a.dR[ax], b1.x, b2.x, u1.x, u2.x)) * a.hod_factor) * hod.x;
+      acc.y += (((R)1 - kap(1, a.dR[ax], b1.y, b2.y, u1.y, u2.y)) * a.hod_factor) * hod.y;
+      acc.z += (((R)1 - kap(1, a.dR[ax], b1.z, b2.z, u1.z, u2.z)) * a.hod_factor) * hod.z;
     }
   }
   return acc;
@@ -583,25 +681,6 @@ struct CurlArgs {
   R inv_d[3];   // (REAL)(1.0/DX) ...
   R Dint[7];
 };
-
-template <typename R, typename F>
-__device__ __forceinline__ R ldc(const F &f, int j, int comp);
-template <>
-__device__ __forceinline__ double ldc<double, SoA<double>>(const SoA<double> &f, int j, int comp) {
-  return __ldg(f.p + comp * f.s + j);
-}
-template <>
-__device__ __forceinline__ float ldc<float, SoA<float>>(const SoA<float> &f, int j, int comp) {
-  return __ldg(f.p + comp * f.s + j);
-}
-template <>
-__device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f, int j, int comp) {
-  return __ldg(reinterpret_cast<const double *>(f.p + j) + comp);
-}
-template <>
-__device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, int j, int comp) {
-  return __ldg(reinterpret_cast<const float *>(f.p + j) + comp);
-}
 
 // curl(b)/rho.  Each axis contributes the derivatives of the two components orthogonal to
 // it; the derivative rows are multiplied by (REAL)(1/DX) and the curl by 1/rho (within one
