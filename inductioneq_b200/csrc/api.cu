@@ -1,6 +1,7 @@
 // api.cu -- the C ABI of include/inductioneq.h: contexts, the name-dispatched reference
 // kernels, the fused/graph-captured time stepping, device-resident CG cleaning and norms.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -434,8 +435,9 @@ CurlArgs<R, F> curl_args(ieq_ctx *c, F b, const R *rho, F out) {
 }
 
 template <typename R, typename F>
-void launch_curl_any(ieq_ctx *c, F b, const R *rho, F out) {
-  const CurlArgs<R, F> a = curl_args<R, F>(c, b, rho, out);
+void launch_curl_any(ieq_ctx *c, F b, const R *rho, F out, R4<R> *out_aos = nullptr) {
+  CurlArgs<R, F> a = curl_args<R, F>(c, b, rho, out);
+  a.out_aos = out_aos;
   const dim3 g = grid3(c->s.nodes[0], c->s.nodes[1], c->s.nodes[2]), bl = block3();
   const bool per = c->s.periodic;
   switch (c->op_id) {

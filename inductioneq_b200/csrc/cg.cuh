@@ -28,6 +28,7 @@
 // of 3 W additions into three.
 #pragma once
 #include "misc_kernels.cuh"
+#include "stage_kernel.cuh"
 
 namespace ieq {
 
@@ -459,22 +460,23 @@ __global__ void __launch_bounds__(kCgThreads, cg_min_blocks<W>()) k_cg_loop(cons
 // interior one sums its 2 RI points with the coefficients from the parameters; boundary rows
 // load every coefficient and then every value before the first sum (a zero coefficient loads
 // nothing, as in diff_rt).  Rows are multiplied by 1 / DX.
-template <typename R>
+// The field is the caller's records or, in the time loop, the fused state (row pitch px).
+template <typename R, typename F>
 struct CgEndArgs {
-  int nx, ny, nz, off, gx, gy, gz, periodic;
+  int nx, ny, nz, px, off, gx, gy, gz, periodic;
   const double *D;     // derivative (or adjoint) rows [2nb+1][SW]
   double Dint[7];      // the interior row, offsets -RI .. RI
   double inv_d[3];
   double sign;
-  R4<R> *b;
+  F b;
   double *phi, *r, *u0, *u1;
   double *partials;    // of <r, r>, one per block
   CgSync *sync;
 };
 
 // sum_c D[row][c] f(i + c - C0) / DX of one axis; load(o) is the value o nodes along the axis
-template <int OP, typename R, typename Load>
-__device__ __forceinline__ double cg_axis(const CgEndArgs<R> &a, int ax, int i, int n, const Load &load) {
+template <int OP, typename R, typename F, typename Load>
+__device__ __forceinline__ double cg_axis(const CgEndArgs<R, F> &a, int ax, int i, int n, const Load &load) {
   constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, RI = Op<OP>::RI;
   double v = 0.0;
   if (i >= (NB > RI ? NB : RI) && i < n - (NB > RI ? NB : RI)) {
@@ -503,10 +505,9 @@ __device__ __forceinline__ double cg_axis(const CgEndArgs<R> &a, int ax, int i, 
 }
 
 // r = div B on the interior; phi, r outside it and both directions zero; partials of <r, r>
-template <typename R, int OP>
-__global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__ CgEndArgs<R> a) {
+template <typename R, typename F, int OP>
+__global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__ CgEndArgs<R, F> a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) a.sync->arrived = a.sync->released = 0u;
-  const long long plane = (long long)a.nx * a.ny;
   const int lane = threadIdx.x & 31, rows = a.ny * a.nz;
   double rr = 0.0;
   for (int row = blockIdx.x * (kCgThreads / 32) + (threadIdx.x >> 5); row < rows;
@@ -517,10 +518,10 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__
       const long long j = (long long)a.nx * row + ix;
       double v = 0.0;
       if (in_yz && ix >= a.off && ix < a.off + a.gx) {
-        const R *p = reinterpret_cast<const R *>(a.b + j);
-        const double vx = cg_axis<OP>(a, 0, ix, a.nx, [&](int o) { return (double)__ldg(p + 4 * o); });
-        const double vy = cg_axis<OP>(a, 1, iy, a.ny, [&](int o) { return (double)__ldg(p + 4ll * o * a.nx + 1); });
-        const double vz = cg_axis<OP>(a, 2, iz, a.nz, [&](int o) { return (double)__ldg(p + 4ll * o * plane + 2); });
+        const int jb = ix + a.px * row, sy = a.px, sz = a.px * a.ny;
+        const double vx = cg_axis<OP>(a, 0, ix, a.nx, [&](int o) { return (double)ldc<R, F>(a.b, jb + o, 0); });
+        const double vy = cg_axis<OP>(a, 1, iy, a.ny, [&](int o) { return (double)ldc<R, F>(a.b, jb + o * sy, 1); });
+        const double vz = cg_axis<OP>(a, 2, iz, a.nz, [&](int o) { return (double)ldc<R, F>(a.b, jb + o * sz, 2); });
         v = (vx + vy) + vz;
         rr += v * v;
       }
@@ -534,8 +535,19 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__
 }
 
 // B += grad(phi), or B -= grad_adj(phi) (sign = -1, D the adjoint rows), the xyz components
-template <typename R, int OP>
-__global__ void __launch_bounds__(kCgThreads) k_cg_project(const __grid_constant__ CgEndArgs<R> a) {
+template <typename R>
+__device__ __forceinline__ void cg_store_xyz(const AoS<R> &f, int j, V3<R> v) {   // .w untouched, as the
+  R *q = reinterpret_cast<R *>(f.p + j);                                          // reference's .xyz store
+  if constexpr (sizeof(R) == 8) *reinterpret_cast<double2 *>(q) = make_double2(v.x, v.y);
+  else *reinterpret_cast<float2 *>(q) = make_float2(v.x, v.y);
+  q[2] = v.z;
+}
+template <typename R>
+__device__ __forceinline__ void cg_store_xyz(const SoA<R> &f, int j, V3<R> v) {
+  stf(f, j, v);
+}
+template <typename R, typename F, int OP>
+__global__ void __launch_bounds__(kCgThreads) k_cg_project(const __grid_constant__ CgEndArgs<R, F> a) {
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
@@ -545,15 +557,10 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_project(const __grid_constant
   const double gx = cg_axis<OP>(a, 0, ix, a.nx, [&](int o) { return __ldg(p + o); });
   const double gy = cg_axis<OP>(a, 1, iy, a.ny, [&](int o) { return __ldg(p + (long long)o * a.nx); });
   const double gz = cg_axis<OP>(a, 2, iz, a.nz, [&](int o) { return __ldg(p + o * plane); });
-  const V3<R> B = ld3_plain(a.b + j);
-  R *q = reinterpret_cast<R *>(a.b + j);
-  const R bx = (R)((double)B.x + a.sign * gx), by = (R)((double)B.y + a.sign * gy);
-  if constexpr (sizeof(R) == 8) {
-    *reinterpret_cast<double2 *>(q) = make_double2(bx, by);
-  } else {
-    *reinterpret_cast<float2 *>(q) = make_float2(bx, by);
-  }
-  q[2] = (R)((double)B.z + a.sign * gz);   // .w untouched, as the reference's .xyz store
+  const int jb = ix + a.px * (iy + a.ny * iz);
+  const V3<R> B = ldf_plain(a.b, jb);
+  cg_store_xyz(a.b, jb, V3<R>{(R)((double)B.x + a.sign * gx), (R)((double)B.y + a.sign * gy),
+                              (R)((double)B.z + a.sign * gz)});
 }
 
 }  // namespace ieq

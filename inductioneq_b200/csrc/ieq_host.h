@@ -145,6 +145,8 @@ struct ieq_ctx {
   double *d_total = nullptr;       // reduction totals
   unsigned *d_counter = nullptr;   // last-block tickets
   int *d_flag = nullptr;
+  int conv_mark = 0;               // the value slot 1 of d_flag takes if u is not zero (new every call)
+  int last_conv = 1;               // whether the last fused call found u non-zero
   void *d_cg = nullptr;            // CgDevice (the CG loop's state)
   int cg_resident = 0;             // resident blocks of the CG loop kernel (0: not asked yet)
   double *d_cg_vec = nullptr;      // FP64 CG vectors: div, phi, r, u, u', lap (6 x n_pad)

@@ -588,15 +588,6 @@ static __global__ void k_cg_start_loop(const double *partials_rr, int np, CgStat
   }
 }
 
-// any non-zero x/y/z component (decides whether the convection terms can vanish)
-template <typename R>
-__global__ void k_any_nonzero(long long n, const R4<R> *v, int *flag) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const V3<R> x = ld3(v + i);
-  if (x.x != (R)0 || x.y != (R)0 || x.z != (R)0) *flag = 1;
-}
-
 // finiteness check of a vector field (sets *flag if any x/y/z is not finite)
 template <typename R>
 __global__ void k_check_finite(long long n, const R4<R> *v, int *flag) {

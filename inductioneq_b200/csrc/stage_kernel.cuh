@@ -673,6 +673,7 @@ struct CurlArgs {
   F b;
   const R *rho;       // nullptr: plain curl (kernel_operator.cl:158 calc_curl)
   F out;
+  R4<R> *out_aos;     // (k_curl_rho) if set, the output goes here as records of nx per row
   F jface;      // (k_curl_e) J on the faces of a non-periodic box
   F hout;       // (k_curl_e_hod) the dissipation sum of b (sum over the axes of the H rows)
   R Hint[7];    // (k_curl_e_hod) interior dissipation row, offsets -RI..RI
@@ -736,7 +737,8 @@ __global__ void __launch_bounds__(256) k_curl_rho(const __grid_constant__ CurlAr
     const R r = (R)1 / a.rho[idx];
     c = {c.x * r, c.y * r, c.z * r};
   }
-  stf(a.out, idx, c);
+  if (a.out_aos) st3(a.out_aos + (ix + a.m.nx * (iy + a.m.ny * iz)), c);
+  else stf(a.out, idx, c);
 }
 
 // explicit launchers, instantiated per (R, OP) in stage_<r>_o<op>.cu
@@ -747,23 +749,47 @@ void launch_stage(const StageArgs<R, F> &a, bool per, bool hall, int diss, int c
 template <typename R, typename F, int OP>
 void launch_curl(const CurlArgs<R, F> &a, bool per, dim3 grid, dim3 block, cudaStream_t s);
 
-// layout conversion of a vector field between REAL4 AoS and SoA (fused path entry/exit)
+// Vector fields between the caller's REAL4 records and the fused state (entry and exit of the
+// fused calls): every field in one launch, field blockIdx.y.  A field without an output is only
+// looked at.  If field `check` has a non-zero x, y or z (a NaN counts), *flag = mark; the mark
+// changes from call to call, so nothing resets the flag.
+struct StateFlag {
+  int check;   // -1: none
+  int mark;
+  int *flag;
+};
 template <typename R>
-__global__ void k_aos_to_soa(unsigned n, unsigned nx, unsigned px, const R4<R> *in, R *out, long long s) {
+struct StateIo {
+  unsigned n, nx, px;
+  R4<R> *aos[5];
+  R *soa[5];
+  long long s;
+};
+template <typename R>
+__global__ void __launch_bounds__(256) k_state_in(const __grid_constant__ StateIo<R> a, const StateFlag f) {
+  const int k = blockIdx.y;
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const V3<R> v = ld3_plain(in + i);
-  const unsigned j = px == nx ? i : i + i / nx * (px - nx);
-  out[j] = v.x;
-  (out + s)[j] = v.y;
-  (out + 2 * s)[j] = v.z;
+  bool set = false;
+  if (i < a.n) {
+    const V3<R> v = ld3(a.aos[k] + i);
+    if (R *out = a.soa[k]) {
+      const unsigned j = a.px == a.nx ? i : i + i / a.nx * (a.px - a.nx);
+      out[j] = v.x;
+      (out + a.s)[j] = v.y;
+      (out + 2 * a.s)[j] = v.z;
+    }
+    set = v.x != (R)0 || v.y != (R)0 || v.z != (R)0;
+  }
+  if (k == f.check && __syncthreads_or(set) && threadIdx.x == 0 && *(volatile int *)f.flag != f.mark) *f.flag = f.mark;
 }
 template <typename R>
-__global__ void k_soa_to_aos(unsigned n, unsigned nx, unsigned px, const R *in, long long s, R4<R> *out) {
+__global__ void __launch_bounds__(256) k_state_out(const __grid_constant__ StateIo<R> a) {
+  const int k = blockIdx.y;
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned j = px == nx ? i : i + i / nx * (px - nx);
-  st3(out + i, V3<R>{in[j], (in + s)[j], (in + 2 * s)[j]});
+  if (i >= a.n) return;
+  const R *in = a.soa[k];
+  const unsigned j = a.px == a.nx ? i : i + i / a.nx * (a.px - a.nx);
+  st3(a.aos[k] + i, V3<R>{in[j], (in + a.s)[j], (in + 2 * a.s)[j]});
 }
 
 }  // namespace ieq
