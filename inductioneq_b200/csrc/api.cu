@@ -281,7 +281,8 @@ int diss_kind(const Settings &s) {
 
 template <typename R, typename F>
 void launch_stage_any(ieq_ctx *c, const StageArgs<R, F> &a, int conv = -1) {
-  const dim3 g = grid3(c->s.nodes[0], c->s.nodes[1], c->s.nodes[2]), b = block3();
+  const dim3 b(32, 2, 2);   // kStageThreads
+  const dim3 g((c->s.nodes[0] + 31) / 32, (c->s.nodes[1] + 1) / 2, (c->s.nodes[2] + 1) / 2);
   const bool per = c->s.periodic, hall = c->s.hall;
   const int d = diss_kind(c->s);
   switch (c->op_id) {

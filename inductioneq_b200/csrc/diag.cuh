@@ -20,83 +20,94 @@ template <typename R, typename F>
 struct DiagArgs {
   Mesh m;
   F b;
-  long long n;
+  int n;
   const R *wx, *wy, *wz;   // per-axis mass weights (norm2 of kernel_operator.cl)
-  const R *D;              // derivative rows [2nb+1][sw]
-  int nb, sw, periodic;
+  const Tables<R> *tab;    // derivative rows (calc_div)
+  int periodic;
   R dS[3];                 // (REAL)DX ...
   int tc;                  // testcase of analytical_b
-  const R *time;           // analytical_b at time[0]
+  const R *time;           // analytical_b at time[0] ...
+  R t;                     // ... or, without one, at t
 };
 
-// the three terms of node i: energy, divergence, error (each as its reduction kernel forms it)
-template <typename R, typename F>
-__device__ __forceinline__ void diag_terms(const DiagArgs<R, F> &a, long long i, double &e, double &dv, double &er) {
-  const int ix = (int)(i % a.m.nx);
-  const long long r = i / a.m.nx;
-  const int iy = (int)(r % a.m.ny);
-  const int iz = (int)(r / a.m.ny);
-  const R fac = (a.wx[ix] * a.wy[iy]) * a.wz[iz];
-  const long long ib = ix + (long long)a.m.px * r;   // the node in the field's layout
+// d/d(axis) of that axis' component (calc_div, kernel_operator.cl:145): the row's non-zero
+// entries, all loads free to issue before the first sum
+template <typename R, typename F, int OP>
+__device__ __forceinline__ R diag_axis(const DiagArgs<R, F> &a, int ax, int i, int n, int ib, int st) {
+  const int row = a.periodic ? Op<OP>::NB : sbp_row(i, n, Op<OP>::NB);
+  R v = 0;
+#pragma unroll
+  for (int t = 0; t < Op<OP>::ND; ++t) {
+    const R c = __ldg(&a.tab->nd[row][t]);
+    int o = __ldg(&a.tab->nd_off[row][t]);
+    if (a.periodic) o = nbr<true>(i, o, n) - i;
+    R f = 0;
+    if (c != (R)0) f = ldc<R, F>(a.b, ib + o * st, ax);
+    v += c * f;
+  }
+  return v / a.dS[ax];
+}
+
+// the terms of node (ix, iy, iz): energy, divergence, error (each as its reduction kernel forms
+// it); A: analytical_b there, div: div B, fac: the mass weight
+template <typename R, typename F, int OP>
+__device__ __forceinline__ void diag_node(const DiagArgs<R, F> &a, int ix, int iy, int iz, double &e, double &dv,
+                                          double &er, V3<R> &A, R &div, R &fac) {
+  const int ib = ix + a.m.px * (iy + a.m.ny * iz);   // the node in the field's layout
+  fac = (a.wx[ix] * a.wy[iy]) * a.wz[iz];
   const V3<R> B = ldf(a.b, ib);
   e += (double)(fac * ((B.x * B.x + B.y * B.y) + B.z * B.z));
-  // calc_div (kernel_operator.cl:145): sum over the axes of d/d(axis) of that component
-  const int ii[3] = {ix, iy, iz};
-  const int nn[3] = {a.m.nx, a.m.ny, a.m.nz};
-  const long long st[3] = {1, a.m.px, (long long)a.m.px * a.m.ny};
-  const int c0 = (a.sw - 1) / 2;
-  R d[3];
-#pragma unroll
-  for (int ax = 0; ax < 3; ++ax) {
-    const int row = a.periodic ? a.nb : sbp_row(ii[ax], nn[ax], a.nb);
-    R v = 0;
-    for (int c = 0; c < a.sw; ++c) {
-      const R cf = a.D[row * a.sw + c];
-      if (cf == (R)0) continue;
-      const long long j = ib + (long long)(nbr_rt<R>(ii[ax], c - c0, nn[ax], a.periodic) - ii[ax]) * st[ax];
-      v += cf * ldc<R, F>(a.b, j, ax);
-    }
-    d[ax] = v / a.dS[ax];
-  }
-  const R dvg = (d[0] + d[1]) + d[2];
-  dv += (double)((fac * dvg) * dvg);
-  const V3<R> A = b_analytical<R>(a.tc, a.m, ix, iy, iz, a.time[0]);
+  const R dx = diag_axis<R, F, OP>(a, 0, ix, a.m.nx, ib, 1), dy = diag_axis<R, F, OP>(a, 1, iy, a.m.ny, ib, a.m.px),
+          dz = diag_axis<R, F, OP>(a, 2, iz, a.m.nz, ib, a.m.px * a.m.ny);
+  div = (dx + dy) + dz;
+  dv += (double)((fac * div) * div);
+  A = b_analytical<R>(a.tc, a.m, ix, iy, iz, a.time ? a.time[0] : a.t);
   const V3<R> w = {B.x - A.x, B.y - A.y, B.z - A.z};
   er += (double)(fac * ((w.x * w.x + w.y * w.y) + w.z * w.z));
 }
 
-// partials[k * gridDim.x + block], k = 0 energy, 1 divergence, 2 error
-template <typename R, typename F>
-__global__ void __launch_bounds__(256) k_diag_partials(const DiagArgs<R, F> a, double *partials) {
-  __shared__ double sm[3][8];
-  double acc[3] = {0.0, 0.0, 0.0};
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n; i += stride)
-    diag_terms(a, i, acc[0], acc[1], acc[2]);
+// partials[k * gridDim.x + block], k = 0 energy, 1 divergence, 2 error; with `results` also 3 the
+// norm of analytical_b, and analytical_b and div B of every node to va and sdiv
+template <typename R, typename F, int OP>
+__global__ void __launch_bounds__(256) k_diag_partials(const __grid_constant__ DiagArgs<R, F> a, double *partials,
+                                                       int results, R4<R> *va, R *sdiv) {
+  __shared__ double sm[4][8];
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  const unsigned nx = a.m.nx, ny = a.m.ny;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)a.n; i += gridDim.x * blockDim.x) {
+    V3<R> A;
+    R div, fac;
+    diag_node<R, F, OP>(a, i % nx, i / nx % ny, i / nx / ny, acc[0], acc[1], acc[2], A, div, fac);
+    if (results) {
+      acc[3] += (double)(fac * ((A.x * A.x + A.y * A.y) + A.z * A.z));
+      st3(va + i, A);
+      sdiv[i] = div;
+    }
+  }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
+  for (int k = 0; k < 4; ++k) {
     const double v = warp_sum(acc[k]);
     if ((threadIdx.x & 31) == 0) sm[k][threadIdx.x >> 5] = v;
   }
   __syncthreads();
   if (threadIdx.x < 32) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
+    for (int k = 0; k < 4; ++k) {
       double v = threadIdx.x < (blockDim.x >> 5) ? sm[k][threadIdx.x] : 0.0;
       v = warp_sum(v);
-      if (threadIdx.x == 0) partials[k * gridDim.x + blockIdx.x] = v;
+      if (threadIdx.x == 0 && (k < 3 || results)) partials[k * gridDim.x + blockIdx.x] = v;
     }
   }
 }
 
-// the three totals of `np` partials each, in the order of k_reduce_final, appended to
+// the totals of `np` partials each, in the order of k_reduce_final: three appended to
 // series[3 * pos .. 3 * pos + 2] (pos = *count, then incremented; nothing is written past
-// `capacity` entries)
-static __global__ void __launch_bounds__(256) k_diag_final(const double *partials, int np, double *series, int *count,
-                                                    int capacity) {
+// `capacity` entries), or, without a count, `quantities` totals to series[0 ..]
+static __global__ void __launch_bounds__(256) k_diag_final(const double *partials, int np, int quantities,
+                                                           double *series, int *count, int capacity) {
   __shared__ double sm[8];
-  const int pos = *count;
-  for (int k = 0; k < 3; ++k) {
+  const int pos = count ? *count : 0;
+  for (int k = 0; k < quantities; ++k) {
     double acc = 0.0;
     for (int i = threadIdx.x; i < np; i += blockDim.x) acc += partials[k * np + i];
     acc = warp_sum(acc);
@@ -109,7 +120,7 @@ static __global__ void __launch_bounds__(256) k_diag_final(const double *partial
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) *count = pos + 1;
+  if (threadIdx.x == 0 && count) *count = pos + 1;
 }
 
 }  // namespace ieq

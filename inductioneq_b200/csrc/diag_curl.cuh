@@ -6,7 +6,7 @@
 // sqrt(norm2_diff(b, analytical_b(time))).  The first kernel of a Hall step, the curl kernel
 // of stage 1, reads exactly that state -- b at every node and its stencil neighbours -- so
 // k_curl_e_diag forms J = curl(B)/rho, E = J x B (and the dissipation sum) as k_curl_e_hod /
-// k_curl_e do, adds each node's three diagnostic terms (diag_terms: the terms of the stand-
+// k_curl_e do, adds each node's three diagnostic terms (diag_node: the terms of the stand-
 // alone reductions) into per-block partials, and the last block to finish (ticket counter)
 // adds the partials in a fixed order and appends the three totals to the device series.  The
 // step graph then has no launch for the diagnostics.
@@ -64,7 +64,9 @@ __global__ void __launch_bounds__(kColThreads) k_curl_e_diag(const __grid_consta
     if (HODS) stf(a.hout, idx, hod);
     if (!PER && (ix == 0 || iy == 0 || iz == 0 || ix == nx - 1 || iy == ny - 1 || iz == nz - 1))
       stf(a.jface, idx, J);
-    diag_terms(d, ix + (long long)nx * (iy + (long long)ny * iz), acc[0], acc[1], acc[2]);
+    V3<R> A;
+    R div, fac;
+    diag_node<R, SoA<R>, OP>(d, ix, iy, iz, acc[0], acc[1], acc[2], A, div, fac);
   }
   // block partials (whole warps: the launcher gives 128-thread blocks), then the last block
   // adds them in a fixed order

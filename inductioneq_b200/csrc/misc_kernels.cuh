@@ -154,10 +154,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 template <typename T>
 __device__ __forceinline__ double reduce_term(const ReduceArgs<T> &a, long long i) {
   if (a.kind == RED_DOT) return (double)(a.sa[i] * a.sb[i]);
-  const int ix = (int)(i % a.nx);
-  const long long r = i / a.nx;
-  const int iy = (int)(r % a.ny);
-  const int iz = (int)(r / a.ny);
+  const unsigned r = (unsigned)i / a.nx;   // (32-bit division: n < 2^31)
+  const unsigned ix = (unsigned)i - r * a.nx, iz = r / a.ny, iy = r - iz * a.ny;
   const T fac = (a.wx[ix] * a.wy[iy]) * a.wz[iz];
   if (a.kind == RED_NORM2_S) return (double)((fac * a.sa[i]) * a.sa[i]);
   V3<T> v = ld3(a.va + i);

@@ -656,8 +656,15 @@ __device__ __forceinline__ void stage_time_post(const StageArgs<R, F> &a) {
   }
 }
 
+// blocks of 128 threads, five resident (<= 102 registers): at 48^3 the 576 blocks of 256 threads
+// were two waves of two per SM.  Confined Hall 48^3, 4th order, high-order dissipation, two steps
+// as kernel lists and the results: 428 us (433 with four blocks, 440 with six and spills)
+#ifndef IEQ_STAGE_MIN_BLOCKS
+#define IEQ_STAGE_MIN_BLOCKS 5
+#endif
+constexpr int kStageThreads = 128;
 template <typename R, typename F, int OP, bool PER, bool HALL, int DISS, int CONV = -1>
-__global__ void __launch_bounds__(256) k_stage(const __grid_constant__ StageArgs<R, F> a) {
+__global__ void __launch_bounds__(kStageThreads, IEQ_STAGE_MIN_BLOCKS) k_stage(const __grid_constant__ StageArgs<R, F> a) {
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
