@@ -18,14 +18,20 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "ieq_host.h"
 
-#include "stage_kernel.cuh"
+#include "stage_col.cuh"
 
 namespace ieq {
 
+// F: the layout of the fields -- the caller's records (AoS: the public operators and the sweep
+// on the reference kernel lists) or planes at the fused state's pitch (SoA: the checkpointed
+// sweep; a neighbour's value is 6 L1 wavefronts a warp instead of 16, and the stage states are
+// the fused stages' own outputs: Hall 64^3, 20 steps, 5951 -> 3807 us, then 3155 us with the PLAIN kernels below)
+template <typename F>
 struct AdjArgs {
   Mesh m;
   const Tables<double> *tab;
@@ -36,18 +42,20 @@ struct AdjArgs {
   double hod_factor;
   double w[6];           // flux-form weights (see stage_kernel.cuh)
   double inv_d[3], two_inv_d[3], sat_s[3];
-  const R4<double> *b0, *J0, *u, *v, *dJ;   // v: tangent direction or adjoint input w
+  F b0, J0, u, v, dJ;    // v: tangent direction or adjoint input w
   const double *rho;
-  R4<double> *out;
-  R4<double> *gJr;       // vjp pass 1 -> pass 2: (Hall adjoint source for J) / rho
-  // epilogue of the vjp's last kernel (dst != nullptr): dst = eal ex + ebe ey + ega z instead
-  // of out = z (ex, ey may be null; dst may be ex or ey, never v)
-  R4<double> *dst;
-  const R4<double> *ex, *ey;
-  double eal, ebe, ega;
+  F out;
+  F gJr;                 // vjp pass 1 -> pass 2: (Hall adjoint source for J) / rho
+  // epilogue of the vjp's last kernel (dst set): dst = eal ex + ebe ey + ede ew + ega z instead
+  // of out = z (ex, ey, ew may be null; dst may be one of them, never v)
+  F dst, ex, ey, ew;
+  double eal, ebe, ede, ega;
 };
 
-__device__ __forceinline__ V3<double> ld(const R4<double> *p, long long j) { return ld3(p + j); }
+template <typename F>
+__device__ __forceinline__ V3<double> ld(const F &f, int j) {
+  return ldf(f, j);
+}
 __device__ __forceinline__ double comp(V3<double> v, int c) { return c == 0 ? v.x : (c == 1 ? v.y : v.z); }
 __device__ __forceinline__ void addc(V3<double> &v, int c, double x) {
   if (c == 0) v.x += x;
@@ -59,17 +67,27 @@ __device__ __forceinline__ V3<double> axpy3(double a, V3<double> x, V3<double> y
 }
 __device__ __forceinline__ double dot3(V3<double> a, V3<double> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 
+// Blocks of 128 (a block's registers then split an SM finer than 256 threads' do).  PLAIN --
+// periodic Hall stages without dissipation, the default flux forms -- has no wall rows, no SAT
+// and no runtime branches: 96 registers without spills up to order 4, so five blocks an SM; the
+// general kernel and order 6 need 114-128.  Hall 64^3 order 4, a sweep of 20 steps: general
+// kernel 3807 us, PLAIN with 4 / 5 / 6 blocks an SM 3225 / 3155 / 3320 us.
+constexpr int kAdjThreads = 128;
+constexpr int pass1_min_blocks(int ri, bool plain) { return plain && ri < 3 ? 5 : 4; }
+
 struct Node {
   int i[3], n[3];
-  long long st[3], idx;
+  int st[3], idx;
 };
 
-__device__ __forceinline__ int row_of(const AdjArgs &a, int i, int n) {
+template <typename F>
+__device__ __forceinline__ int row_of(const AdjArgs<F> &a, int i, int n) {
   return a.periodic ? a.nb : sbp_row(i, n, a.nb);
 }
 
 // neighbour j = node + o along axis; false if outside a non-periodic grid
-__device__ __forceinline__ bool nbr_idx(const AdjArgs &a, const Node &nd, int ax, int o, long long &j, int &jj) {
+template <typename F>
+__device__ __forceinline__ bool nbr_idx(const AdjArgs<F> &a, const Node &nd, int ax, int o, int &j, int &jj) {
   int t = nd.i[ax] + o;
   if (a.periodic) {
     t += (t < 0) ? nd.n[ax] : 0;
@@ -78,20 +96,20 @@ __device__ __forceinline__ bool nbr_idx(const AdjArgs &a, const Node &nd, int ax
     return false;
   }
   jj = t;
-  j = nd.idx + (long long)(t - nd.i[ax]) * nd.st[ax];
+  j = nd.idx + (t - nd.i[ax]) * nd.st[ax];
   return true;
 }
 
 // forward derivative row at the node: sum_o D[row][o] f(node + o)
-template <typename Fn>
-__device__ V3<double> dfwd(const AdjArgs &a, const Node &nd, int ax, Fn f) {
+template <typename Fn, typename F>
+__device__ V3<double> dfwd(const AdjArgs<F> &a, const Node &nd, int ax, Fn f) {
   const int c0 = (a.sw - 1) / 2;
   const int r = row_of(a, nd.i[ax], nd.n[ax]);
   V3<double> s = {0, 0, 0};
   for (int o = -c0; o <= c0; ++o) {
     const double c = a.tab->D[r][o + c0];
     if (c == 0.0) continue;
-    long long j;
+    int j;
     int jj;
     if (!nbr_idx(a, nd, ax, o, j, jj)) continue;
     s = axpy3(c, f(j), s);
@@ -100,12 +118,12 @@ __device__ V3<double> dfwd(const AdjArgs &a, const Node &nd, int ax, Fn f) {
 }
 
 // transposed derivative at the node: sum_j D[row(j)][node - j] f(j)
-template <typename Fn>
-__device__ V3<double> dtr(const AdjArgs &a, const Node &nd, int ax, Fn f) {
+template <typename Fn, typename F>
+__device__ V3<double> dtr(const AdjArgs<F> &a, const Node &nd, int ax, Fn f) {
   const int c0 = (a.sw - 1) / 2;
   V3<double> s = {0, 0, 0};
   for (int p = -c0; p <= c0; ++p) {
-    long long j;
+    int j;
     int jj;
     if (!nbr_idx(a, nd, ax, p, j, jj)) continue;
     const double c = a.tab->D[row_of(a, jj, nd.n[ax])][c0 - p];
@@ -116,12 +134,12 @@ __device__ V3<double> dtr(const AdjArgs &a, const Node &nd, int ax, Fn f) {
 }
 
 // dissipation row (symmetric use: forward with the row of the node, transpose with rows of j)
-template <bool TR>
-__device__ V3<double> hod_apply(const AdjArgs &a, const Node &nd, int ax, const R4<double> *x) {
+template <bool TR, typename F>
+__device__ V3<double> hod_apply(const AdjArgs<F> &a, const Node &nd, int ax, const F &x) {
   const int h0 = a.wh - 1;
   V3<double> s = {0, 0, 0};
   for (int p = -h0; p <= h0; ++p) {
-    long long j;
+    int j;
     int jj;
     if (!nbr_idx(a, nd, ax, p, j, jj)) continue;
     const double c = TR ? a.tab->H[row_of(a, jj, nd.n[ax])][h0 - p] : a.tab->H[row_of(a, nd.i[ax], nd.n[ax])][h0 + p];
@@ -131,15 +149,16 @@ __device__ V3<double> hod_apply(const AdjArgs &a, const Node &nd, int ax, const 
   return s;
 }
 
-__device__ __forceinline__ bool make_node(const AdjArgs &a, Node &nd) {
+template <typename F>
+__device__ __forceinline__ bool make_node(const AdjArgs<F> &a, Node &nd) {
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= a.m.nx || iy >= a.m.ny || iz >= a.m.nz) return false;
   nd.i[0] = ix; nd.i[1] = iy; nd.i[2] = iz;
   nd.n[0] = a.m.nx; nd.n[1] = a.m.ny; nd.n[2] = a.m.nz;
-  nd.st[0] = 1; nd.st[1] = a.m.nx; nd.st[2] = (long long)a.m.nx * a.m.ny;
-  nd.idx = ix + (long long)a.m.nx * (iy + (long long)a.m.ny * iz);
+  nd.st[0] = 1; nd.st[1] = a.m.px; nd.st[2] = a.m.px * a.m.ny;
+  nd.idx = ix + a.m.px * (iy + a.m.ny * iz);
   return true;
 }
 
@@ -150,14 +169,14 @@ __device__ __forceinline__ bool make_node(const AdjArgs &a, Node &nd) {
 __device__ __forceinline__ V3<double> sigma3(V3<double> p, V3<double> q) {
   return {fmax(fabs(p.x), fabs(q.x)), fmax(fabs(p.y), fabs(q.y)), fmax(fabs(p.z), fabs(q.z))};
 }
-template <bool TR>
-__device__ V3<double> fo_apply(const AdjArgs &a, const Node &nd, int ax, const R4<double> *x) {
+template <bool TR, typename F>
+__device__ V3<double> fo_apply(const AdjArgs<F> &a, const Node &nd, int ax, const F &x) {
   const int c0 = (a.sw - 1) / 2;
   const int rk = row_of(a, nd.i[ax], nd.n[ax]);
   const V3<double> uk = ld(a.u, nd.idx), xk = ld(x, nd.idx);
   V3<double> s = {0, 0, 0}, diag = {0, 0, 0};
   for (int o = -c0; o <= c0; ++o) {
-    long long j;
+    int j;
     int jj;
     if (!nbr_idx(a, nd, ax, o, j, jj)) continue;
     const V3<double> uj = ld(a.u, j);
@@ -197,7 +216,8 @@ __device__ V3<double> fo_apply(const AdjArgs &a, const Node &nd, int ax, const R
 struct KapLin {
   double k, dk;
 };
-__device__ __forceinline__ KapLin kap_lin(const AdjArgs &a, unsigned m, double d, double s) {
+template <typename F>
+__device__ __forceinline__ KapLin kap_lin(const AdjArgs<F> &a, unsigned m, double d, double s) {
   m = m + (m == 0);
   const double kk = (double)(m * m);
   const double lo = ((kk * a.mp2min) * a.cmin) * d;
@@ -211,7 +231,8 @@ __device__ __forceinline__ KapLin kap_lin(const AdjArgs &a, unsigned m, double d
 }
 // sigma (kappa + 2 s kappa') of the pair (p, q) per component: the first-order part's
 // linearised weight (symmetric in the pair)
-__device__ __forceinline__ V3<double> ad_pair_weight(const AdjArgs &a, unsigned m, double d, V3<double> bp,
+template <typename F>
+__device__ __forceinline__ V3<double> ad_pair_weight(const AdjArgs<F> &a, unsigned m, double d, V3<double> bp,
                                                      V3<double> bq, V3<double> up, V3<double> uq) {
   const V3<double> sg = sigma3(up, uq);
   const double dl[3] = {bp.x - bq.x, bp.y - bq.y, bp.z - bq.z};
@@ -228,15 +249,15 @@ __device__ __forceinline__ V3<double> ad_pair_weight(const AdjArgs &a, unsigned 
 
 // the first-order part along ax (times 1/d by the caller): the tangent, or its transpose as
 // fo_apply<true> with the pair weights
-template <bool TR>
-__device__ V3<double> ad_fo_apply(const AdjArgs &a, const Node &nd, int ax, const R4<double> *x) {
+template <bool TR, typename F>
+__device__ V3<double> ad_fo_apply(const AdjArgs<F> &a, const Node &nd, int ax, const F &x) {
   const int c0 = (a.sw - 1) / 2;
   const int rk = row_of(a, nd.i[ax], nd.n[ax]);
   const double d = a.m.d[ax];
   const V3<double> uk = ld(a.u, nd.idx), bk = ld(a.b0, nd.idx), xk = ld(x, nd.idx);
   V3<double> s = {0, 0, 0}, diag = {0, 0, 0};
   for (int o = -c0; o <= c0; ++o) {
-    long long j;
+    int j;
     int jj;
     if (!nbr_idx(a, nd, ax, o, j, jj)) continue;
     const double cf = fabs(a.tab->D[rk][o + c0]);
@@ -261,7 +282,8 @@ __device__ V3<double> ad_fo_apply(const AdjArgs &a, const Node &nd, int ax, cons
 
 // position of node + o along ax with the reference's neighbour rule: periodic wrap, or the
 // node itself outside a box (include/utils.h:89-168)
-__device__ __forceinline__ int ad_pos(const AdjArgs &a, int i, int o, int n) {
+template <typename F>
+__device__ __forceinline__ int ad_pos(const AdjArgs<F> &a, int i, int o, int n) {
   int t = i + o;
   if (a.periodic) {
     t += (t < 0) ? n : 0;
@@ -279,13 +301,14 @@ struct AdTerm {
   int p1, p2;
   V3<double> one_minus_k, dfac, h0;
 };
-__device__ AdTerm ad_term(const AdjArgs &a, const Node &nd, int ax, int ik, long long kidx, int rk, int t) {
+template <typename F>
+__device__ AdTerm ad_term(const AdjArgs<F> &a, const Node &nd, int ax, int ik, int kidx, int rk, int t) {
   const int n = nd.n[ax];
-  const long long st = nd.st[ax];
+  const int st = nd.st[ax];
   AdTerm r;
   r.p1 = ad_pos(a, ik, t + a.wh - 1, n);
   r.p2 = ad_pos(a, ik, t + a.wh - 2, n);
-  const long long j1 = kidx + (long long)(r.p1 - ik) * st, j2 = kidx + (long long)(r.p2 - ik) * st;
+  const int j1 = kidx + (r.p1 - ik) * st, j2 = kidx + (r.p2 - ik) * st;
   const V3<double> b1 = ld(a.b0, j1), b2 = ld(a.b0, j2);
   const V3<double> sg = sigma3(ld(a.u, j1), ld(a.u, j2));
   const double dl[3] = {b1.x - b2.x, b1.y - b2.y, b1.z - b2.z}, sgc[3] = {sg.x, sg.y, sg.z};
@@ -306,7 +329,7 @@ __device__ AdTerm ad_term(const AdjArgs &a, const Node &nd, int ax, int ik, long
     for (int i = 0; i < a.wh; ++i) {
       const double cf = ((a.tab->Minv[rk] * a.tab->DHO[rk][t + a.wh - 1]) * a.tab->DHO[a.nb][i]) * a.hsgn;
       const int pi = ad_pos(a, ik, i + t, n);
-      r.h0 = axpy3(cf, ld(a.b0, kidx + (long long)(pi - ik) * st), r.h0);
+      r.h0 = axpy3(cf, ld(a.b0, kidx + (pi - ik) * st), r.h0);
     }
   }
   return r;
@@ -314,10 +337,10 @@ __device__ AdTerm ad_term(const AdjArgs &a, const Node &nd, int ax, int ik, long
 
 // the high-order part along ax (times hod_factor by the caller): the tangent at the node, or
 // its transpose gathered from every node k whose terms reach the node (k within WH-1 along ax)
-template <bool TR>
-__device__ V3<double> ad_ho_apply(const AdjArgs &a, const Node &nd, int ax, const R4<double> *x) {
+template <bool TR, typename F>
+__device__ V3<double> ad_ho_apply(const AdjArgs<F> &a, const Node &nd, int ax, const F &x) {
   const int n = nd.n[ax], im = nd.i[ax];
-  const long long st = nd.st[ax];
+  const int st = nd.st[ax];
   V3<double> out = {0, 0, 0};
   if (!TR) {
     const int rk = row_of(a, im, n);
@@ -327,9 +350,9 @@ __device__ V3<double> ad_ho_apply(const AdjArgs &a, const Node &nd, int ax, cons
       for (int i = 0; i < a.wh; ++i) {
         const double cf = ((a.tab->Minv[rk] * a.tab->DHO[rk][t + a.wh - 1]) * a.tab->DHO[a.nb][i]) * a.hsgn;
         const int pi = ad_pos(a, im, i + t, n);
-        hv = axpy3(cf, ld(x, nd.idx + (long long)(pi - im) * st), hv);
+        hv = axpy3(cf, ld(x, nd.idx + (pi - im) * st), hv);
       }
-      const V3<double> x1 = ld(x, nd.idx + (long long)(T.p1 - im) * st), x2 = ld(x, nd.idx + (long long)(T.p2 - im) * st);
+      const V3<double> x1 = ld(x, nd.idx + (T.p1 - im) * st), x2 = ld(x, nd.idx + (T.p2 - im) * st);
       out.x += T.one_minus_k.x * hv.x - T.dfac.x * (x1.x - x2.x) * T.h0.x;
       out.y += T.one_minus_k.y * hv.y - T.dfac.y * (x1.y - x2.y) * T.h0.y;
       out.z += T.one_minus_k.z * hv.z - T.dfac.z * (x1.z - x2.z) * T.h0.z;
@@ -345,7 +368,7 @@ __device__ V3<double> ad_ho_apply(const AdjArgs &a, const Node &nd, int ax, cons
     } else if (ik < 0 || ik >= n) {
       continue;
     }
-    const long long kidx = nd.idx + (long long)(ik - im) * st;
+    const int kidx = nd.idx + (ik - im) * st;
     const int rk = row_of(a, ik, n);
     const V3<double> wk = ld(x, kidx);
     for (int t = -a.wh + 1; t <= 0; ++t) {
@@ -375,7 +398,8 @@ __device__ V3<double> ad_ho_apply(const AdjArgs &a, const Node &nd, int ax, cons
 struct HallSat {
   double c, tva, sw, side;
 };
-__device__ __forceinline__ bool hall_sat_axis(const AdjArgs &a, const Node &nd, int ax, V3<double> tv, HallSat &h) {
+template <typename F>
+__device__ __forceinline__ bool hall_sat_axis(const AdjArgs<F> &a, const Node &nd, int ax, V3<double> tv, HallSat &h) {
   const bool l = nd.i[ax] == 0, r = nd.i[ax] == nd.n[ax] - 1;
   if (!l && !r) return false;
   h.c = a.sat_s[ax];
@@ -387,7 +411,8 @@ __device__ __forceinline__ bool hall_sat_axis(const AdjArgs &a, const Node &nd, 
 
 // SAT of the inflow boundary (induction_Eq_surface.cl:7-33): linear in b with the diagonal
 // coefficient sum_a s_a c_a u_a on the faces
-__device__ double sat_diag(const AdjArgs &a, const Node &nd, V3<double> um) {
+template <typename F>
+__device__ double sat_diag(const AdjArgs<F> &a, const Node &nd, V3<double> um) {
   if (a.periodic || a.hall || !a.conv) return 0.0;
   double d = 0.0;
   for (int ax = 0; ax < 3; ++ax) {
@@ -400,24 +425,24 @@ __device__ double sat_diag(const AdjArgs &a, const Node &nd, V3<double> um) {
 }
 
 // tangent linear F'(b0) v; dJ = curl(v)/rho precomputed
-template <bool AD>
-__global__ void k_jvp(const AdjArgs a) {
+template <bool AD, typename F>
+__global__ void k_jvp(const __grid_constant__ AdjArgs<F> a) {
   Node nd;
   if (!make_node(a, nd)) return;
-  const long long k = nd.idx;
+  const int k = nd.idx;
   const V3<double> vm = ld(a.v, k), um = a.conv ? ld(a.u, k) : V3<double>{0, 0, 0};
   V3<double> out = {0, 0, 0};
   for (int ax = 0; ax < 3; ++ax) {
     if (a.conv) {
       // the factored split forms with b -> v (linear in b at fixed u)
-      const V3<double> DuiBa = dfwd(a, nd, ax, [&](long long j) {
+      const V3<double> DuiBa = dfwd(a, nd, ax, [&](int j) {
         const V3<double> uu = ld(a.u, j);
         const double va = comp(ld(a.v, j), ax);
         return V3<double>{uu.x * va, uu.y * va, uu.z * va};
       });
-      const V3<double> DU = dfwd(a, nd, ax, [&](long long j) { return ld(a.u, j); });
-      const V3<double> DV = dfwd(a, nd, ax, [&](long long j) { return ld(a.v, j); });
-      const V3<double> DuaB = dfwd(a, nd, ax, [&](long long j) {
+      const V3<double> DU = dfwd(a, nd, ax, [&](int j) { return ld(a.u, j); });
+      const V3<double> DV = dfwd(a, nd, ax, [&](int j) { return ld(a.v, j); });
+      const V3<double> DuaB = dfwd(a, nd, ax, [&](int j) {
         const V3<double> vv = ld(a.v, j);
         const double ua = comp(ld(a.u, j), ax);
         return V3<double>{ua * vv.x, ua * vv.y, ua * vv.z};
@@ -431,7 +456,7 @@ __global__ void k_jvp(const AdjArgs a) {
     }
     if (a.hall) {
       // D_a[dJ_a b0 + J0_a v - dJ b0_a - J0 v_a]
-      const V3<double> s = dfwd(a, nd, ax, [&](long long j) {
+      const V3<double> s = dfwd(a, nd, ax, [&](int j) {
         const V3<double> b = ld(a.b0, j), J = ld(a.J0, j), v = ld(a.v, j), dJ = ld(a.dJ, j);
         const double dJa = comp(dJ, ax), Ja = comp(J, ax), ba = comp(b, ax), va = comp(v, ax);
         return V3<double>{dJa * b.x + Ja * v.x - dJ.x * ba - J.x * va, dJa * b.y + Ja * v.y - dJ.y * ba - J.y * va,
@@ -459,7 +484,7 @@ __global__ void k_jvp(const AdjArgs a) {
       out.z += h.c * (h.sw * (h.tva * vm.z - dJa * b0.z) + h.side * (va * J0.z + ba * dJ.z));
     }
   }
-  st3(a.out + k, out);
+  stf(a.out, k, out);
 }
 
 // Nodes on which every derivative row involved is the interior row of half-width RI: every
@@ -467,8 +492,8 @@ __global__ void k_jvp(const AdjArgs a) {
 // (no boundary row of a neighbour reaches them).  There D^T at the node gathers d[-p] f(k+p)
 // and D gathers d[p] f(k+p), d the interior row; RI = 0 when the interior row has entries
 // beyond the order's half-width (then every node takes the generic row lookups).
-template <int RI>
-__device__ __forceinline__ bool fast_node(const AdjArgs &a, const Node &nd) {
+template <int RI, typename F>
+__device__ __forceinline__ bool fast_node(const AdjArgs<F> &a, const Node &nd) {
   if (RI == 0) return false;
   if (a.periodic) return true;
   const int lo = a.nb + (a.sw - 1) / 2;
@@ -479,18 +504,19 @@ __device__ __forceinline__ bool fast_node(const AdjArgs &a, const Node &nd) {
 }
 
 // neighbour k + o along ax on the fast path (periodic wrap; interior nodes need none)
-__device__ __forceinline__ long long fnbr(const AdjArgs &a, const Node &nd, int ax, int o) {
+template <bool PER = false, typename F>
+__device__ __forceinline__ int fnbr(const AdjArgs<F> &a, const Node &nd, int ax, int o) {
   int t = nd.i[ax] + o;
-  if (a.periodic) {
+  if (PER || a.periodic) {
     t += (t < 0) ? nd.n[ax] : 0;
     t -= (t >= nd.n[ax]) ? nd.n[ax] : 0;
   }
-  return nd.idx + (long long)(t - nd.i[ax]) * nd.st[ax];
+  return nd.idx + (t - nd.i[ax]) * nd.st[ax];
 }
 
 // the interior row d[o + RI] = D[nb][(SW-1)/2 + o]
-template <int RI>
-__device__ __forceinline__ void interior_row(const AdjArgs &a, double (&d)[2 * RI + 1]) {
+template <int RI, typename F>
+__device__ __forceinline__ void interior_row(const AdjArgs<F> &a, double (&d)[2 * RI + 1]) {
   const int c0 = (a.sw - 1) / 2;
 #pragma unroll
   for (int o = -RI; o <= RI; ++o) d[o + RI] = a.tab->D[a.nb][c0 + o];
@@ -498,7 +524,8 @@ __device__ __forceinline__ void interior_row(const AdjArgs &a, double (&d)[2 * R
 
 // the terms of one axis of F'(b0)^T w at the node from q = D_ax^T w, Du = D_ax u,
 // S3 = D_ax^T (u . w), S5 = D_ax^T (u_ax w)
-__device__ __forceinline__ void pass1_axis(const AdjArgs &a, int ax, V3<double> q, V3<double> Du, double S3,
+template <typename F>
+__device__ __forceinline__ void pass1_axis(const AdjArgs<F> &a, bool hall, int ax, V3<double> q, V3<double> Du, double S3,
                                            V3<double> S5, V3<double> wm, V3<double> um, V3<double> b0m,
                                            V3<double> J0m, V3<double> &z, V3<double> &gJ) {
   if (a.conv) {
@@ -507,7 +534,7 @@ __device__ __forceinline__ void pass1_axis(const AdjArgs &a, int ax, V3<double> 
     for (int i = 0; i < 3; ++i)
       addc(z, i, -a.two_inv_d[ax] * (a.w[3] * ua * comp(q, i) + a.w[4] * comp(S5, i) + a.w[5] * Dua * comp(wm, i)));
   }
-  if (a.hall) {
+  if (hall) {
     const V3<double> Q = {q.x * a.inv_d[ax], q.y * a.inv_d[ax], q.z * a.inv_d[ax]};
     const double J0a = comp(J0m, ax), b0a = comp(b0m, ax);
     z = axpy3(J0a, Q, z);
@@ -517,18 +544,20 @@ __device__ __forceinline__ void pass1_axis(const AdjArgs &a, int ax, V3<double> 
   }
 }
 
-// the vjp's result at node k: out = z, or the epilogue dst = eal ex + ebe ey + ega z (the
-// operation order of k_lincomb)
-__device__ __forceinline__ void vjp_store(const AdjArgs &a, long long k, V3<double> z) {
-  if (!a.dst) {
-    st3(a.out + k, z);
+// the vjp's result at node k: out = z, or the epilogue dst = eal ex + ebe ey + ede ew + ega z
+// (the operation order of k_lincomb)
+template <typename F>
+__device__ __forceinline__ void vjp_store(const AdjArgs<F> &a, int k, V3<double> z) {
+  if (!a.dst.p) {
+    stf(a.out, k, z);
     return;
   }
   V3<double> r = {0, 0, 0};
-  if (a.ex) r = axpy3(a.eal, ld3_plain(a.ex + k), r);
-  if (a.ey) r = axpy3(a.ebe, ld3_plain(a.ey + k), r);
+  if (a.ex.p) r = axpy3(a.eal, ldf_plain(a.ex, k), r);
+  if (a.ey.p) r = axpy3(a.ebe, ldf_plain(a.ey, k), r);
+  if (a.ew.p) r = axpy3(a.ede, ldf_plain(a.ew, k), r);
   r = axpy3(a.ega, z, r);
-  st3(a.dst + k, r);
+  stf(a.dst, k, r);
 }
 
 // F'(b0)^T w, pass 1.  With q_a = D_a^T w (per component), the forward terms transpose to
@@ -539,19 +568,23 @@ __device__ __forceinline__ void vjp_store(const AdjArgs &a, long long k, V3<doub
 //   z_i += J0_a Q_a,i,  z_a -= J0 . Q_a,  and the source for dJ: gJ = sum_a (b0.Q_a) e_a - b0_a Q_a,
 // whose curl transpose (pass 2) adds C^T (gJ / rho).  On fast nodes the four gathers of an
 // axis share one pass over the neighbours (u and w loaded once per neighbour).
-template <int RI, bool AD = false>
-__global__ void k_vjp_pass1(const AdjArgs a) {
+template <int RI, typename F, bool AD = false, bool PLAIN = false>
+__global__ void __launch_bounds__(kAdjThreads, pass1_min_blocks(RI, PLAIN)) k_vjp_pass1(const __grid_constant__ AdjArgs<F> a) {
+  pdl_enter();
+  // D^T(u . w) and D^T(u_a w) have no weight with the default flux forms
+  const bool need3 = !PLAIN && a.w[2] != 0.0, need5 = !PLAIN && a.w[4] != 0.0;
+  const bool hall = PLAIN || a.hall;
   Node nd;
   if (!make_node(a, nd)) return;
-  const long long k = nd.idx;
+  const int k = nd.idx;
   const V3<double> wm = ld(a.v, k), um = a.conv ? ld(a.u, k) : V3<double>{0, 0, 0};
   V3<double> z = {0, 0, 0}, gJ = {0, 0, 0};
   V3<double> b0m = {0, 0, 0}, J0m = {0, 0, 0};
-  if (a.hall) b0m = ld(a.b0, k);
-  if (fast_node<RI>(a, nd)) {
+  if (hall) b0m = ld(a.b0, k);
+  if (PLAIN || fast_node<RI>(a, nd)) {
     double d[2 * RI + 1];
     interior_row<RI>(a, d);
-    if (a.hall) {
+    if (hall) {
       // J0 = curl(b0) / rho at the node (as k_curl_rho: interior rows times 1/d, then 1/rho)
       double g[3][3];
 #pragma unroll
@@ -561,7 +594,7 @@ __global__ void k_vjp_pass1(const AdjArgs a) {
 #pragma unroll
         for (int o = -RI; o <= RI; ++o) {
           if (o == 0) continue;
-          const V3<double> bj = ld(a.b0, fnbr(a, nd, ax, o));
+          const V3<double> bj = ld(a.b0, fnbr<PLAIN>(a, nd, ax, o));
           v1 += d[RI + o] * comp(bj, c1);
           v2 += d[RI + o] * comp(bj, c2);
         }
@@ -580,55 +613,57 @@ __global__ void k_vjp_pass1(const AdjArgs a) {
         const double ct = d[RI - o], cf = d[RI + o];
         V3<double> vj = wm, uj = um;
         if (o != 0) {
-          const long long j = fnbr(a, nd, ax, o);
+          const int j = fnbr<PLAIN>(a, nd, ax, o);
           vj = ld(a.v, j);
           if (a.conv) uj = ld(a.u, j);
         }
         q = axpy3(ct, vj, q);
         if (a.conv) {
           Du = axpy3(cf, uj, Du);
-          S3 += ct * dot3(uj, vj);
-          const double uja = comp(uj, ax);
-          S5 = axpy3(ct, V3<double>{uja * vj.x, uja * vj.y, uja * vj.z}, S5);
+          if (need3) S3 += ct * dot3(uj, vj);
+          if (need5) {
+            const double uja = comp(uj, ax);
+            S5 = axpy3(ct, V3<double>{uja * vj.x, uja * vj.y, uja * vj.z}, S5);
+          }
         }
       }
-      pass1_axis(a, ax, q, Du, S3, S5, wm, um, b0m, J0m, z, gJ);
-      if (a.hod) z = axpy3(a.hod_factor, hod_apply<true>(a, nd, ax, a.v), z);
-      if (a.fo) z = axpy3(a.inv_d[ax], fo_apply<true>(a, nd, ax, a.v), z);
+      pass1_axis(a, hall, ax, q, Du, S3, S5, wm, um, b0m, J0m, z, gJ);
+      if (!PLAIN && a.hod) z = axpy3(a.hod_factor, hod_apply<true>(a, nd, ax, a.v), z);
+      if (!PLAIN && a.fo) z = axpy3(a.inv_d[ax], fo_apply<true>(a, nd, ax, a.v), z);
       if (AD) {
         z = axpy3(a.inv_d[ax], ad_fo_apply<true>(a, nd, ax, a.v), z);
         z = axpy3(a.hod_factor, ad_ho_apply<true>(a, nd, ax, a.v), z);
       }
     }
   } else {
-    if (a.hall) J0m = ld(a.J0, k);
+    if (hall) J0m = ld(a.J0, k);
     for (int ax = 0; ax < 3; ++ax) {
-      const V3<double> q = dtr(a, nd, ax, [&](long long j) { return ld(a.v, j); });
+      const V3<double> q = dtr(a, nd, ax, [&](int j) { return ld(a.v, j); });
       V3<double> Du = {0, 0, 0}, S5 = {0, 0, 0};
       double S3 = 0.0;
       if (a.conv) {
-        Du = dfwd(a, nd, ax, [&](long long j) { return ld(a.u, j); });
-        S3 = dtr(a, nd, ax, [&](long long j) {
+        Du = dfwd(a, nd, ax, [&](int j) { return ld(a.u, j); });
+        S3 = dtr(a, nd, ax, [&](int j) {
           const double s = dot3(ld(a.u, j), ld(a.v, j));
           return V3<double>{s, 0, 0};
         }).x;
-        S5 = dtr(a, nd, ax, [&](long long j) {
+        S5 = dtr(a, nd, ax, [&](int j) {
           const double ua = comp(ld(a.u, j), ax);
           const V3<double> ww = ld(a.v, j);
           return V3<double>{ua * ww.x, ua * ww.y, ua * ww.z};
         });
       }
-      pass1_axis(a, ax, q, Du, S3, S5, wm, um, b0m, J0m, z, gJ);
-      if (a.hod) z = axpy3(a.hod_factor, hod_apply<true>(a, nd, ax, a.v), z);
-      if (a.fo) z = axpy3(a.inv_d[ax], fo_apply<true>(a, nd, ax, a.v), z);
+      pass1_axis(a, hall, ax, q, Du, S3, S5, wm, um, b0m, J0m, z, gJ);
+      if (!PLAIN && a.hod) z = axpy3(a.hod_factor, hod_apply<true>(a, nd, ax, a.v), z);
+      if (!PLAIN && a.fo) z = axpy3(a.inv_d[ax], fo_apply<true>(a, nd, ax, a.v), z);
       if (AD) {
         z = axpy3(a.inv_d[ax], ad_fo_apply<true>(a, nd, ax, a.v), z);
         z = axpy3(a.hod_factor, ad_ho_apply<true>(a, nd, ax, a.v), z);
       }
     }
   }
-  z = axpy3(sat_diag(a, nd, um), wm, z);
-  if (a.hall && !a.periodic) {
+  if (!PLAIN) z = axpy3(sat_diag(a, nd, um), wm, z);
+  if (hall && !(PLAIN || a.periodic)) {
     // transpose of the Hall outflow SAT's tangent: the terms in v at the node, and the source
     // for dJ (transposed through the curl by pass 2 with the Hall volume term's)
     const V3<double> tv = {0.5 * um.x - J0m.x, 0.5 * um.y - J0m.y, 0.5 * um.z - J0m.z};
@@ -642,23 +677,24 @@ __global__ void k_vjp_pass1(const AdjArgs a) {
       gJ = axpy3(h.c * h.side * comp(b0m, ax), wm, gJ);
     }
   }
-  if (a.hall) {
-    st3(a.out + k, z);
+  if (hall) {
+    stf(a.out, k, z);
     const double r = 1.0 / a.rho[k];
-    st3(a.gJr + k, V3<double>{gJ.x * r, gJ.y * r, gJ.z * r});
+    stf(a.gJr, k, V3<double>{gJ.x * r, gJ.y * r, gJ.z * r});
   } else {
     vjp_store(a, k, z);
   }
 }
 
 // pass 2: z += C^T g with C the SBP curl (rows / d), g = gJ / rho
-template <int RI>
-__global__ void k_vjp_pass2(const AdjArgs a) {
+template <int RI, typename F, bool PER = false>
+__global__ void __launch_bounds__(kAdjThreads, 8) k_vjp_pass2(const __grid_constant__ AdjArgs<F> a) {
+  pdl_enter();
   Node nd;
   if (!make_node(a, nd)) return;
-  const long long k = nd.idx;
+  const int k = nd.idx;
   V3<double> g[3];
-  if (fast_node<RI>(a, nd)) {
+  if (PER || fast_node<RI>(a, nd)) {
     double d[2 * RI + 1];
     interior_row<RI>(a, d);
     const V3<double> gm = ld(a.gJr, k);
@@ -666,17 +702,17 @@ __global__ void k_vjp_pass2(const AdjArgs a) {
     for (int ax = 0; ax < 3; ++ax) {
       V3<double> t = {0, 0, 0};
 #pragma unroll
-      for (int o = -RI; o <= RI; ++o) t = axpy3(d[RI - o], o == 0 ? gm : ld(a.gJr, fnbr(a, nd, ax, o)), t);
+      for (int o = -RI; o <= RI; ++o) t = axpy3(d[RI - o], o == 0 ? gm : ld(a.gJr, fnbr<PER>(a, nd, ax, o)), t);
       g[ax] = {t.x * a.inv_d[ax], t.y * a.inv_d[ax], t.z * a.inv_d[ax]};
     }
   } else {
     for (int ax = 0; ax < 3; ++ax) {
-      const V3<double> t = dtr(a, nd, ax, [&](long long j) { return ld(a.gJr, j); });
+      const V3<double> t = dtr(a, nd, ax, [&](int j) { return ld(a.gJr, j); });
       g[ax] = {t.x * a.inv_d[ax], t.y * a.inv_d[ax], t.z * a.inv_d[ax]};   // (D_ax^T g_c) / d_ax
     }
   }
   // (C^T g)_x = Dz^T g_y - Dy^T g_z, (C^T g)_y = Dx^T g_z - Dz^T g_x, (C^T g)_z = Dy^T g_x - Dx^T g_y
-  V3<double> z = ld3_plain(a.out + k);
+  V3<double> z = ldf_plain(a.out, k);
   z.x += g[2].y - g[1].z;
   z.y += g[0].z - g[2].x;
   z.z += g[1].x - g[0].y;
@@ -684,15 +720,15 @@ __global__ void k_vjp_pass2(const AdjArgs a) {
 }
 
 // out = alpha*x + beta*y (+ gamma*z) over the nodes (x, y, z may be the same array as out)
-__global__ void k_lincomb(long long n, R4<double> *out, double al, const R4<double> *x, double be,
-                          const R4<double> *y, double ga, const R4<double> *z) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+template <typename F>
+__global__ void k_lincomb(int n, F out, double al, F x, double be, F y, double ga, F z) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   V3<double> r = {0, 0, 0};
-  if (x) r = axpy3(al, ld3_plain(x + i), r);
-  if (y) r = axpy3(be, ld3_plain(y + i), r);
-  if (z) r = axpy3(ga, ld3_plain(z + i), r);
-  st3(out + i, r);
+  if (x.p) r = axpy3(al, ldf_plain(x, i), r);
+  if (y.p) r = axpy3(be, ldf_plain(y, i), r);
+  if (z.p) r = axpy3(ga, ldf_plain(z, i), r);
+  stf(out, i, r);
 }
 
 }  // namespace ieq
@@ -702,17 +738,24 @@ using namespace ieq;
 namespace ieq {
 // from api.cu
 ieq_status adj_run_kernel(ieq_ctx *c, const char *name, void *const *args, int nargs);
-void adj_curl(ieq_ctx *c, const void *b, const void *rho, void *out);
+void adj_curl(ieq_ctx *c, AoS<double> b, const void *rho, AoS<double> out);
+void adj_curl(ieq_ctx *c, SoA<double> b, const void *rho, SoA<double> out);
+void adj_calc_u(ieq_ctx *c, AoS<double> u, double t);
+void adj_calc_u(ieq_ctx *c, SoA<double> u, double t);
 void rk2n_coefficients(bool ck, const double **A, const double **B, const double **C, int *stages);
 void adj_context(ieq_ctx *c, Mesh &m, const Tables<double> *&tab, double w[6], double inv_d[3], double two_inv_d[3],
                  double sat_s[3]);
 // from api_fused.inc
-ieq_status adj_fused_steps(ieq_ctx *c, int conv, void *b, void *b2, void *b3, void *cb, void *u, const void *rho,
-                           void *time, int nsteps, void *const *keep, int P);
-ieq_status adj_read_conv(ieq_ctx *c, const void *u, int &conv);
+ieq_status adj_state_begin(ieq_ctx *c, const void *b0, const void *u, const void *rho, int &conv, SoA<double> &b,
+                           SoA<double> &us, const double *&rhos);
+ieq_status adj_state_steps(ieq_ctx *c, int conv, const double *from, const void *rho, double *time, int nsteps,
+                           double *const *keep, int P, double *&end);
+void adj_to_soa(ieq_ctx *c, const void *aos, SoA<double> f);
+void adj_to_aos(ieq_ctx *c, SoA<double> f, void *aos);
 
-AdjArgs adj_args(ieq_ctx *c) {
-  AdjArgs a;
+template <typename F>
+AdjArgs<F> adj_args(ieq_ctx *c) {
+  AdjArgs<F> a;
   std::memset(&a, 0, sizeof(a));
   adj_context(c, a.m, a.tab, a.w, a.inv_d, a.two_inv_d, a.sat_s);
   a.nb = c->op.nb;
@@ -730,6 +773,7 @@ AdjArgs adj_args(ieq_ctx *c) {
   a.cmax = c->s.cmax;
   a.hsgn = ((c->op.order / 2 + 1) % 2) ? -1.0 : 1.0;
   a.hod_factor = c->s.hod_factor;
+  if (std::is_same<F, SoA<double>>::value) a.m.px = c->px;
   return a;
 }
 }  // namespace ieq
@@ -756,13 +800,22 @@ int fast_ri(const ieq_ctx *c) {
   return ri;
 }
 
-dim3 ablock() { return dim3(32, 4, 2); }
+dim3 ablock() { return dim3(32, 2, 2); }   // kAdjThreads
 dim3 agrid(const ieq_ctx *c) {
-  return dim3((c->s.nodes[0] + 31) / 32, (c->s.nodes[1] + 3) / 4, (c->s.nodes[2] + 1) / 2);
+  return dim3((c->s.nodes[0] + 31) / 32, (c->s.nodes[1] + 1) / 2, (c->s.nodes[2] + 1) / 2);
 }
-
-struct Work {
-  void *J0 = nullptr, *dJ = nullptr, *gJr = nullptr;
+// a vector field in layout F over n elements a component
+template <typename F>
+struct MakeField;
+template <>
+struct MakeField<AoS<double>> {
+  static AoS<double> of(const ieq_ctx *, const void *p) { return {(R4<double> *)p}; }
+  static int nodes(const ieq_ctx *c) { return (int)c->n; }
+};
+template <>
+struct MakeField<SoA<double>> {
+  static SoA<double> of(const ieq_ctx *c, const void *p) { return {(double *)p, (long long)c->soa_n, 0}; }
+  static int nodes(const ieq_ctx *c) { return c->px * c->s.nodes[1] * c->s.nodes[2]; }
 };
 
 ieq_status work_alloc(ieq_ctx *c, std::vector<void *> &bufs, int n, size_t bytes) {
@@ -780,114 +833,131 @@ void free_all(std::vector<void *> &bufs) {
   bufs.clear();
 }
 
-// out = F'(b)^T w (u at the stage time, rho); J0, gJr: work fields
-// optional epilogue of vjp: dst = al x + be y + ga F'(b)^T w (x, y may be null)
+// optional epilogue of vjp: dst = al x + be y + de w + ga F'(b)^T w (x, y, w may be null)
+template <typename F>
 struct Epi {
-  void *dst = nullptr;
-  const void *x = nullptr, *y = nullptr;
-  double al = 0, be = 0, ga = 0;
+  F dst{}, x{}, y{}, w{};
+  double al = 0, be = 0, de = 0, ga = 0;
 };
 
-ieq_status vjp(ieq_ctx *c, const void *b, const void *w, const void *u, const void *rho, void *out, void *J0,
-               void *gJr, const Epi &epi = Epi()) {
-  AdjArgs a = adj_args(c);
-  a.dst = (R4<double> *)epi.dst;
-  a.ex = (const R4<double> *)epi.x;
-  a.ey = (const R4<double> *)epi.y;
+// out = F'(b)^T w (u at the stage time, rho); J0, gJr: work fields
+template <typename F>
+ieq_status vjp(ieq_ctx *c, F b, F w, F u, const void *rho, F out, F J0, F gJr, const Epi<F> &epi = Epi<F>()) {
+  AdjArgs<F> a = adj_args<F>(c);
+  a.dst = epi.dst;
+  a.ex = epi.x;
+  a.ey = epi.y;
+  a.ew = epi.w;
   a.eal = epi.al;
   a.ebe = epi.be;
+  a.ede = epi.de;
   a.ega = epi.ga;
-  a.b0 = (const R4<double> *)b;
-  a.u = (const R4<double> *)u;
-  a.v = (const R4<double> *)w;
+  a.b0 = b;
+  a.u = u;
+  a.v = w;
   a.rho = (const double *)rho;
-  a.out = (R4<double> *)out;
-  a.gJr = (R4<double> *)gJr;
+  a.out = out;
+  a.gJr = gJr;
   // adaptive dissipation: its own instantiation of pass 1, generic rows on every node (the
   // terms of its linearisation would raise the other instantiations' registers)
   const int ri1 = a.ad ? 0 : fast_ri(c);
   if (c->s.hall && (!c->s.periodic || ri1 == 0)) {   // else pass 1 forms J0 at every node itself
     adj_curl(c, b, rho, J0);
-    a.J0 = (const R4<double> *)J0;
+    a.J0 = J0;
   }
-  switch (a.ad ? -1 : ri1) {
-    case -1: k_vjp_pass1<0, true><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-    case 1: k_vjp_pass1<1><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-    case 2: k_vjp_pass1<2><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-    case 3: k_vjp_pass1<3><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-    default: k_vjp_pass1<0><<<agrid(c), ablock(), 0, c->stream>>>(a);
+  const dim3 g = agrid(c), bl = ablock();
+  const bool pdl = c->s.pdl;
+  // the instantiations without walls, SAT and runtime branches (measured at kAdjThreads)
+  const bool plain = c->s.periodic && c->s.hall && !a.hod && !a.fo && !a.ad && a.w[2] == 0.0 && a.w[4] == 0.0;
+  switch (a.ad ? -1 : ri1 + (plain && ri1 ? 3 : 0)) {
+    case -1: launch_pdl(k_vjp_pass1<0, F, true>, g, bl, c->stream, pdl, a); break;
+    case 1: launch_pdl(k_vjp_pass1<1, F>, g, bl, c->stream, pdl, a); break;
+    case 2: launch_pdl(k_vjp_pass1<2, F>, g, bl, c->stream, pdl, a); break;
+    case 3: launch_pdl(k_vjp_pass1<3, F>, g, bl, c->stream, pdl, a); break;
+    case 4: launch_pdl(k_vjp_pass1<1, F, false, true>, g, bl, c->stream, pdl, a); break;
+    case 5: launch_pdl(k_vjp_pass1<2, F, false, true>, g, bl, c->stream, pdl, a); break;
+    case 6: launch_pdl(k_vjp_pass1<3, F, false, true>, g, bl, c->stream, pdl, a); break;
+    default: launch_pdl(k_vjp_pass1<0, F>, g, bl, c->stream, pdl, a);
   }
   if (c->s.hall) {
-    switch (fast_ri(c)) {
-      case 1: k_vjp_pass2<1><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-      case 2: k_vjp_pass2<2><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-      case 3: k_vjp_pass2<3><<<agrid(c), ablock(), 0, c->stream>>>(a); break;
-      default: k_vjp_pass2<0><<<agrid(c), ablock(), 0, c->stream>>>(a);
+    const int ri2 = fast_ri(c);
+    switch (ri2 + (c->s.periodic && ri2 ? 3 : 0)) {
+      case 1: launch_pdl(k_vjp_pass2<1, F>, g, bl, c->stream, pdl, a); break;
+      case 2: launch_pdl(k_vjp_pass2<2, F>, g, bl, c->stream, pdl, a); break;
+      case 3: launch_pdl(k_vjp_pass2<3, F>, g, bl, c->stream, pdl, a); break;
+      case 4: launch_pdl(k_vjp_pass2<1, F, true>, g, bl, c->stream, pdl, a); break;
+      case 5: launch_pdl(k_vjp_pass2<2, F, true>, g, bl, c->stream, pdl, a); break;
+      case 6: launch_pdl(k_vjp_pass2<3, F, true>, g, bl, c->stream, pdl, a); break;
+      default: launch_pdl(k_vjp_pass2<0, F>, g, bl, c->stream, pdl, a);
     }
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? IEQ_OK : afail(c, IEQ_ERR_CUDA, cudaGetErrorString(e));
 }
 
-void lincomb(ieq_ctx *c, void *out, double al, const void *x, double be, const void *y, double ga = 0,
-             const void *z = nullptr) {
-  const long long n = (long long)c->n;
-  k_lincomb<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, (R4<double> *)out, al, (const R4<double> *)x, be,
-                                                               (const R4<double> *)y, ga, (const R4<double> *)z);
+template <typename F>
+void lincomb(ieq_ctx *c, F out, double al, F x, double be, F y, double ga = 0, F z = F{}) {
+  const int n = MakeField<F>::nodes(c);
+  k_lincomb<F><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, out, al, x, be, y, ga, z);
 }
 
-// u at stage time t (calc_u with time[1] = t) into `uw`, or the caller's u
-const void *stage_u(ieq_ctx *c, const void *u, void *uw, double *d_time, double t) {
-  if (!c->s.variable_u) return u;
-  double tt[2] = {t, t};
-  cudaMemcpyAsync(d_time, tt, sizeof(tt), cudaMemcpyHostToDevice, c->stream);
-  void *args[7] = {uw, uw, uw, uw, uw, uw, d_time};   // calc_u_3_args reads u (4) and time (6)
-  adj_run_kernel(c, "calc_u_3_args", args, 7);
-  return uw;
-}
-
-// work fields of one SSPRK33 step adjoint, allocated once per call of the public entry
-// points (the checkpointed sweep reuses them for every step)
+// work fields of one step adjoint, allocated once per call of the public entry points (the
+// checkpointed sweep reuses them for every step): J0, gJr, z, l1, l2, l3, and u at the last two
+// stage times (a step's first stage time is its predecessor's last)
+template <typename F>
 struct VjpWork {
-  std::vector<void *> f;   // J0, gJr, z, l1, l2, l3, uw
-  double *d_time = nullptr;
+  F J0{}, gJr{}, z{}, l1{}, l2{}, l3{}, uw[2]{};
+  double ut[2] = {std::nan(""), std::nan("")};
+  int last = 0;
 };
-
-ieq_status vjp_work_alloc(ieq_ctx *c, VjpWork &w) {
-  ieq_status st = work_alloc(c, w.f, 7, c->n_pad * sizeof(R4<double>));
-  if (st == IEQ_OK && cudaMalloc(&w.d_time, 2 * sizeof(double)) != cudaSuccess)
-    st = afail(c, IEQ_ERR_CUDA, "adjoint work allocation");
-  return st;
+constexpr int kVjpFields = 8;
+template <typename F>
+VjpWork<F> vjp_work(const ieq_ctx *c, void *const *f) {
+  VjpWork<F> w;
+  F *to[kVjpFields] = {&w.J0, &w.gJr, &w.z, &w.l1, &w.l2, &w.l3, &w.uw[0], &w.uw[1]};
+  for (int k = 0; k < kVjpFields; ++k) *to[k] = MakeField<F>::of(c, f[k]);
+  return w;
 }
 
-void vjp_work_free(VjpWork &w) {
-  free_all(w.f);
-  if (w.d_time) cudaFree(w.d_time);
-  w.d_time = nullptr;
+// u at stage time t (calc_u with time[1] = t), or the caller's u
+template <typename F>
+F stage_u(ieq_ctx *c, F u, VjpWork<F> &w, double t) {
+  if (!c->s.variable_u) return u;
+  for (int k = 0; k < 2; ++k)
+    if (w.ut[k] == t) {
+      w.last = k;
+      return w.uw[k];
+    }
+  w.last ^= 1;   // the older of the two makes room
+  w.ut[w.last] = t;
+  adj_calc_u(c, w.uw[w.last], t);
+  return w.uw[w.last];
 }
 
 // lambda <- (d step / d s1)^T lambda for the SSPRK33 step with stage states s1, s2, s3 that
 // started at time t0; enqueued on the context's stream, no allocation, no synchronisation
-ieq_status ssprk33_step_vjp_ws(ieq_ctx *c, const void *s1, const void *s2, const void *s3, double t0, void *lambda,
-                               const void *u, const void *rho, const VjpWork &w) {
-  void *J0 = w.f[0], *gJr = w.f[1], *z = w.f[2], *l1 = w.f[3], *l2 = w.f[4], *l3 = w.f[5], *uw = w.f[6];
-  double *d_time = w.d_time;
+template <typename F>
+ieq_status ssprk33_step_vjp_ws(ieq_ctx *c, F s1, F s2, F s3, double t0, F lambda, F u, const void *rho, VjpWork<F> &w) {
   const double h = c->s.dt;
   const double t2 = t0 + h, t3 = t0 + 0.5 * h;   // SSPRK33_2a / _3a
   ieq_status st;
   // the combinations with F'^T are the vjp's epilogue
-  Epi e;
   // stage 3: lambda3 = 2/3 (lambda + h F'(s3)^T lambda); lambda1 = 1/3 lambda
-  e.dst = l3; e.x = lambda; e.al = 2.0 / 3.0; e.ga = 2.0 / 3.0 * h;
-  if ((st = vjp(c, s3, lambda, stage_u(c, u, uw, d_time, t3), rho, z, J0, gJr, e)) != IEQ_OK) return st;
-  lincomb(c, l1, 1.0 / 3.0, lambda, 0.0, nullptr);
+  Epi<F> e3;
+  e3.dst = w.l3; e3.x = lambda; e3.al = 2.0 / 3.0; e3.ga = 2.0 / 3.0 * h;
+  if ((st = vjp(c, s3, lambda, stage_u(c, u, w, t3), rho, w.z, w.J0, w.gJr, e3)) != IEQ_OK) return st;
   // stage 2: lambda2 = 1/4 (lambda3 + h F'(s2)^T lambda3); lambda1 += 3/4 lambda3
-  e.dst = l2; e.x = l3; e.al = 0.25; e.ga = 0.25 * h;
-  if ((st = vjp(c, s2, l3, stage_u(c, u, uw, d_time, t2), rho, z, J0, gJr, e)) != IEQ_OK) return st;
-  lincomb(c, l1, 1.0, l1, 0.75, l3);
+  Epi<F> e2;
+  e2.dst = w.l2; e2.x = w.l3; e2.al = 0.25; e2.ga = 0.25 * h;
+  if ((st = vjp(c, s2, w.l3, stage_u(c, u, w, t2), rho, w.z, w.J0, w.gJr, e2)) != IEQ_OK) return st;
   // stage 1: lambda1 += lambda2 + h F'(s1)^T lambda2
-  e.dst = lambda; e.x = l1; e.y = l2; e.al = 1.0; e.be = 1.0; e.ga = h;
-  return vjp(c, s1, l2, stage_u(c, u, uw, d_time, t0), rho, z, J0, gJr, e);
+  Epi<F> e1;
+  e1.dst = lambda;
+  e1.x = lambda; e1.al = 1.0 / 3.0;
+  e1.y = w.l3; e1.be = 0.75;
+  e1.w = w.l2; e1.de = 1.0;
+  e1.ga = h;
+  return vjp(c, s1, w.l2, stage_u(c, u, w, t0), rho, w.z, w.J0, w.gJr, e1);
 }
 
 // lambda <- (d step / d b_n)^T lambda for one step of a 2N low-storage scheme
@@ -898,22 +968,24 @@ ieq_status ssprk33_step_vjp_ws(ieq_ctx *c, const void *s1, const void *s2, const
 // A_0 = 0, so b2 after a step does not reach the next):
 //   mu2 += B_s mu1;  mu1 += h F'(x[s], t_s)^T mu2;  mu2 = A_s mu2      (s = S-1 .. 0)
 // (the scaling by A_s and the next stage's B_{s-1} mu1 in one pass; mu1 += h F'^T mu2 as the
-// vjp's epilogue).  w.f[3] holds mu2; no allocation, no synchronisation
-ieq_status rk2n_step_vjp_ws(ieq_ctx *c, bool ck, void *const *x, double t0, void *lambda, const void *u,
-                            const void *rho, const VjpWork &w) {
-  void *J0 = w.f[0], *gJr = w.f[1], *z = w.f[2], *mu2 = w.f[3], *uw = w.f[6];
+// vjp's epilogue).  w.l1 holds mu2; no allocation, no synchronisation
+template <typename F>
+ieq_status rk2n_step_vjp_ws(ieq_ctx *c, bool ck, void *const *x, double t0, F lambda, F u, const void *rho,
+                            VjpWork<F> &w) {
+  const F mu2 = w.l1;
   const double *A, *B, *C;
   int S;
   rk2n_coefficients(ck, &A, &B, &C, &S);
   const double h = c->s.dt;
   ieq_status st;
-  Epi e;
+  Epi<F> e;
   e.dst = lambda; e.x = lambda; e.al = 1.0; e.ga = h;
   for (int s = S - 1; s >= 0; --s) {
     const double ts = s == 0 ? t0 : t0 + C[s - 1] * h;
-    if (s == S - 1) lincomb(c, mu2, B[s], lambda, 0.0, nullptr);   // mu2 = 0 + B_s mu1
-    else lincomb(c, mu2, A[s + 1], mu2, B[s], lambda);             // A_{s+1} mu2 + B_s mu1
-    if ((st = vjp(c, x[s], mu2, stage_u(c, u, uw, w.d_time, ts), rho, z, J0, gJr, e)) != IEQ_OK) return st;
+    if (s == S - 1) lincomb(c, mu2, B[s], lambda, 0.0, F{});   // mu2 = 0 + B_s mu1
+    else lincomb(c, mu2, A[s + 1], mu2, B[s], lambda);         // A_{s+1} mu2 + B_s mu1
+    if ((st = vjp(c, MakeField<F>::of(c, x[s]), mu2, stage_u(c, u, w, ts), rho, w.z, w.J0, w.gJr, e)) != IEQ_OK)
+      return st;
   }
   return IEQ_OK;
 }
@@ -925,36 +997,36 @@ ieq_status rk2n_step_vjp_ws(ieq_ctx *c, bool ck, void *const *x, double t0, void
 // (t = L[dst]; L[dst] = a[dst] t; L[r] += a[r] t for r != dst; LK += k t), then the stage's
 // evaluation K = h F(R[src]) transposed: L[src] += h F'(x)^T LK (the vjp's epilogue).
 // No allocation, no synchronisation
-ieq_status program_step_vjp_ws(ieq_ctx *c, const RkProgram &prog, void *const *x, double t0, void *lambda,
-                               const void *u, const void *rho, const VjpWork &w, void *L1, void *L2, void *LK,
-                               void *tmp) {
-  void *J0 = w.f[0], *gJr = w.f[1], *z = w.f[2], *uw = w.f[6];
-  void *L[3] = {lambda, L1, L2};
-  const size_t vb = c->n_pad * sizeof(R4<double>);
-  cudaMemsetAsync(L1, 0, vb, c->stream);
-  cudaMemsetAsync(L2, 0, vb, c->stream);
+template <typename F>
+ieq_status program_step_vjp_ws(ieq_ctx *c, const RkProgram &prog, void *const *x, double t0, F lambda, F u,
+                               const void *rho, VjpWork<F> &w, void *const *reg, size_t vb) {
+  const F L1 = MakeField<F>::of(c, reg[0]), L2 = MakeField<F>::of(c, reg[1]), LK = MakeField<F>::of(c, reg[2]),
+          tmp = MakeField<F>::of(c, reg[3]);
+  F L[3] = {lambda, L1, L2};
+  cudaMemsetAsync(reg[0], 0, vb, c->stream);
+  cudaMemsetAsync(reg[1], 0, vb, c->stream);
   int e = prog.evaluations;
   for (int si = (int)prog.stages.size() - 1; si >= 0; --si) {
     const RkStage &st = prog.stages[si];
     if (st.src >= 0) {
-      cudaMemsetAsync(LK, 0, vb, c->stream);
+      cudaMemsetAsync(reg[2], 0, vb, c->stream);
       --e;
     }
     for (int ai = (int)st.as.size() - 1; ai >= 0; --ai) {
       const RkAssign &as = st.as[ai];
-      lincomb(c, tmp, 1.0, L[as.dst], 0.0, nullptr);
-      lincomb(c, L[as.dst], as.a[as.dst], tmp, 0.0, nullptr);
+      lincomb(c, tmp, 1.0, L[as.dst], 0.0, F{});
+      lincomb(c, L[as.dst], as.a[as.dst], tmp, 0.0, F{});
       for (int r = 0; r < 3; ++r)
         if (r != as.dst && as.a[r] != 0.0) lincomb(c, L[r], 1.0, L[r], as.a[r], tmp);
       if (st.src >= 0 && as.k != 0.0) lincomb(c, LK, 1.0, LK, as.k, tmp);
     }
     if (st.src >= 0) {
-      Epi ep;
+      Epi<F> ep;
       ep.dst = L[st.src];
       ep.x = L[st.src];
       ep.al = 1.0;
       ep.ga = st.h;
-      const ieq_status r = vjp(c, x[e], LK, stage_u(c, u, uw, w.d_time, t0 + st.t), rho, z, J0, gJr, ep);
+      const ieq_status r = vjp(c, MakeField<F>::of(c, x[e]), LK, stage_u(c, u, w, t0 + st.t), rho, w.z, w.J0, w.gJr, ep);
       if (r != IEQ_OK) return r;
     }
   }
@@ -972,20 +1044,22 @@ ieq_status ieq_operator_jvp(ieq_ctx *c, const void *b, const void *v, const void
   cudaSetDevice(c->device);
   std::vector<void *> w;
   if ((st = work_alloc(c, w, 2, c->n_pad * sizeof(R4<double>))) != IEQ_OK) return st;
-  AdjArgs a = adj_args(c);
-  a.b0 = (const R4<double> *)b;
-  a.u = (const R4<double> *)u;
-  a.v = (const R4<double> *)v;
+  using F = AoS<double>;
+  auto field = [&](const void *p) { return MakeField<F>::of(c, p); };
+  AdjArgs<F> a = adj_args<F>(c);
+  a.b0 = field(b);
+  a.u = field(u);
+  a.v = field(v);
   a.rho = (const double *)rho;
-  a.out = (R4<double> *)out;
+  a.out = field(out);
   if (c->s.hall) {
-    adj_curl(c, b, rho, w[0]);
-    adj_curl(c, v, rho, w[1]);
-    a.J0 = (const R4<double> *)w[0];
-    a.dJ = (const R4<double> *)w[1];
+    a.J0 = field(w[0]);
+    a.dJ = field(w[1]);
+    adj_curl(c, a.b0, rho, a.J0);
+    adj_curl(c, a.v, rho, a.dJ);
   }
-  if (a.ad) k_jvp<true><<<agrid(c), ablock(), 0, c->stream>>>(a);
-  else k_jvp<false><<<agrid(c), ablock(), 0, c->stream>>>(a);
+  if (a.ad) k_jvp<true, F><<<agrid(c), ablock(), 0, c->stream>>>(a);
+  else k_jvp<false, F><<<agrid(c), ablock(), 0, c->stream>>>(a);
   const cudaError_t e = cudaStreamSynchronize(c->stream);
   free_all(w);
   return e == cudaSuccess ? IEQ_OK : afail(c, IEQ_ERR_CUDA, cudaGetErrorString(e));
@@ -998,7 +1072,8 @@ ieq_status ieq_operator_vjp(ieq_ctx *c, const void *b, const void *w, const void
   cudaSetDevice(c->device);
   std::vector<void *> bufs;
   if ((st = work_alloc(c, bufs, 2, c->n_pad * sizeof(R4<double>))) != IEQ_OK) return st;
-  st = vjp(c, b, w, u, rho, out, bufs[0], bufs[1]);
+  auto field = [&](const void *p) { return MakeField<AoS<double>>::of(c, p); };
+  st = vjp(c, field(b), field(w), field(u), rho, field(out), field(bufs[0]), field(bufs[1]));
   const cudaError_t e = cudaStreamSynchronize(c->stream);
   free_all(bufs);
   if (st != IEQ_OK) return st;
@@ -1015,10 +1090,15 @@ ieq_status ieq_ssprk33_step_vjp(ieq_ctx *c, const void *s1, const void *s2, cons
   ieq_status st = check_adjoint_settings(c);
   if (st != IEQ_OK) return st;
   cudaSetDevice(c->device);
-  VjpWork w;
-  if ((st = vjp_work_alloc(c, w)) == IEQ_OK) st = ssprk33_step_vjp_ws(c, s1, s2, s3, t0, lambda, u, rho, w);
+  std::vector<void *> f;
+  if ((st = work_alloc(c, f, kVjpFields, c->n_pad * sizeof(R4<double>))) == IEQ_OK) {
+    using F = AoS<double>;
+    auto field = [&](const void *p) { return MakeField<F>::of(c, p); };
+    VjpWork<F> w = vjp_work<F>(c, f.data());
+    st = ssprk33_step_vjp_ws(c, field(s1), field(s2), field(s3), t0, field(lambda), field(u), rho, w);
+  }
   if (cudaStreamSynchronize(c->stream) != cudaSuccess && st == IEQ_OK) st = afail(c, IEQ_ERR_CUDA, "step vjp");
-  vjp_work_free(w);
+  free_all(f);
   return st;
 }
 
@@ -1028,18 +1108,18 @@ ieq_status ieq_ssprk33_step_vjp(ieq_ctx *c, const void *s1, const void *s2, cons
 }  // extern "C"
 
 namespace {
-// n zeroed vector fields from the context's adjoint pool (grown on demand, kept until
-// ieq_destroy, so repeated sweeps allocate nothing)
+// n vector fields from the context's adjoint pool (grown on demand, zeroed once, kept until
+// ieq_destroy, so repeated sweeps allocate nothing; a sweep writes every field before it reads it)
 ieq_status adj_pool(ieq_ctx *c, size_t n, size_t bytes, std::vector<void *> &out) {
   while (c->adj_bufs.size() < n) {
     void *p = nullptr;
     if (cudaMalloc(&p, bytes) != cudaSuccess) return afail(c, IEQ_ERR_CUDA, "adjoint work allocation");
     c->adj_bufs.push_back(p);
+    cudaMemsetAsync(p, 0, bytes, c->stream);
   }
   if (!c->adj_time && cudaMalloc(&c->adj_time, 4 * sizeof(double)) != cudaSuccess)
     return afail(c, IEQ_ERR_CUDA, "adjoint work allocation");
   out.assign(c->adj_bufs.begin(), c->adj_bufs.begin() + (long)n);
-  for (void *p : out) cudaMemsetAsync(p, 0, bytes, c->stream);
   return IEQ_OK;
 }
 }  // namespace
@@ -1063,7 +1143,8 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   RkProgram prog;
   if (program) rk_step_program(integ, c->s.dt, prog);
   cudaSetDevice(c->device);
-  const size_t vb = c->n_pad * sizeof(R4<double>);
+  // a field in either layout
+  const size_t vb = std::max(c->n_pad * sizeof(R4<double>), 3 * c->soa_n * sizeof(double));
   const int K = checkpoint_every;
   const int nseg = (num_steps + K - 1) / K;
   // states kept per step: SSPRK33 its three stage states, a 2N scheme the input of every stage
@@ -1071,34 +1152,72 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   int S2 = 0;
   if (ck2n || td2n) rk2n_coefficients(ck2n, &A2, &B2, &C2, &S2);
   const int P = program ? prog.evaluations : ssp ? 3 : S2;
-  // checkpoints (nseg), the stage states of one segment (P K), step work (5), step-adjoint
-  // work (7), the program's adjoint registers L1, L2, LK and a temporary (4)
+  // checkpoints (nseg), the stage states of one segment (P K), step work (6), step-adjoint
+  // work, the program's adjoint registers L1, L2, LK and a temporary (4)
   std::vector<void *> pool;
-  if ((st = adj_pool(c, (size_t)nseg + (size_t)P * K + 16, vb, pool)) != IEQ_OK) return st;
-  std::vector<void *> ck(pool.begin(), pool.begin() + nseg), seg(pool.begin() + nseg, pool.begin() + nseg + P * K),
-      w(pool.begin() + nseg + P * K, pool.begin() + nseg + P * K + 5);
-  VjpWork vw;
-  vw.f.assign(pool.begin() + nseg + P * K + 5, pool.begin() + nseg + P * K + 12);
-  void *const *preg = &pool[(size_t)nseg + (size_t)P * K + 12];   // L1, L2, LK, tmp
-  vw.d_time = c->adj_time + 2;
-  void *cur = w[0], *b2 = w[1], *b3 = w[2], *cb = w[3], *uw = w[4];
+  if ((st = adj_pool(c, (size_t)nseg + (size_t)P * K + 6 + kVjpFields + 4, vb, pool)) != IEQ_OK) return st;
+  std::vector<void *> ck(pool.begin(), pool.begin() + nseg), seg(pool.begin() + nseg, pool.begin() + nseg + P * K);
+  void *const *w = &pool[(size_t)nseg + (size_t)P * K];
+  void *const *vf = w + 6, *const *preg = vf + kVjpFields;   // L1, L2, LK, tmp
+  void *cur = w[0], *b2 = w[1], *b3 = w[2], *cb = w[3], *uw = w[4], *lam = w[5];
   double *d_time = c->adj_time;
   std::vector<double> t0s(num_steps + 1, 0.0);
   for (int n = 0; n < num_steps; ++n) t0s[n + 1] = t0s[n] + c->s.dt;   // calc_time_3_args / _2_args
-  // the forward passes run the fused stage kernels (ieq_time_steps' path) unless the settings
-  // ask for the reference kernel lists (IEQ_STAGE_KERNEL=LIST)
-  const bool fused = c->s.stage_kernel != 4;
-  int conv = 1;
-  if (fused && (st = adj_read_conv(c, u, conv)) != IEQ_OK) return st;
-  void *ua = c->s.variable_u ? uw : (void *)u;   // u is rewritten only when it varies in time
   auto set_time = [&](double t0) {
     const double tt[2] = {t0, t0};
     cudaMemcpyAsync(d_time, tt, sizeof(tt), cudaMemcpyHostToDevice, c->stream);
   };
+  // the step adjoints of steps n1 - 1 .. n0, whose stage states are in seg
+  auto reverse = [&](auto lambda, auto us, const void *r, auto &vw, int n0, int n1) -> ieq_status {
+    using F = decltype(lambda);
+    ieq_status s = IEQ_OK;
+    for (int n = n1 - 1; n >= n0 && s == IEQ_OK; --n) {
+      void *const *x = &seg[(size_t)P * (n - n0)];
+      auto field = [&](const void *p) { return MakeField<F>::of(c, p); };
+      if (program) s = program_step_vjp_ws(c, prog, x, t0s[n], lambda, us, r, vw, preg, vb);
+      else if (ssp) s = ssprk33_step_vjp_ws(c, field(x[0]), field(x[1]), field(x[2]), t0s[n], lambda, us, r, vw);
+      else s = rk2n_step_vjp_ws(c, ck2n, x, t0s[n], lambda, us, r, vw);
+    }
+    return s;
+  };
+  if (num_steps == 0) return IEQ_OK;   // lambda stays as it is
+  // The forward passes run the fused stage kernels (ieq_time_steps' path) and the whole sweep
+  // stays in the layout of the fused state; IEQ_STAGE_KERNEL=LIST runs the reference kernel
+  // lists on the caller's records instead.
+  if (c->s.stage_kernel != 4) {
+    using F = SoA<double>;
+    const size_t sb = 3 * c->soa_n * sizeof(double);
+    int conv = 1;
+    F b{}, us{};
+    const double *rhos = nullptr;
+    if ((st = adj_state_begin(c, b0, u, rho, conv, b, us, rhos)) != IEQ_OK) return st;
+    const F lambda_s = MakeField<F>::of(c, lam);
+    adj_to_soa(c, lambda, lambda_s);
+    VjpWork<F> vw = vjp_work<F>(c, vf);
+    auto advance = [&](const void *from, double t0, int nsteps, bool keep, double *&end) -> ieq_status {
+      set_time(t0);
+      return adj_state_steps(c, conv, (const double *)from, rho, d_time, nsteps,
+                             keep ? (double *const *)seg.data() : nullptr, P, end);
+    };
+    double *at = b.p;
+    for (int s = 0; s < nseg && st == IEQ_OK; ++s) {
+      cudaMemcpyAsync(ck[s], at, sb, cudaMemcpyDeviceToDevice, c->stream);
+      if (s + 1 < nseg) st = advance(at, t0s[(size_t)s * K], K, false, at);
+    }
+    for (int s = nseg - 1; s >= 0 && st == IEQ_OK; --s) {
+      const int n0 = s * K, n1 = std::min(num_steps, n0 + K);
+      if ((st = advance(ck[s], t0s[n0], n1 - n0, true, at)) == IEQ_OK) st = reverse(lambda_s, us, rhos, vw, n0, n1);
+    }
+    adj_to_aos(c, lambda_s, lambda);
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess && st == IEQ_OK) st = afail(c, IEQ_ERR_CUDA, "adjoint sweep");
+    return st;
+  }
+  void *ua = c->s.variable_u ? uw : (void *)u;   // u is rewritten only when it varies in time
+  const size_t ab = c->n_pad * sizeof(R4<double>);
   // one step through the reference kernels; keep (optional) receives the P states of the step
   auto step = [&](void *state, void *const *keep) -> ieq_status {
     if (ssp) {
-      if (keep) cudaMemcpyAsync(keep[0], state, vb, cudaMemcpyDeviceToDevice, c->stream);
+      if (keep) cudaMemcpyAsync(keep[0], state, ab, cudaMemcpyDeviceToDevice, c->stream);
       void *args[7] = {state, b2, b3, cb, ua, (void *)rho, d_time};
       const char *seq[] = {"calc_curlB_rho_1_3args", "calc_u_3_args", "SSPRK33_1", "SSPRK33_2a",
                            "calc_curlB_rho_2_3args", "calc_u_3_args", "SSPRK33_2b", "SSPRK33_3a",
@@ -1108,8 +1227,8 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
         if (!c->s.variable_u && std::strncmp(k, "calc_u", 6) == 0) continue;
         ieq_status s = adj_run_kernel(c, k, args, 7);
         if (s != IEQ_OK) return s;
-        if (std::strcmp(k, "SSPRK33_1") == 0 && keep) cudaMemcpyAsync(keep[1], b2, vb, cudaMemcpyDeviceToDevice, c->stream);
-        if (std::strcmp(k, "SSPRK33_2b") == 0 && keep) cudaMemcpyAsync(keep[2], b3, vb, cudaMemcpyDeviceToDevice, c->stream);
+        if (std::strcmp(k, "SSPRK33_1") == 0 && keep) cudaMemcpyAsync(keep[1], b2, ab, cudaMemcpyDeviceToDevice, c->stream);
+        if (std::strcmp(k, "SSPRK33_2b") == 0 && keep) cudaMemcpyAsync(keep[2], b3, ab, cudaMemcpyDeviceToDevice, c->stream);
       }
       return IEQ_OK;
     }
@@ -1118,7 +1237,7 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
     void *args[6] = {state, b2, cb, ua, (void *)rho, d_time};
     const std::string p = ck2n ? "CarpenterKennedy2N54_" : "ToulorgeDesmet2N84F_";
     for (int s = 0; s < S2; ++s) {
-      if (keep) cudaMemcpyAsync(keep[s], state, vb, cudaMemcpyDeviceToDevice, c->stream);
+      if (keep) cudaMemcpyAsync(keep[s], state, ab, cudaMemcpyDeviceToDevice, c->stream);
       ieq_status r;
       if (c->s.hall && (r = adj_run_kernel(c, "calc_curlB_rho_1_2args", args, 6)) != IEQ_OK) return r;
       if (c->s.variable_u && (r = adj_run_kernel(c, "calc_u_2_args", args, 6)) != IEQ_OK) return r;
@@ -1130,32 +1249,26 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   // nsteps steps of `state` from time t0, the stage states of step k into keep[P k ..] if given
   auto advance = [&](void *state, double t0, int nsteps, void *const *keep) -> ieq_status {
     set_time(t0);
-    if (fused) return adj_fused_steps(c, conv, state, b2, b3, cb, ua, rho, d_time, nsteps, keep, P);
     ieq_status r = IEQ_OK;
     for (int k = 0; k < nsteps && r == IEQ_OK; ++k) r = step(state, keep ? keep + (size_t)P * k : nullptr);
     return r;
   };
   // forward sweep: the checkpoints at the start of every segment (the last segment's steps are
   // run by the reverse sweep only)
-  cudaMemcpyAsync(cur, b0, vb, cudaMemcpyDeviceToDevice, c->stream);
+  using F = AoS<double>;
+  VjpWork<F> vw = vjp_work<F>(c, vf);
+  cudaMemcpyAsync(cur, b0, ab, cudaMemcpyDeviceToDevice, c->stream);
   for (int s = 0; s < nseg && st == IEQ_OK; ++s) {
-    cudaMemcpyAsync(ck[s], cur, vb, cudaMemcpyDeviceToDevice, c->stream);
+    cudaMemcpyAsync(ck[s], cur, ab, cudaMemcpyDeviceToDevice, c->stream);
     if (s + 1 < nseg) st = advance(cur, t0s[(size_t)s * K], K, nullptr);
   }
   // reverse sweep: recompute a segment from its checkpoint keeping the stage states, then
   // apply the step adjoints backwards
   for (int s = nseg - 1; s >= 0 && st == IEQ_OK; --s) {
     const int n0 = s * K, n1 = std::min(num_steps, n0 + K);
-    cudaMemcpyAsync(cur, ck[s], vb, cudaMemcpyDeviceToDevice, c->stream);
+    cudaMemcpyAsync(cur, ck[s], ab, cudaMemcpyDeviceToDevice, c->stream);
     st = advance(cur, t0s[n0], n1 - n0, seg.data());
-    for (int n = n1 - 1; n >= n0 && st == IEQ_OK; --n) {
-      void *const *x = &seg[(size_t)P * (n - n0)];
-      if (program)
-        st = program_step_vjp_ws(c, prog, x, t0s[n], lambda, u, rho, vw, preg[0], preg[1], preg[2], preg[3]);
-      else
-        st = ssp ? ssprk33_step_vjp_ws(c, x[0], x[1], x[2], t0s[n], lambda, u, rho, vw)
-                 : rk2n_step_vjp_ws(c, ck2n, x, t0s[n], lambda, u, rho, vw);
-    }
+    if (st == IEQ_OK) st = reverse(MakeField<F>::of(c, lambda), MakeField<F>::of(c, u), rho, vw, n0, n1);
   }
   if (cudaStreamSynchronize(c->stream) != cudaSuccess && st == IEQ_OK) st = afail(c, IEQ_ERR_CUDA, "adjoint sweep");
   return st;

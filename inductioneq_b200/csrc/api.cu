@@ -416,6 +416,13 @@ void launch_curl_brick_any(ieq_ctx *c, SoA<R> b, const R *rho, SoA<R> E, SoA<R> 
   }
 }
 
+// u = u_analytical at time[1], or at t without one
+template <typename R>
+void launch_calc_u(ieq_ctx *c, const Mesh &m, R *u, long long stride, const R *time, R t) {
+  launch_pdl(k_init<R>, grid3(m.nx, m.ny, m.nz), block3(), c->stream, c->s.pdl, m, (int)c->s.testcase, (int)CALC_U, u,
+             stride, (R *)nullptr, time, t);
+}
+
 template <typename R, typename F>
 CurlArgs<R, F> curl_args(ieq_ctx *c, F b, const R *rho, F out) {
   CurlArgs<R, F> a;
@@ -576,7 +583,7 @@ ieq_status run_one(ieq_ctx *c, const char *name, const uint32_t *g, void *const 
     if ((st = need(nm == "analytical_b" ? 2 : 1)) != IEQ_OK) return st;
     const int kind = nm == "init_b" ? INIT_B : nm == "init_u" ? INIT_U : nm == "init_rho" ? INIT_RHO : ANALYTICAL_B;
     k_init<R><<<grid, blk, 0, c->stream>>>(m, c->s.testcase, kind, (R *)args[0], 0, (R *)args[0],
-                                           nargs > 1 ? (const R *)args[1] : nullptr);
+                                           nargs > 1 ? (const R *)args[1] : nullptr, (R)0);
     IEQ_LAUNCHED(c);
     return IEQ_OK;
   }
@@ -664,7 +671,7 @@ ieq_status run_one(ieq_ctx *c, const char *name, const uint32_t *g, void *const 
   auto fv = [&](int k) { return AoS<R>{(R4<R> *)f.b[k]}; };
   if (nm == "calc_time_2_args" || nm == "calc_time_3_args") return launch_time<R>(c, f.time, 2, (R)0);
   if (nm == "calc_u_2_args" || nm == "calc_u_3_args") {
-    k_init<R><<<grid, blk, 0, c->stream>>>(m, c->s.testcase, CALC_U, (R *)f.u, 0, nullptr, (const R *)f.time);
+    launch_calc_u<R>(c, m, (R *)f.u, 0, (const R *)f.time, (R)0);
     IEQ_LAUNCHED(c);
     return IEQ_OK;
   }

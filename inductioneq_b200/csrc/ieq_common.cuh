@@ -6,6 +6,33 @@
 
 namespace ieq {
 
+// Programmatic dependent launch: the curl and stage kernels of consecutive stages depend on
+// each other's complete output.  Launched with programmatic stream serialization (launch_pdl), a kernel may be scheduled while its predecessor still runs; each block first
+// waits for the predecessor grid to complete and its writes to be visible (griddepcontrol.wait,
+// a hardware dependency wait that ends when the predecessor ends) and only then allows its own
+// dependents to be scheduled (griddepcontrol.launch_dependents).  No block reads or writes
+// fields before its wait, and a kernel never runs more than one launch ahead.  Launched
+// without the attribute both instructions return at once.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename Kern, typename... Args>
+inline void launch_pdl(Kern kernel, dim3 grid, dim3 block, cudaStream_t s, bool pdl, const Args &...a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = 0;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, a...);
+}
+
 // --------------------------------------------------------------------------- layout
 // REAL4 array-of-structs at the boundary (x, y, z, w with w = 0): one 32-byte (FP64) or
 // 16-byte (FP32) record per node, index ix + NX*(iy + NY*iz).

@@ -9,7 +9,8 @@ namespace ieq {
 // ---------------------------------------------------------------- testcase evaluation
 enum InitKind : int { INIT_B = 0, INIT_U = 1, INIT_RHO = 2, ANALYTICAL_B = 3, CALC_U = 4 };
 
-// kernel_init.cl:3-48 and kernel_time_integrator.cl:93-125 (u = u_analytical(time[1]))
+// kernel_init.cl:3-48 and kernel_time_integrator.cl:93-125 (u = u_analytical(time[1]), or at t
+// without a time array)
 // vout: REAL4 AoS (vstride = 0) or SoA with component stride vstride
 template <typename R>
 __device__ __forceinline__ void st_any(R *base, long long vstride, long long idx, V3<R> v) {
@@ -52,10 +53,12 @@ __device__ void hall_periodic_u_block(const Mesh &m, R *vout, long long vstride,
 }
 
 template <typename R>
-__global__ void k_init(Mesh m, int tc, int kind, R *vout, long long vstride, R *sout, const R *time) {
+__global__ void k_init(Mesh m, int tc, int kind, R *vout, long long vstride, R *sout, const R *time, R t) {
+  pdl_enter();
+  if (kind == CALC_U && time) t = time[1];
   if (kind == CALC_U && tc == TC_HALL_PERIODIC && blockDim.x <= 32 && blockDim.y <= 32 && blockDim.z <= 32 &&
       blockDim.x * blockDim.y * blockDim.z >= blockDim.x + blockDim.y + blockDim.z) {
-    hall_periodic_u_block<R>(m, vout, vstride, time[1]);
+    hall_periodic_u_block<R>(m, vout, vstride, t);
     return;
   }
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -68,7 +71,7 @@ __global__ void k_init(Mesh m, int tc, int kind, R *vout, long long vstride, R *
     case INIT_U: st_any(vout, vstride, idx, u_analytical<R>(tc, m, ix, iy, iz, (R)0)); break;
     case INIT_RHO: sout[idx] = (R)1; break;
     case ANALYTICAL_B: st_any(vout, vstride, idx, b_analytical<R>(tc, m, ix, iy, iz, time[0])); break;
-    case CALC_U: st_any(vout, vstride, idx, u_analytical<R>(tc, m, ix, iy, iz, time[1])); break;
+    case CALC_U: st_any(vout, vstride, idx, u_analytical<R>(tc, m, ix, iy, iz, t)); break;
   }
 }
 
