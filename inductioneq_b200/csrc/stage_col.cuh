@@ -14,6 +14,8 @@
 // non-periodic box, where the outflow SAT needs it), so the stage kernel reads two values
 // per stencil point and axis instead of six and forms no products there.
 #pragma once
+#include <cmath>
+
 #include "stage_kernel.cuh"
 
 namespace ieq {
@@ -638,13 +640,59 @@ inline ColShape fit_rows(ColShape sh, int nxe) {
   sh.y = yz / sh.z > 0 ? yz / sh.z : 1;
   return sh;
 }
-inline ColShape pair_shape(ColShape sh, bool curl, long long nodes, int nx, int K = 2) {
-  if (!sh.given && (curl || nodes <= (1ll << 20))) {
+// The pair kernels' shape on a box of more than one round of the GPU: evenly divided rows, or a
+// shape that takes fewer rounds.  A block costs its whole slot of an SM however many of its
+// threads have nodes, and a warp that holds an x boundary lane gathers the x axis node by node:
+// blocks 8 or 16 pairs wide leave most warps without one (and load whole 128-byte lines).  Up to
+// three rounds count whole, beyond that the last one half; a width other than 8 or 16 pairs costs
+// 10 % and one z plane per block 3 % at equal rounds, and the even division stays
+// unless another shape gains 4 % (fitted to 13 boxes of 20-40 shapes each, rotation and confined
+// Hall, 4th order: 0-37 % faster than even division, 7 % on average, 1 % from the best shape).  A
+// launch over the interior columns only (band) has no boundary lanes, so only the rounds count,
+// from 10 % on.  Rotation, even division / this rule, us a stage: 50^3 4th order 17.3 / 14.0,
+// 96^3 6th order 71 / 61, 128^3 6th order 141 / 128.  Within one round, on periodic grids
+// (0.8-1.1 times the speed) and in FP32 (a warp row of 8 pairs is half a line; 0.85-1.25 times) the
+// even division stays.
+constexpr int kSms = 148;
+inline ColShape wave_shape(ColShape sh, int nxe, int ny, int nz, int resident, bool band) {
+  if (sh.given) return sh;
+  const auto rounds = [&](int x, int y, int z) {
+    const auto parts = [](int n, int d) { return (long long)((n + d - 1) / d); };
+    return (double)(parts(nxe, x) * parts(ny, y) * parts(nz, z)) / (kSms * resident);
+  };
+  const auto cost = [&](int x, int y, int z) {
+    const double r = rounds(x, y, z);
+    return (r <= 3 ? std::ceil(r) : r + 0.5) * ((x % 8 || x > 16) && !band ? 1.10 : 1.0) * (z == 1 && !band ? 1.03 : 1.0) *
+           (1 + 1e-3 * r);
+  };
+  if (rounds(sh.x, sh.y, sh.z) <= 1) return sh;
+  double best = cost(sh.x, sh.y, sh.z) * (band ? 0.90 : 0.96);
+  for (int w = 1; w <= 11; ++w) {
+    const int x = w <= 8 ? (nxe + w - 1) / w : 8 << (w - 9);
+    if (x < 8 || x > 32) continue;
+    for (int z = 2; z >= 1; --z) {
+      const int y = kColThreads / (x * z);
+      const double c = cost(x, y, z);
+      if (c < best) {
+        best = c;
+        sh.x = x;
+        sh.y = y;
+        sh.z = z;
+      }
+    }
+  }
+  return sh;
+}
+// (even: rows evenly divided; nxe threads per row; resident: blocks of the kernel per SM)
+inline ColShape pair_shape(ColShape sh, bool curl, const Mesh &m, bool even, int nxe, int resident,
+                           bool band = false) {
+  if (!sh.given && (curl || (long long)m.nx * m.ny * m.nz <= (1ll << 20))) {
     sh.x = 32;
     sh.y = 2;
     sh.z = 2;
   }
-  return fit_rows(sh, nx / K);
+  sh = fit_rows(sh, nxe);
+  return even ? sh : wave_shape(sh, nxe, m.ny, m.nz, resident, band);
 }
 inline dim3 col_block(ColShape sh) { return dim3((unsigned)sh.x, (unsigned)sh.y, (unsigned)sh.z); }
 inline dim3 col_grid(ColShape sh, int nx, int ny, int nz, int nodes) {

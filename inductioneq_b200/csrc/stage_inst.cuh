@@ -88,31 +88,40 @@ static void launch_col_ph(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool hod, int c
   }
 }
 
+// whether the pair kernels' blocks divide rows evenly (else wave_shape)
+static constexpr bool even_rows(bool per) { return per || sizeof(IEQ_R) == 4; }
+
 // a box's stage as two launches: the pair kernel `kint` over the interior x range
 // [xband, nx - xband) (no time bookkeeping) and the one-node kernel `kband` over the 2 *
 // xband boundary columns of every row (with it)
 template <typename KI, typename KB>
-static void launch_banded(KI kint, KB kband, const StageArgs<IEQ_R, SoA<IEQ_R>> &a, ColShape sh, cudaStream_t s) {
+static void launch_banded(KI kint, KB kband, const StageArgs<IEQ_R, SoA<IEQ_R>> &a, ColShape sh, int resident,
+                          cudaStream_t s) {
   constexpr int XB = xband<IEQ_OP>();
   StageArgs<IEQ_R, SoA<IEQ_R>> ai = a;
   ai.tpost = TP_NONE;
   const int np = (a.m.nx - 2 * XB) / 2;
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const ColShape ps = pair_shape(sh, false, a.m, even_rows(false), np, resident, true);
   launch_pdl(kint, col_grid(ps, np, a.m.ny, a.m.nz, 1), col_block(ps), s, sh.pdl, ai);
-  const long long nb = 2ll * XB * a.m.ny * a.m.nz;
+  const long long nb = (long long)xband_columns<IEQ_OP>(a.m.nx) * a.m.ny * a.m.nz;
   launch_pdl(kband, dim3((unsigned)((nb + kColThreads - 1) / kColThreads)), dim3(kColThreads), s, sh.pdl, a);
 }
-// whether a box's stage splits off its x boundary columns: even rows in which the band is at
-// most a tenth of the row, and for a band of two columns a side (2nd order) rows of at least
-// 96 (measured on B200: rotation 2nd order 96^3 +10 %, 6th order 128^3 +23 %, confined Hall
-// 4th order 128^3 +12 % FP64 / +20 % FP32; 4th order 64^3, a band of 8 of 64 columns, 14 %
-// slower; rotation, SSPRK33, 40 steps: 2nd order banded 5-43 % slower at 40^3 .. 80^3 and 12 %
-// faster at 96^3 -- its one boundary row a side costs the pair kernel little, the band's
-// launch more -- 4th order banded faster from 80^3 (+8 %), 6th order from 120^3 (+29 %))
-inline int band_min_nx(int xb) { return xb <= 2 ? 96 : 20 * xb; }
-static bool banded(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, ColShape sh) {
-  if (per || sh.band == 0 || a.m.nx % 2 != 0 || a.m.nx < 2 * xband<IEQ_OP>() + 2) return false;
-  return sh.band == 2 || a.m.nx >= band_min_nx(xband<IEQ_OP>());
+// whether a box's stage splits off its x boundary columns.  The band's launch and its one node
+// per thread pay where every warp of the pair kernel would hold a boundary lane, which blocks 8
+// pairs wide avoid in rows of whole 8-pair blocks (wave_shape).  Measured on B200 over 21 sizes
+// of 40^3 .. 160^3: 2nd order (two columns a side) from rows of 97 on, 1-28 % faster with the
+// band; rotation 4th and 6th order from 90 on where the row is not whole 8-pair blocks (97^3
+// 12 / 6 %, 130^3 23 / 18 %; 96^3 with it 7 % slower, 84^3 8 % slower), 4th order also from
+// 128 on (128^3 5 %); with the Hall term 4th
+// and 6th order never (97^3 .. 160^3 0-15 % slower with it).  FP32 (evenly divided rows): even
+// rows in which the band is at most a tenth of the row, 2nd order from 96 on (confined Hall 4th
+// order 128^3 +20 %)
+static bool banded(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, ColShape sh, bool hall) {
+  constexpr int XB = xband<IEQ_OP>();
+  const int nx = a.m.nx;
+  if (per || sh.band == 0 || nx < 2 * XB + 2) return false;
+  if (sizeof(IEQ_R) == 4) return nx % 2 == 0 && (sh.band == 2 || nx >= (XB <= 2 ? 96 : 20 * XB));
+  return sh.band == 2 || (XB <= 2 ? nx > 96 : !hall && ((nx >= 90 && (nx + 1) / 2 % 8 != 0) || (XB <= 4 && nx >= 128)));
 }
 
 // the Hall stage kernel without convection, K x-adjacent nodes per thread
@@ -123,7 +132,8 @@ static void launch_stage_hall_k(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per,
     return;   // (quads are FP32 only; the caller never asks for them in FP64)
   } else {
     const int np = (a.m.nx + K - 1) / K;
-    const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, K * np, K);
+    const ColShape ps = pair_shape(sh, false, a.m, even_rows(per), np,
+                                   K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS : IEQ_STAGE_X2_MIN_BLOCKS);
     const dim3 g = col_grid(ps, np, a.m.ny, a.m.nz, 1), b = col_block(ps);
     if (per) {
       if (hodp) launch_pdl(k_stage_hall_x2<IEQ_R, IEQ_OP, true, true, K>, g, b, s, sh.pdl, a);
@@ -156,17 +166,17 @@ static void launch_col_x2_ph(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool hod, in
 template <int N>
 static void launch_hall_conv_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, bool hodp, ColShape sh,
                                    cudaStream_t s) {
-  if (banded(a, per, sh)) {
+  if (banded(a, per, sh, true)) {
     if (hodp)
       launch_banded(k_stage_col_x2<IEQ_R, IEQ_OP, false, true, true, 1, true, false, N, true>,
-                    k_stage_xband<IEQ_R, IEQ_OP, true, true, 1, N, true, false>, a, sh, s);
+                    k_stage_xband<IEQ_R, IEQ_OP, true, true, 1, N, true, false>, a, sh, conv_min_blocks<N>(), s);
     else
       launch_banded(k_stage_col_x2<IEQ_R, IEQ_OP, false, true, false, 1, false, false, N, true>,
-                    k_stage_xband<IEQ_R, IEQ_OP, true, false, 1, N, false, false>, a, sh, s);
+                    k_stage_xband<IEQ_R, IEQ_OP, true, false, 1, N, false, false>, a, sh, conv_min_blocks<N>(), s);
     return;
   }
   const int np = (a.m.nx + 1) / 2;
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const ColShape ps = pair_shape(sh, false, a.m, even_rows(per), np, conv_min_blocks<N>());
   const dim3 g2 = col_grid(ps, np, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
   if (per) {
     if (hodp) launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, true, true, 1, true, false, N>, g2, b2, s, sh.pdl, a);
@@ -180,13 +190,13 @@ static void launch_hall_conv_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool p
 // the convection pair kernels (no Hall term, no dissipation) with the flux-form mask N
 template <int N>
 static void launch_conv_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, ColShape sh, cudaStream_t s) {
-  if (banded(a, per, sh)) {
+  if (banded(a, per, sh, false)) {
     launch_banded(k_stage_col_x2<IEQ_R, IEQ_OP, false, false, false, 1, false, false, N, true>,
-                  k_stage_xband<IEQ_R, IEQ_OP, false, false, 1, N, false, false>, a, sh, s);
+                  k_stage_xband<IEQ_R, IEQ_OP, false, false, 1, N, false, false>, a, sh, conv_min_blocks<N>(), s);
     return;
   }
   const int np = (a.m.nx + 1) / 2;
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const ColShape ps = pair_shape(sh, false, a.m, even_rows(per), np, conv_min_blocks<N>());
   const dim3 g2 = col_grid(ps, np, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
   if (per) launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, false, false, 1, false, false, N>, g2, b2, s, sh.pdl, a);
   else launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, false, false, false, 1, false, false, N>, g2, b2, s, sh.pdl, a);
@@ -195,13 +205,13 @@ static void launch_conv_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, C
 // the pair kernels with first-order dissipation summed in their gathers (FOF)
 template <bool H>
 static void launch_fo_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, ColShape sh, cudaStream_t s) {
-  if (banded(a, per, sh)) {
+  if (banded(a, per, sh, H)) {
     launch_banded(k_stage_col_x2<IEQ_R, IEQ_OP, false, H, false, 1, false, false, 10, true, true>,
-                  k_stage_xband<IEQ_R, IEQ_OP, H, false, 1, 10, false, false, true>, a, sh, s);
+                  k_stage_xband<IEQ_R, IEQ_OP, H, false, 1, 10, false, false, true>, a, sh, fo_min_blocks<IEQ_OP, false>(), s);
     return;
   }
   const int np = (a.m.nx + 1) / 2;
-  const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+  const ColShape ps = pair_shape(sh, false, a.m, even_rows(per), np, per ? fo_min_blocks<IEQ_OP, true>() : fo_min_blocks<IEQ_OP, false>());
   const dim3 g2 = col_grid(ps, np, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
   if (per) launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, true, H, false, 1, false, false, 10, false, true>, g2, b2, s, sh.pdl, a);
   else launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, false, H, false, 1, false, false, 10, false, true>, g2, b2, s, sh.pdl, a);
@@ -224,13 +234,13 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
       launch_stage_hall_k<4>(a, per, hodp, sh, s);
       return;
     }
-    if (banded(a, per, sh)) {
+    if (banded(a, per, sh, true)) {
       if (hodp)
         launch_banded(k_stage_hall_x2<IEQ_R, IEQ_OP, false, true, 2, true>,
-                      k_stage_xband<IEQ_R, IEQ_OP, true, true, 0, -1, true, false>, a, sh, s);
+                      k_stage_xband<IEQ_R, IEQ_OP, true, true, 0, -1, true, false>, a, sh, IEQ_STAGE_X2_MIN_BLOCKS, s);
       else
         launch_banded(k_stage_hall_x2<IEQ_R, IEQ_OP, false, false, 2, true>,
-                      k_stage_xband<IEQ_R, IEQ_OP, true, false, 0, -1, false, false>, a, sh, s);
+                      k_stage_xband<IEQ_R, IEQ_OP, true, false, 0, -1, false, false>, a, sh, IEQ_STAGE_X2_MIN_BLOCKS, s);
       return;
     }
     launch_stage_hall_k<2>(a, per, hodp, sh, s);
@@ -279,7 +289,8 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
   if (sh.pairs && per && hall && !foad && pair_rows(a.m, per) && pair_ok(a.bk) && pair_ok(a.u) && pair_ok(a.E) &&
       pair_ok(a.Hpre) && pair_ok(a.X) && pair_ok(a.Y) && pair_ok(a.Z) && pair_ok(a.out) && pair_ok(a.out2) &&
       pair_ok(a.out3)) {
-    const ColShape ps = pair_shape(sh, false, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx);
+    const ColShape ps = pair_shape(sh, false, a.m, even_rows(per), a.m.nx / 2,
+                                   conv ? IEQ_COL_X2_CONV_MIN_BLOCKS : IEQ_COL_X2_MIN_BLOCKS);
     launch_col_x2_ph<true, true>(a, hod, conv, hodp, col_grid(ps, a.m.nx / 2, a.m.ny, a.m.nz, 1), col_block(ps), sh.pdl,
                                  s);
     return;
@@ -331,14 +342,15 @@ void launch_curl_e<IEQ_R, IEQ_OP>(const CurlArgs<IEQ_R, SoA<IEQ_R>> &a, bool per
       if ((sh.quads || quads_fill((long long)a.m.nx * a.m.ny * a.m.nz)) && a.m.nx % 4 == 0 && group_ok<4>(a.b) &&
           group_ok<4>(a.out) && group_ok<4>(a.hout) &&
           (a.rho == nullptr || reinterpret_cast<uintptr_t>(a.rho) % 16 == 0)) {
-        const ColShape ps = pair_shape(sh, true, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx, 4);
+        const ColShape ps = pair_shape(sh, true, a.m, even_rows(per), a.m.nx / 4, IEQ_CURL_X4_MIN_BLOCKS);
         const dim3 g4 = col_grid(ps, a.m.nx / 4, a.m.ny, a.m.nz, 1), b4 = col_block(ps);
         if (hod) launch_pdl(k_curl_e_x2<IEQ_R, IEQ_OP, true, true, 4>, g4, b4, s, sh.pdl, a);
         else launch_pdl(k_curl_e_x2<IEQ_R, IEQ_OP, true, false, 4>, g4, b4, s, sh.pdl, a);
         return;
       }
     }
-    const ColShape ps = pair_shape(sh, true, (long long)a.m.nx * a.m.ny * a.m.nz, a.m.nx);
+    const ColShape ps = pair_shape(sh, true, a.m, even_rows(per), a.m.nx / 2,
+                                   hod ? IEQ_CURL_X2_MIN_BLOCKS : IEQ_CURL_X2_PLAIN_MIN_BLOCKS);
     const dim3 g2 = col_grid(ps, a.m.nx / 2, a.m.ny, a.m.nz, 1), b2 = col_block(ps);
     if (hod) launch_pdl(k_curl_e_x2<IEQ_R, IEQ_OP, true, true>, g2, b2, s, sh.pdl, a);
     else launch_pdl(k_curl_e_x2<IEQ_R, IEQ_OP, true, false>, g2, b2, s, sh.pdl, a);
@@ -354,9 +366,10 @@ void launch_curl_e<IEQ_R, IEQ_OP>(const CurlArgs<IEQ_R, SoA<IEQ_R>> &a, bool per
       (a.rho == nullptr || reinterpret_cast<uintptr_t>(a.rho) % (2 * sizeof(IEQ_R)) == 0)) {
     constexpr int XB = xband<IEQ_OP>();
     const int np = (a.m.nx - 2 * XB) / 2;
-    const ColShape ps = pair_shape(sh, true, (long long)a.m.nx * a.m.ny * a.m.nz, 2 * np);
+    const ColShape ps =
+        pair_shape(sh, true, a.m, even_rows(per), np, hod ? IEQ_CURL_X2_MIN_BLOCKS : IEQ_CURL_X2_PLAIN_MIN_BLOCKS, true);
     const dim3 gi = col_grid(ps, np, a.m.ny, a.m.nz, 1), bi = col_block(ps);
-    const long long nb = 2ll * XB * a.m.ny * a.m.nz;
+    const long long nb = (long long)xband_columns<IEQ_OP>(a.m.nx) * a.m.ny * a.m.nz;
     const dim3 gb((unsigned)((nb + kColThreads - 1) / kColThreads)), bb(kColThreads);
     if (hod) {
       launch_pdl(k_curl_e_x2<IEQ_R, IEQ_OP, false, true, 2, true>, gi, bi, s, sh.pdl, a);

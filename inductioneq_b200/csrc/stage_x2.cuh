@@ -189,15 +189,34 @@ __device__ __forceinline__ bool x_pair_interior(int ix, int nx) {
 }
 
 // Boxes: the x boundary columns in a band of their own.  A pair kernel launched with XBAND
-// covers only the nodes xband(OP) <= ix < nx - xband(OP), whose x stencils are all interior
-// rows inside the row (no per-node fallback, no SAT on the x faces in its warps); the 2 *
-// xband(OP) boundary columns of every row run one node per thread in k_stage_xband, which
+// covers only the node pairs of xband(OP) <= ix < nx - xband(OP), whose x stencils are all
+// interior rows inside the row (no per-node fallback, no SAT on the x faces in its warps); the
+// xband_columns(OP, nx) other columns of every row run one node per thread in k_stage_xband, which
 // also does the stage's time bookkeeping.  xband is even, >= NUM_BOUNDS and >= the pair
 // window's reach 2*ceil(RI/2).
 template <int OP>
 __host__ __device__ constexpr int xband() {
   constexpr int nb = Op<OP>::NB + (Op<OP>::NB & 1), w = 2 * ((Op<OP>::RI + 1) / 2);
   return nb > w ? nb : w;
+}
+// columns of the band: an odd row's last interior node has no partner and goes with it
+template <int OP>
+__host__ __device__ constexpr int xband_columns(int nx) {
+  return 2 * xband<OP>() + (nx & 1);
+}
+// what a pair's first column stays short of the band by (FP32 bands have even rows only: the
+// test for odd ones raised the 2nd order kernel from 96 to 105 registers, 8 % slower)
+template <typename R, bool XBAND>
+__device__ __forceinline__ constexpr int band_tail() {
+  return XBAND && sizeof(R) == 8 ? 1 : 0;
+}
+// row and column of the band's i-th node
+template <int OP>
+__device__ __forceinline__ void xband_node(int i, int nx, int &row, int &ix) {
+  constexpr int XB = xband<OP>();
+  row = nx & 1 ? i / (2 * XB + 1) : i / (2 * XB);
+  const int slot = i - row * xband_columns<OP>(nx);
+  ix = slot < XB ? slot : nx - xband_columns<OP>(nx) + slot;
 }
 
 // resident 128-thread blocks per SM the register allocation targets (measured on B200 at
@@ -241,7 +260,7 @@ __global__ void __launch_bounds__(kColThreads, HODS ? (K == 4 ? IEQ_CURL_X4_MIN_
   const int ix = X0 + K * (blockIdx.x * blockDim.x + threadIdx.x);
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
-  if (ix >= nx - X0 || iy >= ny || iz >= nz) return;
+  if (ix + band_tail<R, XBAND>() >= nx - X0 || iy >= ny || iz >= nz) return;
   const int row0 = a.m.px * (iy + ny * iz);
   const int idx = row0 + ix;
   const long long cs = a.b.s;
@@ -484,7 +503,7 @@ __global__ void __launch_bounds__(kColThreads, K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS 
   const int ix = X0 + K * (blockIdx.x * blockDim.x + threadIdx.x);
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
-  if (ix < nx - X0 && iy < ny && iz < nz) {
+  if (ix + band_tail<R, XBAND>() < nx - X0 && iy < ny && iz < nz) {
     const int row0 = a.m.px * (iy + ny * iz);
     const int idx = row0 + ix;
     const long long es = a.E.s;
@@ -782,7 +801,7 @@ __global__ void __launch_bounds__(kColThreads, FOF ? fo_min_blocks<OP, PER>()
   const int ix = X0 + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
-  if (ix < nx - X0 && iy < ny && iz < nz) {
+  if (ix + band_tail<R, XBAND>() < nx - X0 && iy < ny && iz < nz) {
     const int row0 = a.m.px * (iy + ny * iz);
     const int idx = row0 + ix;
     const V3<R> zero = {0, 0, 0};
@@ -878,35 +897,31 @@ __device__ __forceinline__ void col_stage_node(const StageArgs<R, SoA<R>> &a, in
   stage_epilogue<R, SoA<R>>(a, idx, db);
 }
 
-// the x boundary columns of a box (2 * xband nodes per row, one per thread), and the stage's
+// the x boundary columns of a box (xband_columns nodes per row, one per thread), and the stage's
 // time bookkeeping
 template <typename R, int OP, bool HALL, bool HOD_, int CONV, int NEED, bool HODP, bool FOAD, bool FOF = false>
 __global__ void __launch_bounds__(kColThreads) k_stage_xband(const __grid_constant__ StageArgs<R, SoA<R>> a) {
-  constexpr int XB = xband<OP>();
   pdl_enter();
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long rows = (long long)a.m.ny * a.m.nz;
-  if (i < rows * 2 * XB) {
-    const int slot = (int)(i % (2 * XB));
-    const long long row = i / (2 * XB);
-    const int ix = slot < XB ? slot : a.m.nx - 2 * XB + slot;
-    col_stage_node<R, OP, HALL, HOD_, CONV, NEED, HODP, FOAD, FOF>(a, ix, (int)(row % a.m.ny), (int)(row / a.m.ny));
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.m.ny * a.m.nz * xband_columns<OP>(a.m.nx)) {
+    int row, ix;
+    xband_node<OP>(i, a.m.nx, row, ix);
+    col_stage_node<R, OP, HALL, HOD_, CONV, NEED, HODP, FOAD, FOF>(a, ix, row % a.m.ny, row / a.m.ny);
   }
   stage_time_post(a);
 }
 
 // J = curl(B)/rho, E = J x B, (HODS) the dissipation sum and J on the faces at one node of a
-// box's x boundary columns (2 * xband per row, one per thread; the order of k_curl_e_hod)
+// box's x boundary columns (xband_columns per row, one per thread; the order of k_curl_e_hod)
 template <typename R, int OP, bool HODS>
 __global__ void __launch_bounds__(kColThreads) k_curl_xband(const __grid_constant__ CurlArgs<R, SoA<R>> a) {
-  constexpr int XB = xband<OP>();
   pdl_enter();
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
-  if (i >= (long long)ny * nz * 2 * XB) return;
-  const int slot = (int)(i % (2 * XB));
-  const long long row = i / (2 * XB);
-  const int ix = slot < XB ? slot : nx - 2 * XB + slot, iy = (int)(row % ny), iz = (int)(row / ny);
+  if (i >= ny * nz * xband_columns<OP>(nx)) return;
+  int row, ix;
+  xband_node<OP>(i, nx, row, ix);
+  const int iy = row % ny, iz = row / ny;
   const int idx = ix + a.m.px * (iy + ny * iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {nx, ny, nz};
