@@ -24,6 +24,9 @@ CASES = [(dict(base, order=o, nodes=n, xband=band), dt)
          for band in (1, 2)]
 CASES += [(dict(CONF, order=4, nodes=n, xband=2, dissipation="HIGH_ORDER"), 1e-6) for n in ((31, 17, 18), (32, 17, 18))]
 CASES += [(dict(ROT, order=o, nodes=(33, 17, 18), xband=2, dissipation="FIRST_ORDER"), 2e-3) for o in (2, 4, 6)]
+# adaptive dissipation: compact blocks from three rounds on, against blocks of 32-node rows
+CASES += [(dict(base, order=o, nodes=n, xband=1, dissipation="ADAPTIVE"), dt)
+          for base, dt in ((ROT, 2e-3), (CONF, 1e-6)) for o, n in ((2, (57, 66, 71)), (4, (97, 41, 67)), (6, (66, 65, 64)))]
 
 
 def _run(c, dt, **kw):
@@ -45,7 +48,7 @@ def _run(c, dt, **kw):
 
 @pytest.mark.parametrize("c, dt", CASES)
 def test_pair_launches_equal_one_node_per_thread(c, dt):
-    ref = _run(dict(c, xband=0), dt, col_pairs=0)
+    ref = _run(dict(c, xband=0), dt, col_pairs=0, col_block=(32, 4, 1))
     got = _run(c, dt)
     assert np.isfinite(ref).all()
     assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
