@@ -64,10 +64,10 @@ struct Settings {
   // IEQ_NZ_GLOBAL planes whose plane 0 is global plane IEQ_Z_OFFSET (testcase coordinates
   // are the global grid's); 0 / 0: the grid is the whole domain
   int zoff = 0, nzg = 0;
-  // IEQ_CG_PASS_A: the CG's pass A as the 2.5D kernel (2, the default) or the per-node gather (1)
+  // IEQ_CG_PASS_A: the CG as one cooperative kernel with a z march (2, the default) or as the
+  // per-node gathers in a graph loop node (1)
   int cg_passes = 2;
   // IEQ_CG_LOOP=HOST (profiling): the CG iterations as max_iterations launches in sequence
-  // instead of a graph loop node (kernels inside a loop node are invisible to the profiler)
   bool cg_host_loop = false;
   // IEQ_HODP: Hall + high-order dissipation -- 1 the curl kernel forms the dissipation sum and
   // the stage kernel reads it; 0 the stage kernel gathers the dissipation rows itself
@@ -164,8 +164,8 @@ struct ieq_ctx {
     cudaGraphExec_t exec1 = nullptr, exec2 = nullptr;
   };
   std::map<std::vector<uintptr_t>, GraphEntry> graphs;
-  // cleaning graphs (div B, CG loop as a conditional WHILE node, projection) keyed by the
-  // field and the loop parameters; a second stream on which the loop body is captured
+  // IEQ_CG_PASS_A=1: cleaning graphs (div B, CG loop as a conditional WHILE node, projection)
+  // keyed by the field and the loop parameters; a second stream on which the loop body is captured
   std::map<std::vector<uintptr_t>, cudaGraphExec_t> clean_graphs;
   cudaStream_t aux_stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
