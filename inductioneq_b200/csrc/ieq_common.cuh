@@ -7,8 +7,9 @@
 namespace ieq {
 
 // Programmatic dependent launch: the curl and stage kernels of consecutive stages depend on
-// each other's complete output.  Launched with programmatic stream serialization (launch_pdl), a kernel may be scheduled while its predecessor still runs; each block first
-// waits for the predecessor grid to complete and its writes to be visible (griddepcontrol.wait,
+// each other's complete output.  Launched with programmatic stream serialization (launch_pdl), a
+// kernel may be scheduled while its predecessor still runs; each block first waits for the
+// predecessor grid to complete and its writes to be visible (griddepcontrol.wait,
 // a hardware dependency wait that ends when the predecessor ends) and only then allows its own
 // dependents to be scheduled (griddepcontrol.launch_dependents).  No block reads or writes
 // fields before its wait, and a kernel never runs more than one launch ahead.  Launched

@@ -111,9 +111,8 @@ static void launch_banded(KI kint, KB kband, const StageArgs<IEQ_R, SoA<IEQ_R>> 
 // pairs wide avoid in rows of whole 8-pair blocks (wave_shape).  Measured on B200 over 21 sizes
 // of 40^3 .. 160^3: 2nd order (two columns a side) from rows of 97 on, 1-28 % faster with the
 // band; rotation 4th and 6th order from 90 on where the row is not whole 8-pair blocks (97^3
-// 12 / 6 %, 130^3 23 / 18 %; 96^3 with it 7 % slower, 84^3 8 % slower), 4th order also from
-// 128 on (128^3 5 %); with the Hall term 4th
-// and 6th order never (97^3 .. 160^3 0-15 % slower with it).  FP32 (evenly divided rows): even
+// 12 / 6 %, 130^3 23 / 18 %; 96^3 with it 7 % slower, 84^3 8 % slower), 4th order also from 128
+// on (128^3 5 %); with the Hall term 4th and 6th order never (97^3 .. 160^3 0-15 % slower with it).  FP32 (evenly divided rows): even
 // rows in which the band is at most a tenth of the row, 2nd order from 96 on (confined Hall 4th
 // order 128^3 +20 %)
 static bool banded(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, ColShape sh, bool hall) {
