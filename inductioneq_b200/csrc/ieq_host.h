@@ -128,7 +128,8 @@ struct ieq_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   size_t n = 0, n_pad = 0, n_groups = 0;
-  int px = 0;                      // row pitch of the fused state (nx, or nx + 1: boxes with odd rows)
+  int px = 0;                      // row pitch of the fused state (nx, or nx + 1: boxes with odd rows;
+                                   // nx within the calls of a stage session)
   size_t soa_n = 0;                // elements of one component plane of the fused state
   int op_id = 0;
   // device tables
