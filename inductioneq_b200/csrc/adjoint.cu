@@ -75,6 +75,8 @@ __device__ __forceinline__ double dot3(V3<double> a, V3<double> b) { return a.x 
 constexpr int kAdjThreads = 128;
 constexpr int pass1_min_blocks(int ri, bool plain) { return plain && ri < 3 ? 5 : 4; }
 
+// (32-bit indices for the records too: every call here holds at least four FP64 fields, two of
+// them its own, and those of 2^31 nodes are 275 GB)
 struct Node {
   int i[3], n[3];
   int st[3], idx;
@@ -800,9 +802,11 @@ int fast_ri(const ieq_ctx *c) {
   return ri;
 }
 
-dim3 ablock() { return dim3(32, 2, 2); }   // kAdjThreads
+// kAdjThreads; deeper in y where two rows a block would be more than 65,535 blocks
+dim3 ablock(const ieq_ctx *c) { return c->s.nodes[1] <= 2 * 65535 ? dim3(32, 2, 2) : dim3(32, 4, 1); }
 dim3 agrid(const ieq_ctx *c) {
-  return dim3((c->s.nodes[0] + 31) / 32, (c->s.nodes[1] + 1) / 2, (c->s.nodes[2] + 1) / 2);
+  const dim3 b = ablock(c);
+  return dim3((c->s.nodes[0] + b.x - 1) / b.x, (c->s.nodes[1] + b.y - 1) / b.y, (c->s.nodes[2] + b.z - 1) / b.z);
 }
 // a vector field in layout F over n elements a component
 template <typename F>
@@ -865,7 +869,7 @@ ieq_status vjp(ieq_ctx *c, F b, F w, F u, const void *rho, F out, F J0, F gJr, c
     adj_curl(c, b, rho, J0);
     a.J0 = J0;
   }
-  const dim3 g = agrid(c), bl = ablock();
+  const dim3 g = agrid(c), bl = ablock(c);
   const bool pdl = c->s.pdl;
   // the instantiations without walls, SAT and runtime branches (measured at kAdjThreads)
   const bool plain = c->s.periodic && c->s.hall && !a.hod && !a.fo && !a.ad && a.w[2] == 0.0 && a.w[4] == 0.0;
@@ -1058,8 +1062,8 @@ ieq_status ieq_operator_jvp(ieq_ctx *c, const void *b, const void *v, const void
     adj_curl(c, a.b0, rho, a.J0);
     adj_curl(c, a.v, rho, a.dJ);
   }
-  if (a.ad) k_jvp<true, F><<<agrid(c), ablock(), 0, c->stream>>>(a);
-  else k_jvp<false, F><<<agrid(c), ablock(), 0, c->stream>>>(a);
+  if (a.ad) k_jvp<true, F><<<agrid(c), ablock(c), 0, c->stream>>>(a);
+  else k_jvp<false, F><<<agrid(c), ablock(c), 0, c->stream>>>(a);
   const cudaError_t e = cudaStreamSynchronize(c->stream);
   free_all(w);
   return e == cudaSuccess ? IEQ_OK : afail(c, IEQ_ERR_CUDA, cudaGetErrorString(e));

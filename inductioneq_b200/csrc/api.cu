@@ -281,8 +281,9 @@ int diss_kind(const Settings &s) {
 
 template <typename R, typename F>
 void launch_stage_any(ieq_ctx *c, const StageArgs<R, F> &a, int conv = -1) {
-  const dim3 b(32, 2, 2);   // kStageThreads
-  const dim3 g((c->s.nodes[0] + 31) / 32, (c->s.nodes[1] + 1) / 2, (c->s.nodes[2] + 1) / 2);
+  // kStageThreads; rows of blocks deeper in y where two nodes each would be more than 65,535
+  const dim3 b = c->s.nodes[1] <= 2 * 65535 ? dim3(32, 2, 2) : dim3(32, 4, 1);
+  const dim3 g((c->s.nodes[0] + b.x - 1) / b.x, (c->s.nodes[1] + b.y - 1) / b.y, (c->s.nodes[2] + b.z - 1) / b.z);
   const bool per = c->s.periodic, hall = c->s.hall;
   const int d = diss_kind(c->s);
   switch (c->op_id) {

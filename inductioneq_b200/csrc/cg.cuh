@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__
       const long long j = (long long)a.nx * row + ix;
       double v = 0.0;
       if (in_yz && ix >= a.off && ix < a.off + a.gx) {
-        const int jb = ix + a.px * row, sy = a.px, sz = a.px * a.ny;
+        const Idx<F> jb = ix + (Idx<F>)a.px * row, sy = a.px, sz = (Idx<F>)a.px * a.ny;
         const double vx = cg_axis<OP>(a, 0, ix, a.nx, [&](int o) { return (double)ldc<R, F>(a.b, jb + o, 0); });
         const double vy = cg_axis<OP>(a, 1, iy, a.ny, [&](int o) { return (double)ldc<R, F>(a.b, jb + o * sy, 1); });
         const double vz = cg_axis<OP>(a, 2, iz, a.nz, [&](int o) { return (double)ldc<R, F>(a.b, jb + o * sz, 2); });
@@ -536,8 +536,8 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__
 
 // B += grad(phi), or B -= grad_adj(phi) (sign = -1, D the adjoint rows), the xyz components
 template <typename R>
-__device__ __forceinline__ void cg_store_xyz(const AoS<R> &f, int j, V3<R> v) {   // .w untouched, as the
-  R *q = reinterpret_cast<R *>(f.p + j);                                          // reference's .xyz store
+__device__ __forceinline__ void cg_store_xyz(const AoS<R> &f, long long j, V3<R> v) {   // .w untouched, as the
+  R *q = reinterpret_cast<R *>(f.p + j);                                                // reference's .xyz store
   if constexpr (sizeof(R) == 8) *reinterpret_cast<double2 *>(q) = make_double2(v.x, v.y);
   else *reinterpret_cast<float2 *>(q) = make_float2(v.x, v.y);
   q[2] = v.z;
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_project(const __grid_constant
   const double gx = cg_axis<OP>(a, 0, ix, a.nx, [&](int o) { return __ldg(p + o); });
   const double gy = cg_axis<OP>(a, 1, iy, a.ny, [&](int o) { return __ldg(p + (long long)o * a.nx); });
   const double gz = cg_axis<OP>(a, 2, iz, a.nz, [&](int o) { return __ldg(p + o * plane); });
-  const int jb = ix + a.px * (iy + a.ny * iz);
+  const Idx<F> jb = ix + (Idx<F>)a.px * (iy + (Idx<F>)a.ny * iz);
   const V3<R> B = ldf_plain(a.b, jb);
   cg_store_xyz(a.b, jb, V3<R>{(R)((double)B.x + a.sign * gx), (R)((double)B.y + a.sign * gy),
                               (R)((double)B.z + a.sign * gz)});

@@ -20,7 +20,7 @@ template <typename R, typename F>
 struct DiagArgs {
   Mesh m;
   F b;
-  int n;
+  long long n;
   const R *wx, *wy, *wz;   // per-axis mass weights (norm2 of kernel_operator.cl)
   const Tables<R> *tab;    // derivative rows (calc_div)
   int periodic;
@@ -33,7 +33,7 @@ struct DiagArgs {
 // d/d(axis) of that axis' component (calc_div, kernel_operator.cl:145): the row's non-zero
 // entries, all loads free to issue before the first sum
 template <typename R, typename F, int OP>
-__device__ __forceinline__ R diag_axis(const DiagArgs<R, F> &a, int ax, int i, int n, int ib, int st) {
+__device__ __forceinline__ R diag_axis(const DiagArgs<R, F> &a, int ax, int i, int n, Idx<F> ib, Idx<F> st) {
   const int row = a.periodic ? Op<OP>::NB : sbp_row(i, n, Op<OP>::NB);
   R v = 0;
 #pragma unroll
@@ -53,12 +53,12 @@ __device__ __forceinline__ R diag_axis(const DiagArgs<R, F> &a, int ax, int i, i
 template <typename R, typename F, int OP>
 __device__ __forceinline__ void diag_node(const DiagArgs<R, F> &a, int ix, int iy, int iz, double &e, double &dv,
                                           double &er, V3<R> &A, R &div, R &fac) {
-  const int ib = ix + a.m.px * (iy + a.m.ny * iz);   // the node in the field's layout
+  const Idx<F> ib = node_at<F>(a.m, ix, iy, iz);
   fac = (a.wx[ix] * a.wy[iy]) * a.wz[iz];
   const V3<R> B = ldf(a.b, ib);
   e += (double)(fac * ((B.x * B.x + B.y * B.y) + B.z * B.z));
   const R dx = diag_axis<R, F, OP>(a, 0, ix, a.m.nx, ib, 1), dy = diag_axis<R, F, OP>(a, 1, iy, a.m.ny, ib, a.m.px),
-          dz = diag_axis<R, F, OP>(a, 2, iz, a.m.nz, ib, a.m.px * a.m.ny);
+          dz = diag_axis<R, F, OP>(a, 2, iz, a.m.nz, ib, (Idx<F>)a.m.px * a.m.ny);
   div = (dx + dy) + dz;
   dv += (double)((fac * div) * div);
   A = b_analytical<R>(a.tc, a.m, ix, iy, iz, a.time ? a.time[0] : a.t);
@@ -73,11 +73,13 @@ __global__ void __launch_bounds__(256) k_diag_partials(const __grid_constant__ D
                                                        int results, R4<R> *va, R *sdiv) {
   __shared__ double sm[4][8];
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  const unsigned nx = a.m.nx, ny = a.m.ny;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)a.n; i += gridDim.x * blockDim.x) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n; i += stride) {
     V3<R> A;
     R div, fac;
-    diag_node<R, F, OP>(a, i % nx, i / nx % ny, i / nx / ny, acc[0], acc[1], acc[2], A, div, fac);
+    int ix, iy, iz;
+    node_position(i, a.m.nx, a.m.ny, ix, iy, iz);
+    diag_node<R, F, OP>(a, ix, iy, iz, acc[0], acc[1], acc[2], A, div, fac);
     if (results) {
       acc[3] += (double)(fac * ((A.x * A.x + A.y * A.y) + A.z * A.z));
       st3(va + i, A);

@@ -154,11 +154,27 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// the position of node i of a field (32-bit divisions as far as they reach: a 64-bit one is some
+// twenty instructions)
+__device__ __forceinline__ void node_position(long long i, int nx, int ny, int &ix, int &iy, int &iz) {
+  if (i >> 32 == 0) {
+    const unsigned k = (unsigned)i, r = k / (unsigned)nx, z = r / (unsigned)ny;
+    ix = (int)(k - r * (unsigned)nx);
+    iy = (int)(r - z * (unsigned)ny);
+    iz = (int)z;
+  } else {
+    const long long r = i / nx;
+    ix = (int)(i - r * nx);
+    iy = (int)(r % ny);
+    iz = (int)(r / ny);
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ double reduce_term(const ReduceArgs<T> &a, long long i) {
   if (a.kind == RED_DOT) return (double)(a.sa[i] * a.sb[i]);
-  const unsigned r = (unsigned)i / a.nx;   // (32-bit division: n < 2^31)
-  const unsigned ix = (unsigned)i - r * a.nx, iz = r / a.ny, iy = r - iz * a.ny;
+  int ix, iy, iz;
+  node_position(i, a.nx, a.ny, ix, iy, iz);
   const T fac = (a.wx[ix] * a.wy[iy]) * a.wz[iz];
   if (a.kind == RED_NORM2_S) return (double)((fac * a.sa[i]) * a.sa[i]);
   V3<T> v = ld3(a.va + i);

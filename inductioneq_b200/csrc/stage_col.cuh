@@ -640,6 +640,10 @@ inline ColShape fit_rows(ColShape sh, int nxe) {
   sh.y = yz / sh.z > 0 ? yz / sh.z : 1;
   return sh;
 }
+// whether a launch of shape sh has at most the 65,535 blocks in y and z that one takes
+inline bool shape_fits(ColShape sh, int ny, int nz) {
+  return (ny + sh.y - 1) / sh.y <= 65535 && (nz + sh.z - 1) / sh.z <= 65535;
+}
 // The pair kernels' shape on a box of more than one round of the GPU: evenly divided rows, or a
 // shape that takes fewer rounds.  A block costs its whole slot of an SM however many of its
 // threads have nodes, and a warp that holds an x boundary lane gathers the x axis node by node:
@@ -673,11 +677,13 @@ inline ColShape wave_shape(ColShape sh, int nxe, int ny, int nz, int resident, b
     for (int z = 2; z >= 1; --z) {
       const int y = kColThreads / (x * z);
       const double c = cost(x, y, z);
-      if (c < best) {
+      ColShape to = sh;
+      to.x = x;
+      to.y = y;
+      to.z = z;
+      if (c < best && shape_fits(to, ny, nz)) {
         best = c;
-        sh.x = x;
-        sh.y = y;
-        sh.z = z;
+        sh = to;
       }
     }
   }

@@ -216,13 +216,13 @@ static void launch_fo_pairs(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, Col
   else launch_pdl(k_stage_col_x2<IEQ_R, IEQ_OP, false, H, false, 1, false, false, 10, false, true>, g2, b2, s, sh.pdl, a);
 }
 
-// the block shape x * y * z unless the settings gave one
-static ColShape shaped(ColShape sh, int x, int y, int z) {
-  if (sh.given) return sh;
-  sh.x = x;
-  sh.y = y;
-  sh.z = z;
-  return sh;
+// the block shape x * y * z, unless the settings gave one or the grid is too long for it
+static ColShape shaped(ColShape sh, const Mesh &m, int x, int y, int z) {
+  ColShape to = sh;
+  to.x = x;
+  to.y = y;
+  to.z = z;
+  return sh.given || !shape_fits(to, m.ny, m.nz) ? sh : to;
 }
 
 template <>
@@ -237,13 +237,13 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
     // 50^3 0.9-1.05x).  CK2N54, 4 steps, rows of 32 / this, 4th order: Hall periodic 64^3 955 /
     // 921 us, 112^3 5216 / 4147; rotation 64^3 1737 / 1433, 97^3 6114 / 4940, 112^3 9847 / 5400.
     // FP32 keeps the rows (0.95-1.3x).
-    const ColShape c = shaped(sh, 8, 8, 2);
+    const ColShape c = shaped(s1, a.m, 8, 8, 2);
     const dim3 gc = col_grid(c, a.m.nx, a.m.ny, a.m.nz, col_nodes(conv));
     if (2ll * gc.x * gc.y * gc.z > 5ll * kSms * foad_min_blocks<IEQ_OP>()) s1 = c;
   } else if (sizeof(IEQ_R) == 8 && !per && !hall && hod && conv && !foad) {
     // half the warps hold an x boundary lane (rotation with high-order dissipation, 40^3 ..
     // 112^3, orders 2/4/6: 1.01-1.21x the speed of rows of 32)
-    s1 = shaped(sh, 16, 4, 2);
+    s1 = shaped(s1, a.m, 16, 4, 2);
   }
   const dim3 g = col_grid(s1, a.m.nx, a.m.ny, a.m.nz, col_nodes(conv)), b = col_block(s1);
   // the precomputed dissipation sum comes with the Hall curl kernel only
@@ -357,7 +357,8 @@ void launch_curl_e<IEQ_R, IEQ_OP>(const CurlArgs<IEQ_R, SoA<IEQ_R>> &a, bool per
                                   cudaStream_t s) {
   // boxes, FP64: half the warps hold an x boundary lane (confined Hall 48^3 .. 128^3, a whole
   // step, 4th and 6th order: 0-3 % faster than rows of 32; 2nd order -1 .. 2 %)
-  const ColShape s1 = sizeof(IEQ_R) == 8 && !per && Op<IEQ_OP>::RI >= 2 ? shaped(sh, 16, 4, 2) : fit_rows(sh, a.m.nx);
+  ColShape s1 = fit_rows(sh, a.m.nx);
+  if (sizeof(IEQ_R) == 8 && !per && Op<IEQ_OP>::RI >= 2) s1 = shaped(s1, a.m, 16, 4, 2);
   const dim3 b = col_block(s1);
   // pairs on periodic grids only (on boxes the x boundary rows run per node and the
   // one-node kernels measured faster)

@@ -64,8 +64,25 @@ __device__ __forceinline__ void stf(const SoAcg<R> &f, long long j, V3<R> v) {
   f.p[j + f.s] = v.y;
   f.p[j + 2 * f.s] = v.z;
 }
-// (offsets of the fused path's nodes are 32-bit: a state of 2^31 nodes does not fit 180 GB; the
-// component bases are uniform, so a load's address is one multiply-add)
+// The type of a node's index.  The fused state's are 32-bit: it holds 27 planes beside the
+// caller's fields, and 2^31 nodes of it do not fit 180 GB (the component bases are uniform, so a
+// load's address is one multiply-add).  A single field of the caller's records has room for
+// more: FP32 records of 2^31 nodes are 34 GB, a curl of them 69 GB.
+template <typename F>
+struct NodeIndex {
+  using T = int;
+};
+template <typename R>
+struct NodeIndex<AoS<R>> {
+  using T = long long;
+};
+template <typename F>
+using Idx = typename NodeIndex<F>::T;
+// node (ix, iy, iz) of a field of layout F
+template <typename F>
+__device__ __forceinline__ Idx<F> node_at(const Mesh &m, int ix, int iy, int iz) {
+  return ix + (Idx<F>)m.px * (iy + (Idx<F>)m.ny * iz);
+}
 template <typename R>
 __device__ __forceinline__ V3<R> ldf(const SoA<R> &f, int j) {
   return {__ldg(f.p + j), __ldg(f.p + f.s + j), __ldg(f.p + 2 * f.s + j)};
@@ -159,7 +176,7 @@ struct AxisSums {
 // this with compile-time knowledge instead (only the centre derivative coefficient is zero)
 template <typename R, typename F, bool HALL, bool HOD, bool CHK>
 __device__ __forceinline__ void accumulate(AxisSums<R> &s, const StageArgs<R, F> &a, int conv, int axis, R cD, R cH,
-                                           int j) {
+                                           Idx<F> j) {
   const V3<R> B = ldf(a.bk, j);
   if (conv && (!CHK || cD != (R)0)) {
     const V3<R> U = ldf(a.u, j);
@@ -189,7 +206,7 @@ __device__ __forceinline__ void accumulate(AxisSums<R> &s, const StageArgs<R, F>
 }
 
 template <typename R, typename F>
-__device__ __forceinline__ R ldc(const F &f, int j, int comp);
+__device__ __forceinline__ R ldc(const F &f, Idx<F> j, int comp);
 template <>
 __device__ __forceinline__ double ldc<double, SoA<double>>(const SoA<double> &f, int j, int comp) {
   return __ldg(f.p + comp * f.s + j);
@@ -199,11 +216,11 @@ __device__ __forceinline__ float ldc<float, SoA<float>>(const SoA<float> &f, int
   return __ldg(f.p + comp * f.s + j);
 }
 template <>
-__device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f, int j, int comp) {
+__device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f, long long j, int comp) {
   return __ldg(reinterpret_cast<const double *>(f.p + j) + comp);
 }
 template <>
-__device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, int j, int comp) {
+__device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, long long j, int comp) {
   return __ldg(reinterpret_cast<const float *>(f.p + j) + comp);
 }
 
@@ -222,7 +239,8 @@ __device__ __forceinline__ double ad_kappa(double s, double lo, double hi, doubl
 // 2 RI + 1 points serve the first-order part and the high-order part, whose pairs lie within
 // them; the two pairs at the node are in both.
 template <typename R, typename F, int OP, bool PER>
-__device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, int i, int n, int idx, int st) {
+__device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, int i, int n, Idx<F> idx,
+                                              Idx<F> st) {
   constexpr int NB = Op<OP>::NB, RI = Op<OP>::RI, WH = Op<OP>::WH;
   static_assert(WH == RI + 1, "the dissipation pairs lie within the derivative's points");
   const bool wrap = PER && (i < RI || i >= n - RI);
@@ -234,7 +252,7 @@ __device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, 
     R b[2 * RI + 1], u[2 * RI + 1], kf[2 * RI + 1];
 #pragma unroll
     for (int o = -RI; o <= RI; ++o) {
-      const int j = wrap ? idx + (nbr<true>(i, o, n) - i) * st : idx + o * st;
+      const Idx<F> j = wrap ? idx + (nbr<true>(i, o, n) - i) * st : idx + o * st;
       b[o + RI] = ldc<R, F>(a.bk, j, c);
       u[o + RI] = fabs(ldc<R, F>(a.u, j, c));
     }
@@ -289,7 +307,7 @@ __device__ __forceinline__ bool ad_test(const V3<R> &b1, const V3<R> &u1, const 
 // from the host, 0.79 with the axes whose kappas are all zero summed in col_axis.)
 template <typename R, typename F, int OP, bool PER>
 __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], const int nn[3],
-                                   const int st[3], int idx, V3<R> Bm, V3<R> um, int skip = 0) {
+                                   const Idx<F> st[3], Idx<F> idx, V3<R> Bm, V3<R> um, int skip = 0) {
   constexpr int NB = Op<OP>::NB, SW = Op<OP>::SW, C0 = (SW - 1) / 2, WH = Op<OP>::WH;
   V3<R> acc = {0, 0, 0};
   const bool adaptive = a.diss_form == 3;
@@ -316,7 +334,7 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
       const int o = c - C0;
       const R cd = fabs(a.tab->D[row][c]);
       if (cd == (R)0) continue;   // a zero coefficient adds a zero term: skip its loads
-      const int j = idx + (nbr<PER>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
+      const Idx<F> j = idx + (nbr<PER>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
       const V3<R> Bk = ldf(a.bk, j);
       const V3<R> uk = ldf(a.u, j);
       V3<R> sg = {fmax(fabs(uk.x), fabs(um.x)), fmax(fabs(uk.y), fabs(um.y)), fmax(fabs(uk.z), fabs(um.z))};
@@ -335,15 +353,15 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
     if (!adaptive) continue;
     // high-order part weighted by (1 - kappa) of the neighbouring pair
     for (int term = -WH + 1; term <= 0; ++term) {
-      const int j1 = idx + (nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
-      const int j2 = idx + (nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
+      const Idx<F> j1 = idx + (nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
+      const Idx<F> j2 = idx + (nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
       const V3<R> b1 = ldf(a.bk, j1), b2 = ldf(a.bk, j2), u1 = ldf(a.u, j1), u2 = ldf(a.u, j2);
       // diff_HOD (artificial_dissipation.h:58-101) for this start offset
       const R sgn = (Op<OP>::ORDER / 2 + 1) % 2 ? (R)-1 : (R)1;
       V3<R> hod = {0, 0, 0};
       for (int i = 0; i < WH; ++i) {
         const R coef = ((a.tab->Minv[row] * a.tab->DHO[row][term + WH - 1]) * a.tab->DHO[NB][i]) * sgn;
-        const int j = idx + (nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
+        const Idx<F> j = idx + (nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
         const V3<R> Bk = ldf(a.bk, j);
         hod.x += coef * Bk.x; hod.y += coef * Bk.y; hod.z += coef * Bk.z;
       }
@@ -381,7 +399,7 @@ __device__ __forceinline__ void sat_inflow_add(const R (&f)[3], const V3<R> &df,
 
 // SAT surface terms on the faces of a non-periodic box (added into db)
 template <typename R, typename F, bool HALL>
-__device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii[3], const int nn[3], int idx,
+__device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii[3], const int nn[3], Idx<F> idx,
                                           const V3<R> &Bm, const V3<R> &um, int conv, V3<R> &db) {
   const int ix = ii[0], iy = ii[1], iz = ii[2], nx = nn[0], ny = nn[1], nz = nn[2];
   const bool face = ix == 0 || iy == 0 || iz == 0 || ix == nx - 1 || iy == ny - 1 || iz == nz - 1;
@@ -454,7 +472,7 @@ struct EpIn {
 };
 
 template <typename R, typename F>
-__device__ __forceinline__ EpIn<R> epilogue_load(const StageArgs<R, F> &a, int idx) {
+__device__ __forceinline__ EpIn<R> epilogue_load(const StageArgs<R, F> &a, Idx<F> idx) {
   EpIn<R> e = {{0, 0, 0}, {0, 0, 0}};
   switch (a.mode) {
     case EP_X_PLUS_HF:
@@ -529,7 +547,7 @@ __device__ __forceinline__ EpOut<R> epilogue_values(const StageArgs<R, F> &a, co
 }
 
 template <typename R, typename F>
-__device__ __forceinline__ void epilogue_store(const StageArgs<R, F> &a, int idx, const V3<R> &db,
+__device__ __forceinline__ void epilogue_store(const StageArgs<R, F> &a, Idx<F> idx, const V3<R> &db,
                                                const EpIn<R> &e) {
   const EpOut<R> r = epilogue_values(a, db, e);
   stf(a.out, idx, r.o1);
@@ -538,7 +556,7 @@ __device__ __forceinline__ void epilogue_store(const StageArgs<R, F> &a, int idx
 }
 
 template <typename R, typename F>
-__device__ __forceinline__ void stage_epilogue(const StageArgs<R, F> &a, int idx, const V3<R> &db) {
+__device__ __forceinline__ void stage_epilogue(const StageArgs<R, F> &a, Idx<F> idx, const V3<R> &db) {
   epilogue_store(a, idx, db, epilogue_load(a, idx));
 }
 
@@ -549,10 +567,10 @@ __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int
   constexpr bool HOD = DISS == DISS_HO;
   const int nx = a.m.nx, ny = a.m.ny, nz = a.m.nz;
   {
-    const int idx = ix + a.m.px * (iy + ny * iz);
+    const Idx<F> idx = node_at<F>(a.m, ix, iy, iz);
     const int ii[3] = {ix, iy, iz};
     const int nn[3] = {nx, ny, nz};
-    const int st[3] = {1, a.m.px, a.m.px * ny};
+    const Idx<F> st[3] = {1, a.m.px, (Idx<F>)a.m.px * ny};
     const int conv = CONV >= 0 ? CONV : (a.conv_flag ? *a.conv_flag : a.conv);
     const V3<R> Bm = ldf(a.bk, idx);
     V3<R> um = {0, 0, 0};
@@ -570,7 +588,7 @@ __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int
         for (int o = -RI; o <= RI; ++o) {
           const R cD = a.Dint[o + RI];
           const R cH = a.Hint[o + RI];
-          int j = idx;
+          Idx<F> j = idx;
           if (o != 0) {
             if (wrap) j = idx + (nbr<true>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
             else j = idx + o * st[ax];
@@ -700,10 +718,10 @@ __global__ void __launch_bounds__(256) k_curl_rho(const __grid_constant__ CurlAr
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
   if (ix >= a.m.nx || iy >= a.m.ny || iz >= a.m.nz) return;
-  const int idx = ix + a.m.px * (iy + a.m.ny * iz);
+  const Idx<F> idx = node_at<F>(a.m, ix, iy, iz);
   const int ii[3] = {ix, iy, iz};
   const int nn[3] = {a.m.nx, a.m.ny, a.m.nz};
-  const int st[3] = {1, a.m.px, a.m.px * a.m.ny};
+  const Idx<F> st[3] = {1, a.m.px, (Idx<F>)a.m.px * a.m.ny};
   R g[3][3];   // g[axis][component]
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
@@ -716,7 +734,7 @@ __global__ void __launch_bounds__(256) k_curl_rho(const __grid_constant__ CurlAr
       for (int o = -RI; o <= RI; ++o) {
         if (o == 0) continue;   // the interior row has a zero centre
         const R c = a.Dint[o + RI];
-        int j;
+        Idx<F> j;
         if (wrap) j = idx + (nbr<true>(ii[ax], o, nn[ax]) - ii[ax]) * st[ax];
         else j = idx + o * st[ax];
         v1 += c * ldc<R, F>(a.b, j, c1);
@@ -726,7 +744,7 @@ __global__ void __launch_bounds__(256) k_curl_rho(const __grid_constant__ CurlAr
 #pragma unroll
       for (int t = 0; t < Op<OP>::ND; ++t) {
         const R c = __ldg(&a.tab->nd[row][t]);
-        const int j = idx + __ldg(&a.tab->nd_off[row][t]) * st[ax];
+        const Idx<F> j = idx + __ldg(&a.tab->nd_off[row][t]) * st[ax];
         R p1 = 0, p2 = 0;
         if (c != (R)0) {
           p1 = ldc<R, F>(a.b, j, c1);
