@@ -1,6 +1,9 @@
 // stage_inst.cuh -- instantiates the stage and curl kernels for one (REAL, operator) pair in
 // both field layouts.  Included by stage_<real>_o<op>.cu with IEQ_R and IEQ_OP defined, so
 // the instantiations compile in parallel.
+#include <climits>
+#include <cstring>
+
 #include "stage_brick.cuh"
 #include "stage_x2.cuh"
 #include "stage_z.cuh"
@@ -36,13 +39,26 @@ static void launch_stage_layout(const StageArgs<IEQ_R, F> &a, bool per, bool hal
 #undef IEQ_L
 }
 
+// whether 32 bits index a grid's nodes, and the arguments of a kernel on records for them
+static bool near_nodes(const Mesh &m) { return (long long)m.nx * m.ny * m.nz <= INT_MAX; }
+template <typename To, typename From>
+static To near_args(const From &a) {
+  static_assert(sizeof(To) == sizeof(From), "the layouts differ in their index type alone");
+  To n;
+  std::memcpy(static_cast<void *>(&n), &a, sizeof(n));
+  return n;
+}
+
 // the per-kernel entry points (AoS) decide the convection switch at run time; the fused
 // path (SoA) knows it before capturing its graph
 template <>
 void launch_stage<IEQ_R, AoS<IEQ_R>, IEQ_OP>(const StageArgs<IEQ_R, AoS<IEQ_R>> &a, bool per, bool hall, int diss,
                                              int conv, dim3 grid, dim3 block, cudaStream_t s) {
   (void)conv;
-  launch_stage_layout<AoS<IEQ_R>, -1>(a, per, hall, diss, grid, block, s);
+  if (near_nodes(a.m))
+    launch_stage_layout<AoSNear<IEQ_R>, -1>(near_args<StageArgs<IEQ_R, AoSNear<IEQ_R>>>(a), per, hall, diss, grid, block, s);
+  else
+    launch_stage_layout<AoS<IEQ_R>, -1>(a, per, hall, diss, grid, block, s);
 }
 template <>
 void launch_stage<IEQ_R, SoA<IEQ_R>, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, bool hall, int diss,
@@ -54,8 +70,14 @@ void launch_stage<IEQ_R, SoA<IEQ_R>, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> 
 template <>
 void launch_curl<IEQ_R, AoS<IEQ_R>, IEQ_OP>(const CurlArgs<IEQ_R, AoS<IEQ_R>> &a, bool per, dim3 grid, dim3 block,
                                             cudaStream_t s) {
-  if (per) k_curl_rho<IEQ_R, AoS<IEQ_R>, IEQ_OP, true><<<grid, block, 0, s>>>(a);
-  else k_curl_rho<IEQ_R, AoS<IEQ_R>, IEQ_OP, false><<<grid, block, 0, s>>>(a);
+  if (near_nodes(a.m)) {
+    const auto n = near_args<CurlArgs<IEQ_R, AoSNear<IEQ_R>>>(a);
+    if (per) k_curl_rho<IEQ_R, AoSNear<IEQ_R>, IEQ_OP, true><<<grid, block, 0, s>>>(n);
+    else k_curl_rho<IEQ_R, AoSNear<IEQ_R>, IEQ_OP, false><<<grid, block, 0, s>>>(n);
+  } else {
+    if (per) k_curl_rho<IEQ_R, AoS<IEQ_R>, IEQ_OP, true><<<grid, block, 0, s>>>(a);
+    else k_curl_rho<IEQ_R, AoS<IEQ_R>, IEQ_OP, false><<<grid, block, 0, s>>>(a);
+  }
 }
 template <>
 void launch_curl<IEQ_R, SoA<IEQ_R>, IEQ_OP>(const CurlArgs<IEQ_R, SoA<IEQ_R>> &a, bool per, dim3 grid, dim3 block,

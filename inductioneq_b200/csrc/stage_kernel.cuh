@@ -67,11 +67,15 @@ __device__ __forceinline__ void stf(const SoAcg<R> &f, long long j, V3<R> v) {
 // The type of a node's index.  The fused state's are 32-bit: it holds 27 planes beside the
 // caller's fields, and 2^31 nodes of it do not fit 180 GB (the component bases are uniform, so a
 // load's address is one multiply-add).  A single field of the caller's records has room for
-// more: FP32 records of 2^31 nodes are 34 GB, a curl of them 69 GB.
+// more: FP32 records of 2^31 nodes are 34 GB, a curl of them 69 GB.  AoSNear is AoS where the
+// grid has fewer nodes, for the stage and curl kernels (with 64-bit indices the stage kernels
+// spill: kernel lists 48^3 443 us against 435).
 template <typename F>
 struct NodeIndex {
   using T = int;
 };
+template <typename R>
+struct AoSNear : AoS<R> {};
 template <typename R>
 struct NodeIndex<AoS<R>> {
   using T = long long;
@@ -222,6 +226,15 @@ __device__ __forceinline__ double ldc<double, AoS<double>>(const AoS<double> &f,
 template <>
 __device__ __forceinline__ float ldc<float, AoS<float>>(const AoS<float> &f, long long j, int comp) {
   return __ldg(reinterpret_cast<const float *>(f.p + j) + comp);
+}
+
+template <>
+__device__ __forceinline__ double ldc<double, AoSNear<double>>(const AoSNear<double> &f, int j, int comp) {
+  return ldc<double, AoS<double>>(f, j, comp);
+}
+template <>
+__device__ __forceinline__ float ldc<float, AoSNear<float>>(const AoSNear<float> &f, int j, int comp) {
+  return ldc<float, AoS<float>>(f, j, comp);
 }
 
 // kappa of adaptive dissipation for one pair (include/artificial_dissipation.h:23-45): s =
