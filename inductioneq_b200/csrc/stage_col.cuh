@@ -125,11 +125,37 @@ __device__ __forceinline__ void col_load(const StageArgs<R, F> &a, int ax, int j
   }
 }
 
+// the high-order row at an interior node of a warp that also holds boundary rows, with the tests
+// and the order of col_axis; whether every kappa is zero.  (Not unrolled: it would take the
+// registers and the instruction cache of the path that most warps run.)
+template <typename R, int OP, typename F>
+__device__ __forceinline__ bool ad_quiet_row(ColSums<R> &s, const StageArgs<R, F> &a, int ax, int idx, int st,
+                                             const V3<R> &Bm, const V3<R> &Um) {
+  constexpr int RI = Op<OP>::RI;
+  V3<R> Bp = Bm, Up = Um;
+#pragma unroll 1
+  for (int o = -RI; o <= RI; ++o) {
+    const V3<R> B = o == 0 ? Bm : ldf(a.bk, idx + o * st);
+    mad3(s.SHo, a.Hint[o + RI], B);
+    if (o == 0) continue;
+    const V3<R> U = ldf(a.u, idx + o * st);
+    if (ad_test(B, U, Bm, Um, __ldg(&a.tab->ad_thr[ax][o < 0 ? -o : o]))) return false;
+    if (o > 1 && ad_test(B, U, Bp, Up, __ldg(&a.tab->ad_thr[ax][1]))) return false;
+    if (o > 0) {
+      Bp = B;
+      Up = U;
+    }
+  }
+  return true;
+}
+
 // the sums of one axis at one node (interior row, periodic wrap or SBP boundary row);
 // NEED >= 0 fixes the flux-form mask (StageArgs::need) at compile time
 // FOF: also the first-order dissipation terms of the axis (*Um: u at the node)
-// AD: adaptive dissipation -- on the interior row, where every kappa of the warp's nodes is
-// zero, it is the high-order row, summed here (*quiet = true); else the caller adds the axis
+// AD: adaptive dissipation -- on the interior row, where every kappa of the node is zero, it is
+// the high-order row, summed here (*quiet = true); else the caller adds the axis.  That goes by
+// the node, whatever else its warp holds: a node's sum must not depend on the block shape or on
+// the warp's other nodes, or a z slab would differ from the whole grid in its last bits
 template <typename R, int OP, bool PER, bool HALL, bool HOD, int CONV, typename F = SoA<R>, int NEED = -1,
           bool FOF = false, bool AD = false>
 __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a, int ax, int i, int n,
@@ -149,7 +175,11 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
         // the interior derivative rows have a zero centre
         if (HOD) col_acc<R, false, HOD, 0>(s, ax, 0, (R)0, a.Hint[RI], false, true, Bm, zero, (R)0, (R)0);
         if (AD) {
-          s.SHo.x += a.Hint[RI] * Bm.x; s.SHo.y += a.Hint[RI] * Bm.y; s.SHo.z += a.Hint[RI] * Bm.z;
+          if (PER) {   // (nothing to agree with there: written out, it spills 130 bytes more)
+            s.SHo.x += a.Hint[RI] * Bm.x; s.SHo.y += a.Hint[RI] * Bm.y; s.SHo.z += a.Hint[RI] * Bm.z;
+          } else {
+            mad3(s.SHo, a.Hint[RI], Bm);
+          }
         }
         continue;
       }
@@ -161,7 +191,11 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
       if (FOF) fo_acc(s, a.Dint[o + RI], B, U, Bm, *Um);
       if (AD) {
         const R cH = a.Hint[o + RI];
-        s.SHo.x += cH * B.x; s.SHo.y += cH * B.y; s.SHo.z += cH * B.z;
+        if (PER) {
+          s.SHo.x += cH * B.x; s.SHo.y += cH * B.y; s.SHo.z += cH * B.z;
+        } else {
+          mad3(s.SHo, cH, B);
+        }
         loud = ad_test(B, U, Bm, *Um, __ldg(&a.tab->ad_thr[ax][o < 0 ? -o : o])) || loud;
         if (o > 1) loud = ad_test(B, U, Bp, Up, __ldg(&a.tab->ad_thr[ax][1])) || loud;
         if (o > 0) {
@@ -170,9 +204,8 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
         }
       }
     }
-    if (AD) *quiet = !__any_sync(__activemask(), loud);
+    if (AD) *quiet = !loud;
   } else {
-    if (AD) *quiet = false;
     // boundary rows, and every row of a warp that holds one: the row's non-zero entries, all
     // loads free to issue before the first sum (as a run-time loop over the columns with a
     // test per column the loads came one at a time).  Padding entries load nothing, add zeros
@@ -188,6 +221,7 @@ __device__ __forceinline__ void col_axis(ColSums<R> &s, const StageArgs<R, F> &a
       col_acc<R, HALL, HOD, CONV>(s, ax, need, cD, cH, !HOD || cD != (R)0, cH != (R)0, B, U, e1, e2);
       if (FOF) fo_acc(s, cD, B, U, Bm, *Um);
     }
+    if (AD) *quiet = row == NB && ad_quiet_row<R, OP, F>(s, a, ax, idx, st, Bm, *Um);
   }
 }
 
@@ -202,26 +236,26 @@ __device__ __forceinline__ void col_combine(const StageArgs<R, F> &a, int ax, co
     const R *w = a.w;
     auto term = [&](R SuiBa, R SU, R SB, R SuaB, R B, R U) -> R {
       R p = 0, m = 0;
-      if (NEED & 1) p = w[0] * SuiBa;
-      if (NEED & 2) p = p + w[1] * Ba * SU;
-      if (NEED & 4) p = p + w[2] * U * SBa;
-      if (NEED & 8) m = w[3] * SuaB;
-      if (NEED & 4) m = m + w[4] * Ua * SB;
-      if (NEED & 2) m = m + w[5] * B * SUa;
-      return p - m;
+      if (NEED & 1) p = mul(w[0], SuiBa);
+      if (NEED & 2) p = mad(w[1] * Ba, SU, p);
+      if (NEED & 4) p = mad(w[2] * U, SBa, p);
+      if (NEED & 8) m = mul(w[3], SuaB);
+      if (NEED & 4) m = mad(w[4] * Ua, SB, m);
+      if (NEED & 2) m = mad(w[5] * B, SUa, m);
+      return sub(p, m);
     };
-    db.x += a.two_inv_d[ax] * term(s.SuiBa.x, s.SU.x, s.SB.x, s.SuaB.x, Bm.x, um.x);
-    db.y += a.two_inv_d[ax] * term(s.SuiBa.y, s.SU.y, s.SB.y, s.SuaB.y, Bm.y, um.y);
-    db.z += a.two_inv_d[ax] * term(s.SuiBa.z, s.SU.z, s.SB.z, s.SuaB.z, Bm.z, um.z);
+    db.x = mad(a.two_inv_d[ax], term(s.SuiBa.x, s.SU.x, s.SB.x, s.SuaB.x, Bm.x, um.x), db.x);
+    db.y = mad(a.two_inv_d[ax], term(s.SuiBa.y, s.SU.y, s.SB.y, s.SuaB.y, Bm.y, um.y), db.y);
+    db.z = mad(a.two_inv_d[ax], term(s.SuiBa.z, s.SU.z, s.SB.z, s.SuaB.z, Bm.z, um.z), db.z);
   }
   if (HALL) {
-    const R f1 = a.inv_d[ax] * s.h1, f2 = a.inv_d[ax] * s.h2;
+    const R d = a.inv_d[ax];
     if (ax == 0) {
-      db.y += f1; db.z += f2;
+      db.y = mad(d, s.h1, db.y); db.z = mad(d, s.h2, db.z);
     } else if (ax == 1) {
-      db.x -= f1; db.z += f2;
+      db.x = mad(-d, s.h1, db.x); db.z = mad(d, s.h2, db.z);
     } else {
-      db.x -= f1; db.y -= f2;
+      db.x = mad(-d, s.h1, db.x); db.y = mad(-d, s.h2, db.y);
     }
   }
   if (HOD) {
@@ -358,9 +392,7 @@ __global__ void __launch_bounds__(kColThreads, (FOAD ? foad_min_blocks<OP>() : C
         if (!PER) stage_sat<R, SoA<R>, HALL>(a, ii, nn, idx, Bm[k], um[k], CONV, d);
         if (HOD_) {
           const V3<R> hv = HODP ? ldf(a.Hpre, idx) : hod[k];
-          d.x += a.hod_factor * hv.x;
-          d.y += a.hod_factor * hv.y;
-          d.z += a.hod_factor * hv.z;
+          mad3(d, a.hod_factor, hv);
         }
         if (FOF) {
           d.x += fo.x; d.y += fo.y; d.z += fo.z;
@@ -370,9 +402,7 @@ __global__ void __launch_bounds__(kColThreads, (FOAD ? foad_min_blocks<OP>() : C
             const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, PER>(a, ii, nn, st, idx, Bm[k], um[k], quiet_axes);
             d.x += ds.x; d.y += ds.y; d.z += ds.z;
           }
-          d.x += a.hod_factor * quiet_sum.x;
-          d.y += a.hod_factor * quiet_sum.y;
-          d.z += a.hod_factor * quiet_sum.z;
+          mad3(d, a.hod_factor, quiet_sum);
         }
         stage_epilogue<R, SoA<R>>(a, idx, d);
       }

@@ -106,6 +106,25 @@ __device__ __forceinline__ void stf(const SoA<R> &f, int j, V3<R> v) {
   (f.p + 2 * f.s)[j] = v.z;
 }
 
+// Rounding written out: a b + c in one rounding, a b and a - b each in their own.  A sum s += c v
+// is always one rounding, but which product of two is contracted, and whether one is contracted
+// at all into a sum that stands elsewhere, depends on the kernel around it.  The stage kernels
+// must round alike whichever of them runs a node, or a z slab would differ from the whole grid in
+// its last bits: what follows the sums over a stencil uses these.
+__device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
+// s += a v, by component
+template <typename R>
+__device__ __forceinline__ void mad3(V3<R> &s, R a, const V3<R> &v) {
+  s.x = mad(a, v.x, s.x);
+  s.y = mad(a, v.y, s.y);
+  s.z = mad(a, v.z, s.z);
+}
+
 enum EpilogueMode : int {
   EP_X_PLUS_HF = 0,   // out = X + h*F                 SSPRK33_1, SSPRK104, KCL_5, CFR_6
   EP_PX_QYHF = 1,     // out = p*X + q*(Y + h*F)       SSPRK33_2b/3b, SSPRK104_11b
@@ -242,7 +261,7 @@ __device__ __forceinline__ float ldc<float, AoSNear<float>>(const AoSNear<float>
 // between them.  (0 * s carries a NaN, as there.)
 __device__ __forceinline__ double ad_kappa(double s, double lo, double hi, double inv) {
   if (s >= hi) return 1.0 + 0.0 * s;
-  if (s > lo) return sqrt((s - lo) * inv);
+  if (s > lo) return sqrt(sub(s, lo) * inv);
   return 0.0 * s;
 }
 
@@ -250,7 +269,8 @@ __device__ __forceinline__ double ad_kappa(double s, double lo, double hi, doubl
 // row, one component at a time (the loop is not unrolled: a warp comes here only where some
 // kappa is not zero, and 60 inlined kappas would crowd out the rest of the kernel's code).  The
 // 2 RI + 1 points serve the first-order part and the high-order part, whose pairs lie within
-// them; the two pairs at the node are in both.
+// them; the two pairs at the node are in both.  Every operation is that of fo_ad_dissipation's
+// general path, which interior nodes of a warp with boundary rows take.
 template <typename R, typename F, int OP, bool PER>
 __device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, int i, int n, Idx<F> idx,
                                               Idx<F> st) {
@@ -278,7 +298,7 @@ __device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, 
       const R sg = fmax(u[o + RI], u[RI]), d = b[o + RI] - b[RI];
       kf[o + RI] = (R)ad_kappa((double)((sg * d) * d), __ldg(&a.tab->ad_lo[ax][k]), __ldg(&a.tab->ad_hi[ax][k]),
                                __ldg(&a.tab->ad_inv[ax][k]));
-      fo += ((fabs(a.Dint[o + RI]) * kf[o + RI]) * sg) * d;
+      fo = mad((fabs(a.Dint[o + RI]) * kf[o + RI]) * sg, d, fo);
     }
     // high-order part: (1 - kappa) of the pair (e, e - 1) weights the difference that starts
     // at e - RI (interior row: M_INV = 1, D_HO integer)
@@ -286,7 +306,7 @@ __device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, 
     for (int e = 0; e <= RI; ++e) {
       R h = 0;
 #pragma unroll
-      for (int k = 0; k < WH; ++k) h += __ldg(&a.tab->DHO[NB][k]) * b[e + k];
+      for (int k = 0; k < WH; ++k) h = mad(__ldg(&a.tab->DHO[NB][k]), b[e + k], h);
       R kap;
       if (e == 0) kap = kf[RI - 1];
       else if (e == 1) kap = kf[RI + 1];
@@ -294,7 +314,7 @@ __device__ __forceinline__ V3<R> ad_axis_full(const StageArgs<R, F> &a, int ax, 
         const R sg = fmax(u[RI + e], u[RI + e - 1]), d = b[RI + e] - b[RI + e - 1];
         kap = (R)ad_kappa((double)((sg * d) * d), lo1, hi1, inv1);
       }
-      ho += (((R)1 - kap) * a.hod_factor) * ((__ldg(&a.tab->DHO[NB][e]) * sgn) * h);
+      ho = mad(((R)1 - kap) * a.hod_factor, (__ldg(&a.tab->DHO[NB][e]) * sgn) * h, ho);
     }
     const R v = fo / a.dR[ax] + ho;
     if (c == 0) out.x = v;
@@ -314,7 +334,8 @@ __device__ __forceinline__ bool ad_test(const V3<R> &b1, const V3<R> &u1, const 
 
 // first-order / adaptive dissipation (artificial_dissipation.cl:36-160), evaluated as in
 // the reference per stencil point; used only by the DISS_FO_OR_AD instantiation.  Axes in `skip`
-// are left out; adaptive axes on which the whole warp sits on the interior row take ad_axis_full.
+// are left out; adaptive axes on which the whole warp sits on the interior row take ad_axis_full,
+// which rounds alike.
 // (Hall periodic 64^3 with a current sheet, adaptive, 4th order, 20 stages: 2.37 ms with every
 // kappa evaluated from the table rows, 0.92 with the interior points loaded once and thresholds
 // from the host, 0.79 with the axes whose kappas are all zero summed in col_axis.)
@@ -328,10 +349,9 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
     const R s = (fmax(fabs(u1), fabs(u2)) * (b1 - b2)) * (b1 - b2);
     k = k + (k == 0);
     const double kk = (double)(k * k);
-    const double lo = ((kk * a.mp2min) * a.cmin) * (double)dx;
-    const double hi = ((kk * a.mp2max) * a.cmax) * (double)dx;
-    const double sd = (double)s;
-    return (R)(((lo < sd) && (sd < hi)) * sqrt(fabs(sd - lo) / fabs(hi - lo)) + (double)(sd >= hi));
+    const double lo = mul(mul(mul(kk, a.mp2min), a.cmin), (double)dx);
+    const double hi = mul(mul(mul(kk, a.mp2max), a.cmax), (double)dx);
+    return (R)ad_kappa((double)s, lo, hi, 1.0 / fabs(hi - lo));
   };
 #pragma unroll 1
   for (int ax = 0; ax < 3; ++ax) {
@@ -353,35 +373,39 @@ __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], co
       V3<R> sg = {fmax(fabs(uk.x), fabs(um.x)), fmax(fabs(uk.y), fabs(um.y)), fmax(fabs(uk.z), fabs(um.z))};
       if (adaptive) {
         const unsigned k = (unsigned)(o < 0 ? -o : o);
-        tmp.x += ((cd * kap(k, a.dR[ax], Bk.x, Bm.x, uk.x, um.x)) * sg.x) * (Bk.x - Bm.x);
-        tmp.y += ((cd * kap(k, a.dR[ax], Bk.y, Bm.y, uk.y, um.y)) * sg.y) * (Bk.y - Bm.y);
-        tmp.z += ((cd * kap(k, a.dR[ax], Bk.z, Bm.z, uk.z, um.z)) * sg.z) * (Bk.z - Bm.z);
+        tmp.x = mad((cd * kap(k, a.dR[ax], Bk.x, Bm.x, uk.x, um.x)) * sg.x, Bk.x - Bm.x, tmp.x);
+        tmp.y = mad((cd * kap(k, a.dR[ax], Bk.y, Bm.y, uk.y, um.y)) * sg.y, Bk.y - Bm.y, tmp.y);
+        tmp.z = mad((cd * kap(k, a.dR[ax], Bk.z, Bm.z, uk.z, um.z)) * sg.z, Bk.z - Bm.z, tmp.z);
       } else {
         tmp.x += (cd * sg.x) * (Bk.x - Bm.x);
         tmp.y += (cd * sg.y) * (Bk.y - Bm.y);
         tmp.z += (cd * sg.z) * (Bk.z - Bm.z);
       }
     }
-    acc.x += tmp.x / a.dR[ax]; acc.y += tmp.y / a.dR[ax]; acc.z += tmp.z / a.dR[ax];
-    if (!adaptive) continue;
+    const V3<R> fo = {tmp.x / a.dR[ax], tmp.y / a.dR[ax], tmp.z / a.dR[ax]};
+    if (!adaptive) {
+      acc.x += fo.x; acc.y += fo.y; acc.z += fo.z;
+      continue;
+    }
     // high-order part weighted by (1 - kappa) of the neighbouring pair
+    V3<R> ho = {0, 0, 0};
     for (int term = -WH + 1; term <= 0; ++term) {
       const Idx<F> j1 = idx + (nbr<PER>(ii[ax], term + WH - 1, nn[ax]) - ii[ax]) * st[ax];
       const Idx<F> j2 = idx + (nbr<PER>(ii[ax], term + WH - 2, nn[ax]) - ii[ax]) * st[ax];
       const V3<R> b1 = ldf(a.bk, j1), b2 = ldf(a.bk, j2), u1 = ldf(a.u, j1), u2 = ldf(a.u, j2);
       // diff_HOD (artificial_dissipation.h:58-101) for this start offset
       const R sgn = (Op<OP>::ORDER / 2 + 1) % 2 ? (R)-1 : (R)1;
+      const R c = (a.tab->Minv[row] * a.tab->DHO[row][term + WH - 1]) * sgn;
       V3<R> hod = {0, 0, 0};
       for (int i = 0; i < WH; ++i) {
-        const R coef = ((a.tab->Minv[row] * a.tab->DHO[row][term + WH - 1]) * a.tab->DHO[NB][i]) * sgn;
         const Idx<F> j = idx + (nbr<PER>(ii[ax], i + term, nn[ax]) - ii[ax]) * st[ax];
-        const V3<R> Bk = ldf(a.bk, j);
-        hod.x += coef * Bk.x; hod.y += coef * Bk.y; hod.z += coef * Bk.z;
+        mad3(hod, a.tab->DHO[NB][i], ldf(a.bk, j));
       }
-      acc.x += (((R)1 - kap(1, a.dR[ax], b1.x, b2.x, u1.x, u2.x)) * a.hod_factor) * hod.x;
-      acc.y += (((R)1 - kap(1, a.dR[ax], b1.y, b2.y, u1.y, u2.y)) * a.hod_factor) * hod.y;
-      acc.z += (((R)1 - kap(1, a.dR[ax], b1.z, b2.z, u1.z, u2.z)) * a.hod_factor) * hod.z;
+      ho.x = mad(((R)1 - kap(1, a.dR[ax], b1.x, b2.x, u1.x, u2.x)) * a.hod_factor, c * hod.x, ho.x);
+      ho.y = mad(((R)1 - kap(1, a.dR[ax], b1.y, b2.y, u1.y, u2.y)) * a.hod_factor, c * hod.y, ho.y);
+      ho.z = mad(((R)1 - kap(1, a.dR[ax], b1.z, b2.z, u1.z, u2.z)) * a.hod_factor, c * hod.z, ho.z);
     }
+    acc.x += fo.x + ho.x; acc.y += fo.y + ho.y; acc.z += fo.z + ho.z;
   }
   return acc;
 }
@@ -406,7 +430,7 @@ __device__ __forceinline__ void sat_inflow_add(const R (&f)[3], const V3<R> &df,
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
     if (f[ax] == (R)0) continue;
-    db.x += f[ax] * df.x; db.y += f[ax] * df.y; db.z += f[ax] * df.z;
+    mad3(db, f[ax], df);
   }
 }
 
@@ -420,7 +444,7 @@ __device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii
     if (HALL) {
       // induction_Eq_surface.cl:35-81 (outflow, directional do-nothing)
       const V3<R> Jm = ldf(a.J, idx);
-      const V3<R> tv = {(R)0.5 * um.x - Jm.x, (R)0.5 * um.y - Jm.y, (R)0.5 * um.z - Jm.z};
+      const V3<R> tv = {mad((R)0.5, um.x, -Jm.x), mad((R)0.5, um.y, -Jm.y), mad((R)0.5, um.z, -Jm.z)};
       for (int ax = 0; ax < 3; ++ax) {
         const bool l = ii[ax] == 0, r = ii[ax] == nn[ax] - 1;
         if (!l && !r) continue;
@@ -429,15 +453,14 @@ __device__ __forceinline__ void stage_sat(const StageArgs<R, F> &a, const int ii
         const R c1 = (l && tva > (R)0 ? (R)-1 : (R)0) + (r && tva < (R)0 ? (R)1 : (R)0);
         const R c2 = (l ? (R)-1 : (R)0) + (r ? (R)1 : (R)0);
         const R f1 = c1 * tva, f2 = c2 * Ba;
-        db.x += a.sat_s[ax] * (f1 * Bm.x + f2 * Jm.x);
-        db.y += a.sat_s[ax] * (f1 * Bm.y + f2 * Jm.y);
-        db.z += a.sat_s[ax] * (f1 * Bm.z + f2 * Jm.z);
+        mad3(db, a.sat_s[ax],
+             V3<R>{mad(f1, Bm.x, mul(f2, Jm.x)), mad(f1, Bm.y, mul(f2, Jm.y)), mad(f1, Bm.z, mul(f2, Jm.z))});
       }
     } else if (conv) {
       R f[3];
       if (sat_inflow(a, ii, nn, um, f)) {
         const V3<R> bb = b_boundary<R>(a.tc, a.m, ix, iy, iz, a.time[1]);
-        sat_inflow_add(f, V3<R>{Bm.x - bb.x, Bm.y - bb.y, Bm.z - bb.z}, db);
+        sat_inflow_add(f, V3<R>{sub(Bm.x, bb.x), sub(Bm.y, bb.y), sub(Bm.z, bb.z)}, db);
       }
     }
   }
@@ -465,7 +488,7 @@ __device__ __forceinline__ void stage_sat_pair(const StageArgs<R, F> &a, int ix,
     const V3<R> B = k ? Bm[1] : Bm[0];
     V3<R> d = k ? db[1] : db[0];
     const R f[3] = {k ? f1[0] : f0[0], k ? f1[1] : f0[1], k ? f1[2] : f0[2]};
-    sat_inflow_add(f, V3<R>{B.x - bb.x, B.y - bb.y, B.z - bb.z}, d);
+    sat_inflow_add(f, V3<R>{sub(B.x, bb.x), sub(B.y, bb.y), sub(B.z, bb.z)}, d);
     if (k) {
       db[1] = d;
       break;
@@ -526,32 +549,32 @@ __device__ __forceinline__ EpOut<R> epilogue_values(const StageArgs<R, F> &a, co
   EpOut<R> r = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   switch (a.mode) {
     case EP_X_PLUS_HF:
-      r.o1 = V3<R>{X.x + a.h * db.x, X.y + a.h * db.y, X.z + a.h * db.z};
+      r.o1 = V3<R>{mad(a.h, db.x, X.x), mad(a.h, db.y, X.y), mad(a.h, db.z, X.z)};
       break;
     case EP_PX_QYHF:
-      r.o1 = V3<R>{a.p * X.x + a.q * (Y.x + a.h * db.x), a.p * X.y + a.q * (Y.y + a.h * db.y),
-                   a.p * X.z + a.q * (Y.z + a.h * db.z)};
+      r.o1 = V3<R>{mad(a.p, X.x, mul(a.q, mad(a.h, db.x, Y.x))), mad(a.p, X.y, mul(a.q, mad(a.h, db.y, Y.y))),
+                   mad(a.p, X.z, mul(a.q, mad(a.h, db.z, Y.z)))};
       break;
     case EP_HF:
-      r.o1 = V3<R>{a.h * db.x, a.h * db.y, a.h * db.z};
+      r.o1 = V3<R>{mul(a.h, db.x), mul(a.h, db.y), mul(a.h, db.z)};
       break;
     case EP_AX_HF:
-      r.o1 = V3<R>{a.A * X.x + a.h * db.x, a.A * X.y + a.h * db.y, a.A * X.z + a.h * db.z};
+      r.o1 = V3<R>{mad(a.A, X.x, mul(a.h, db.x)), mad(a.A, X.y, mul(a.h, db.y)), mad(a.A, X.z, mul(a.h, db.z))};
       break;
     case EP_2N_FUSED:
     case EP_2N_FUSED_FIRST: {
       V3<R> t;
-      if (a.mode == EP_2N_FUSED) t = {a.A * X.x + a.h * db.x, a.A * X.y + a.h * db.y, a.A * X.z + a.h * db.z};
-      else t = {a.h * db.x, a.h * db.y, a.h * db.z};
+      t = {mul(a.h, db.x), mul(a.h, db.y), mul(a.h, db.z)};
+      if (a.mode == EP_2N_FUSED) t = {mad(a.A, X.x, t.x), mad(a.A, X.y, t.y), mad(a.A, X.z, t.z)};
       r.o1 = t;
-      r.o2 = V3<R>{Y.x + a.Bc * t.x, Y.y + a.Bc * t.y, Y.z + a.Bc * t.z};
+      r.o2 = V3<R>{mad(a.Bc, t.x, Y.x), mad(a.Bc, t.y, Y.y), mad(a.Bc, t.z, Y.z)};
       break;
     }
     case EP_2R_FUSED: {
-      const V3<R> t = {a.h * db.x, a.h * db.y, a.h * db.z};
-      const V3<R> o = {X.x + a.A * t.x, X.y + a.A * t.y, X.z + a.A * t.z};
+      const V3<R> t = {mul(a.h, db.x), mul(a.h, db.y), mul(a.h, db.z)};
+      const V3<R> o = {mad(a.A, t.x, X.x), mad(a.A, t.y, X.y), mad(a.A, t.z, X.z)};
       r.o1 = o;
-      r.o2 = V3<R>{o.x + a.Bc * t.x, o.y + a.Bc * t.y, o.z + a.Bc * t.z};
+      r.o2 = V3<R>{mad(a.Bc, t.x, o.x), mad(a.Bc, t.y, o.y), mad(a.Bc, t.z, o.z)};
       r.o3 = t;
       break;
     }
@@ -650,9 +673,7 @@ __device__ __forceinline__ void stage_node(const StageArgs<R, F> &a, int ix, int
     }
     if (!PER) stage_sat<R, F, HALL>(a, ii, nn, idx, Bm, um, conv, db);
     if (HOD) {
-      db.x += a.hod_factor * hod.x;
-      db.y += a.hod_factor * hod.y;
-      db.z += a.hod_factor * hod.z;
+      mad3(db, a.hod_factor, hod);
     }
     if (DISS == DISS_FO_OR_AD) {
       const V3<R> ds = fo_ad_dissipation<R, F, OP, PER>(a, ii, nn, st, idx, Bm, um);

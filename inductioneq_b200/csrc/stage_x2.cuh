@@ -601,9 +601,7 @@ __global__ void __launch_bounds__(kColThreads, K == 4 ? IEQ_STAGE_X4_MIN_BLOCKS 
         stage_sat<R, SoA<R>, true>(a, iik, nn, idx + k, ldf(a.bk, idx + k), zero, 0, db[k]);
       }
       if (HODP) {
-        db[k].x += a.hod_factor * hv[k].x;
-        db[k].y += a.hod_factor * hv[k].y;
-        db[k].z += a.hod_factor * hv[k].z;
+        mad3(db[k], a.hod_factor, hv[k]);
       }
     }
     stage_epilogue_k<R, K>(a, idx, db);
@@ -843,9 +841,7 @@ __global__ void __launch_bounds__(kColThreads, FOF ? fo_min_blocks<OP, PER>()
       const int ii[3] = {ix + k, iy, iz};
       if (!PER && HALL && ix + k < nx) stage_sat<R, SoA<R>, HALL>(a, ii, nn, idx + k, Bm[k], um[k], CONV, db[k]);
       if (HOD_) {
-        db[k].x += a.hod_factor * hv[k].x;
-        db[k].y += a.hod_factor * hv[k].y;
-        db[k].z += a.hod_factor * hv[k].z;
+        mad3(db[k], a.hod_factor, hv[k]);
       }
       if (FOAD) {
         const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, PER>(a, ii, nn, st, idx + k, Bm[k], um[k]);
@@ -883,9 +879,7 @@ __device__ __forceinline__ void col_stage_node(const StageArgs<R, SoA<R>> &a, in
   stage_sat<R, SoA<R>, HALL>(a, ii, nn, idx, Bm, um, CONV, db);
   if (HOD_) {
     const V3<R> hv = HODP ? ldf(a.Hpre, idx) : hod;
-    db.x += a.hod_factor * hv.x;
-    db.y += a.hod_factor * hv.y;
-    db.z += a.hod_factor * hv.z;
+    mad3(db, a.hod_factor, hv);
   }
   if (FOAD) {
     const V3<R> ds = fo_ad_dissipation<R, SoA<R>, OP, false>(a, ii, nn, st, idx, Bm, um);
