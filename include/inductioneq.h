@@ -176,6 +176,14 @@ ieq_status ieq_check_finite(ieq_ctx *ctx, const void *vec_field);
  * the context's results are then undefined and it should be destroyed. */
 ieq_status ieq_test_brick_wait(ieq_ctx *ctx, int first_wait_gives_up);
 
+/* Test hook of the grid barriers of the divergence cleaning's CG loop: they then wait for
+ * `extra_arrivals` blocks beyond the grid (1: a block that never comes, so that every wait runs
+ * out) with a limit of `spin_limit` polls (<= 0: the default, a few seconds).  A cleaning whose
+ * barrier gives up leaves the field as it is and returns IEQ_ERR_TIMEOUT; the time loop with
+ * cleaning goes on without it and returns that in the end.  (0, 0) restores the production
+ * barrier. */
+ieq_status ieq_test_cg_barrier(ieq_ctx *ctx, int extra_arrivals, long long spin_limit);
+
 /* The reference kernel list of one time step of the configured integrator, as the MATLAB
  * host builds it (compute_numerical_solution_setup.m:140-371): names separated by '\n'
  * written to `names` (NUL-terminated; `capacity` bytes) and their number to *count.  With

@@ -68,12 +68,14 @@ struct CgLoopArgs {
   int max_it;
   int first;             // 1: the loop starts here (rr from rr0), 0: it goes on from *cs
   int launch_it;         // iterations this launch may do
+  unsigned extra;        // arrivals its barriers wait for beyond the grid (0; a test sets 1 to
+  long long spin_limit;  // make every wait run out) and the polls of a wait before it gives up
   int tiles_x, tiles_y, chunks, tz;
 };
 
 // every block of the (cooperative) launch arrives; false if the wait gave up.  The
 // arrival releases the block's earlier writes, the poll acquires those of every block.
-__device__ __forceinline__ bool cg_barrier(CgSync *s, unsigned &target) {
+__device__ __forceinline__ bool cg_barrier(CgSync *s, unsigned &target, unsigned extra, long long spin_limit) {
   __shared__ int ok;
   target += gridDim.x;
   __syncthreads();
@@ -81,14 +83,14 @@ __device__ __forceinline__ bool cg_barrier(CgSync *s, unsigned &target) {
     ok = 1;
     unsigned n;
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(n) : "l"(&s->arrived) : "memory");
-    if (n + 1u == target) {
+    if (n + 1u == target + extra) {
       asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&s->released), "r"(target) : "memory");
     } else {
       for (long long spins = 0;; ++spins) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&s->released) : "memory");
         if (n == target) break;
         if (spins > 256) {
-          if (*(volatile int *)&s->timeout || spins > kCgSpinLimit) {
+          if (*(volatile int *)&s->timeout || spins > spin_limit) {
             *(volatile int *)&s->timeout = 1;
             ok = 0;
             break;
@@ -432,15 +434,15 @@ __global__ void __launch_bounds__(kCgThreads, cg_min_blocks<W>()) k_cg_loop(cons
   CgItem<W> item;
   const bool many = a.tiles_x * a.tiles_y * a.chunks > (int)gridDim.x;
   if (!many) item.set(a, blockIdx.x);
-  bool ok = cg_barrier(a.sync, target);
+  bool ok = cg_barrier(a.sync, target, a.extra, a.spin_limit);
   for (int k = 0; ok && k < a.launch_it && rr > a.tol && it < a.max_it; ++k) {
     const double *uo = (it & 1) ? a.u1 : a.u0;
     double *un = (it & 1) ? a.u0 : a.u1;
     cg_block_partial(cg_pass_a<W>(a, item, many, uo, un, rr / old, pl, tab), a.partials_a);
-    if (!(ok = cg_barrier(a.sync, target))) break;
+    if (!(ok = cg_barrier(a.sync, target, a.extra, a.spin_limit))) break;
     const double alpha = rr / cg_total(a.partials_a, gridDim.x);
     cg_block_partial(cg_pass_b<W>(a, un, alpha), a.partials_b);
-    if (!(ok = cg_barrier(a.sync, target))) break;
+    if (!(ok = cg_barrier(a.sync, target, a.extra, a.spin_limit))) break;
     old = rr;
     rr = cg_total(a.partials_b, gridDim.x);
     ++it;
@@ -534,7 +536,8 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_begin(const __grid_constant__
   cg_block_partial(rr, a.partials);
 }
 
-// B += grad(phi), or B -= grad_adj(phi) (sign = -1, D the adjoint rows), the xyz components
+// B += grad(phi), or B -= grad_adj(phi) (sign = -1, D the adjoint rows), the xyz components.  B
+// stays as it is if a barrier of the loop gave up: phi is then a part of an iteration
 template <typename R>
 __device__ __forceinline__ void cg_store_xyz(const AoS<R> &f, long long j, V3<R> v) {   // .w untouched, as the
   R *q = reinterpret_cast<R *>(f.p + j);                                                // reference's .xyz store
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_project(const __grid_constant
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z * blockDim.z + threadIdx.z;
-  if (ix >= a.nx || iy >= a.ny || iz >= a.nz) return;
+  if (ix >= a.nx || iy >= a.ny || iz >= a.nz || a.sync->timeout) return;
   const long long plane = (long long)a.nx * a.ny, j = ix + (long long)a.nx * iy + plane * iz;
   const double *p = a.phi + j;
   const double gx = cg_axis<OP>(a, 0, ix, a.nx, [&](int o) { return __ldg(p + o); });

@@ -150,6 +150,8 @@ struct ieq_ctx {
   int last_conv = 1;               // whether the last fused call found u non-zero
   void *d_cg = nullptr;            // CgDevice (the CG loop's state)
   int cg_resident = 0;             // resident blocks of the CG loop kernel (0: not asked yet)
+  int cg_extra = 0;                // ieq_test_cg_barrier: arrivals beyond the grid ...
+  long long cg_spin_limit = 0;     // ... and polls of a wait (0: kCgSpinLimit)
   double *d_cg_vec = nullptr;      // FP64 CG vectors: div, phi, r, u, u', lap (6 x n_pad)
   double *d_cg_hist = nullptr;
   double *d_lap_s = nullptr;       // the CG Laplacian's rows divided by DX^2, DY^2, DZ^2

@@ -88,6 +88,7 @@ def load() -> ctypes.CDLL:
     lib.ieq_compute_results.argtypes = [vp, vp, ctypes.c_double, vp, vp, ctypes.POINTER(ctypes.c_double * 4)]
     lib.ieq_check_finite.argtypes = [vp, vp]
     lib.ieq_test_brick_wait.argtypes = [vp, ctypes.c_int]
+    lib.ieq_test_cg_barrier.argtypes = [vp, ctypes.c_int, ctypes.c_longlong]
     lib.ieq_step_kernels.argtypes = [vp, ctypes.c_char_p, sz, ctypes.POINTER(ctypes.c_int)]
     lib.ieq_stages_begin.argtypes = [vp] * 6 + [ctypes.POINTER(ctypes.c_int)]
     lib.ieq_stages_run.argtypes = [vp, vp, vp, ctypes.c_int]
@@ -352,6 +353,10 @@ class Context:
 
     def check_finite(self, b) -> None:
         self._check(self.lib.ieq_check_finite(self.h, _ptr(b)))
+
+    def test_cg_barrier(self, extra_arrivals: int, spin_limit: int = 0) -> None:
+        """Failure-path test hook of the CG loop's grid barriers (ieq_test_cg_barrier)."""
+        self._check(self.lib.ieq_test_cg_barrier(self.h, int(extra_arrivals), int(spin_limit)))
 
     def test_brick_wait(self, first_wait_gives_up: bool) -> None:
         """Failure-path test hook of the TMA brick kernels' waits (ieq_test_brick_wait)."""
