@@ -915,11 +915,27 @@ struct VjpWork {
   int last = 0;
 };
 constexpr int kVjpFields = 8;
+// which of them a step adjoint of the context's settings works on (a 2N step in l1, an SSPRK33
+// step in l2 and l3, a register program in registers of its own); returns how many
+enum VjpScheme { VJP_SSPRK33, VJP_2N, VJP_PROGRAM };
+int vjp_fields(const ieq_ctx *c, VjpScheme scheme, bool (&use)[kVjpFields]) {
+  const bool hall = c->s.hall;
+  const bool adaptive = c->s.diss_form == 3;
+  use[0] = hall && (!c->s.periodic || adaptive || fast_ri(c) == 0);   // J0: else formed at every node
+  use[1] = use[2] = hall;
+  use[3] = scheme == VJP_2N;
+  use[4] = use[5] = scheme == VJP_SSPRK33;
+  use[6] = use[7] = c->s.variable_u;
+  int n = 0;
+  for (const bool u : use) n += u;
+  return n;
+}
 template <typename F>
-VjpWork<F> vjp_work(const ieq_ctx *c, void *const *f) {
+VjpWork<F> vjp_work(const ieq_ctx *c, const bool (&use)[kVjpFields], void *const *f) {
   VjpWork<F> w;
   F *to[kVjpFields] = {&w.J0, &w.gJr, &w.z, &w.l1, &w.l2, &w.l3, &w.uw[0], &w.uw[1]};
-  for (int k = 0; k < kVjpFields; ++k) *to[k] = MakeField<F>::of(c, f[k]);
+  for (int k = 0; k < kVjpFields; ++k)
+    if (use[k]) *to[k] = MakeField<F>::of(c, *f++);
   return w;
 }
 
@@ -1095,10 +1111,11 @@ ieq_status ieq_ssprk33_step_vjp(ieq_ctx *c, const void *s1, const void *s2, cons
   if (st != IEQ_OK) return st;
   cudaSetDevice(c->device);
   std::vector<void *> f;
-  if ((st = work_alloc(c, f, kVjpFields, c->n_pad * sizeof(R4<double>))) == IEQ_OK) {
+  bool use[kVjpFields];
+  if ((st = work_alloc(c, f, vjp_fields(c, VJP_SSPRK33, use), c->n_pad * sizeof(R4<double>))) == IEQ_OK) {
     using F = AoS<double>;
     auto field = [&](const void *p) { return MakeField<F>::of(c, p); };
-    VjpWork<F> w = vjp_work<F>(c, f.data());
+    VjpWork<F> w = vjp_work<F>(c, use, f.data());
     st = ssprk33_step_vjp_ws(c, field(s1), field(s2), field(s3), t0, field(lambda), field(u), rho, w);
   }
   if (cudaStreamSynchronize(c->stream) != cudaSuccess && st == IEQ_OK) st = afail(c, IEQ_ERR_CUDA, "step vjp");
@@ -1147,8 +1164,9 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   RkProgram prog;
   if (program) rk_step_program(integ, c->s.dt, prog);
   cudaSetDevice(c->device);
-  // a field in either layout
-  const size_t vb = std::max(c->n_pad * sizeof(R4<double>), 3 * c->soa_n * sizeof(double));
+  // planes of the fused state or the caller's records (a context's settings choose one of them)
+  const bool planes = c->s.stage_kernel != 4;
+  const size_t vb = planes ? 3 * c->soa_n * sizeof(double) : c->n_pad * sizeof(R4<double>);
   const int K = checkpoint_every;
   const int nseg = (num_steps + K - 1) / K;
   // states kept per step: SSPRK33 its three stage states, a 2N scheme the input of every stage
@@ -1156,14 +1174,16 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   int S2 = 0;
   if (ck2n || td2n) rk2n_coefficients(ck2n, &A2, &B2, &C2, &S2);
   const int P = program ? prog.evaluations : ssp ? 3 : S2;
-  // checkpoints (nseg), the stage states of one segment (P K), step work (6), step-adjoint
-  // work, the program's adjoint registers L1, L2, LK and a temporary (4)
+  // checkpoints (nseg), the stage states of one segment (P K), lambda in planes or the five
+  // fields of the kernel lists' steps, step-adjoint work, the program's adjoint registers L1,
+  // L2, LK and a temporary (4)
+  bool use[kVjpFields];
+  const int nw = planes ? 1 : 5, nv = vjp_fields(c, program ? VJP_PROGRAM : ssp ? VJP_SSPRK33 : VJP_2N, use);
   std::vector<void *> pool;
-  if ((st = adj_pool(c, (size_t)nseg + (size_t)P * K + 6 + kVjpFields + 4, vb, pool)) != IEQ_OK) return st;
+  if ((st = adj_pool(c, (size_t)nseg + (size_t)P * K + nw + nv + (program ? 4 : 0), vb, pool)) != IEQ_OK) return st;
   std::vector<void *> ck(pool.begin(), pool.begin() + nseg), seg(pool.begin() + nseg, pool.begin() + nseg + P * K);
-  void *const *w = &pool[(size_t)nseg + (size_t)P * K];
-  void *const *vf = w + 6, *const *preg = vf + kVjpFields;   // L1, L2, LK, tmp
-  void *cur = w[0], *b2 = w[1], *b3 = w[2], *cb = w[3], *uw = w[4], *lam = w[5];
+  void *const *w = pool.data() + (size_t)nseg + (size_t)P * K;
+  void *const *vf = w + nw, *const *preg = vf + nv;   // L1, L2, LK, tmp
   double *d_time = c->adj_time;
   std::vector<double> t0s(num_steps + 1, 0.0);
   for (int n = 0; n < num_steps; ++n) t0s[n + 1] = t0s[n] + c->s.dt;   // calc_time_3_args / _2_args
@@ -1188,16 +1208,15 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   // The forward passes run the fused stage kernels (ieq_time_steps' path) and the whole sweep
   // stays in the layout of the fused state; IEQ_STAGE_KERNEL=LIST runs the reference kernel
   // lists on the caller's records instead.
-  if (c->s.stage_kernel != 4) {
+  if (planes) {
     using F = SoA<double>;
-    const size_t sb = 3 * c->soa_n * sizeof(double);
     int conv = 1;
     F b{}, us{};
     const double *rhos = nullptr;
     if ((st = adj_state_begin(c, b0, u, rho, conv, b, us, rhos)) != IEQ_OK) return st;
-    const F lambda_s = MakeField<F>::of(c, lam);
+    const F lambda_s = MakeField<F>::of(c, w[0]);
     adj_to_soa(c, lambda, lambda_s);
-    VjpWork<F> vw = vjp_work<F>(c, vf);
+    VjpWork<F> vw = vjp_work<F>(c, use, vf);
     auto advance = [&](const void *from, double t0, int nsteps, bool keep, double *&end) -> ieq_status {
       set_time(t0);
       return adj_state_steps(c, conv, (const double *)from, rho, d_time, nsteps,
@@ -1205,7 +1224,7 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
     };
     double *at = b.p;
     for (int s = 0; s < nseg && st == IEQ_OK; ++s) {
-      cudaMemcpyAsync(ck[s], at, sb, cudaMemcpyDeviceToDevice, c->stream);
+      cudaMemcpyAsync(ck[s], at, vb, cudaMemcpyDeviceToDevice, c->stream);
       if (s + 1 < nseg) st = advance(at, t0s[(size_t)s * K], K, false, at);
     }
     for (int s = nseg - 1; s >= 0 && st == IEQ_OK; --s) {
@@ -1216,12 +1235,12 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
     if (cudaStreamSynchronize(c->stream) != cudaSuccess && st == IEQ_OK) st = afail(c, IEQ_ERR_CUDA, "adjoint sweep");
     return st;
   }
-  void *ua = c->s.variable_u ? uw : (void *)u;   // u is rewritten only when it varies in time
-  const size_t ab = c->n_pad * sizeof(R4<double>);
+  void *cur = w[0], *b2 = w[1], *b3 = w[2], *cb = w[3];
+  void *ua = c->s.variable_u ? w[4] : (void *)u;   // u is rewritten only when it varies in time
   // one step through the reference kernels; keep (optional) receives the P states of the step
   auto step = [&](void *state, void *const *keep) -> ieq_status {
     if (ssp) {
-      if (keep) cudaMemcpyAsync(keep[0], state, ab, cudaMemcpyDeviceToDevice, c->stream);
+      if (keep) cudaMemcpyAsync(keep[0], state, vb, cudaMemcpyDeviceToDevice, c->stream);
       void *args[7] = {state, b2, b3, cb, ua, (void *)rho, d_time};
       const char *seq[] = {"calc_curlB_rho_1_3args", "calc_u_3_args", "SSPRK33_1", "SSPRK33_2a",
                            "calc_curlB_rho_2_3args", "calc_u_3_args", "SSPRK33_2b", "SSPRK33_3a",
@@ -1231,8 +1250,8 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
         if (!c->s.variable_u && std::strncmp(k, "calc_u", 6) == 0) continue;
         ieq_status s = adj_run_kernel(c, k, args, 7);
         if (s != IEQ_OK) return s;
-        if (std::strcmp(k, "SSPRK33_1") == 0 && keep) cudaMemcpyAsync(keep[1], b2, ab, cudaMemcpyDeviceToDevice, c->stream);
-        if (std::strcmp(k, "SSPRK33_2b") == 0 && keep) cudaMemcpyAsync(keep[2], b3, ab, cudaMemcpyDeviceToDevice, c->stream);
+        if (std::strcmp(k, "SSPRK33_1") == 0 && keep) cudaMemcpyAsync(keep[1], b2, vb, cudaMemcpyDeviceToDevice, c->stream);
+        if (std::strcmp(k, "SSPRK33_2b") == 0 && keep) cudaMemcpyAsync(keep[2], b3, vb, cudaMemcpyDeviceToDevice, c->stream);
       }
       return IEQ_OK;
     }
@@ -1241,7 +1260,7 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
     void *args[6] = {state, b2, cb, ua, (void *)rho, d_time};
     const std::string p = ck2n ? "CarpenterKennedy2N54_" : "ToulorgeDesmet2N84F_";
     for (int s = 0; s < S2; ++s) {
-      if (keep) cudaMemcpyAsync(keep[s], state, ab, cudaMemcpyDeviceToDevice, c->stream);
+      if (keep) cudaMemcpyAsync(keep[s], state, vb, cudaMemcpyDeviceToDevice, c->stream);
       ieq_status r;
       if (c->s.hall && (r = adj_run_kernel(c, "calc_curlB_rho_1_2args", args, 6)) != IEQ_OK) return r;
       if (c->s.variable_u && (r = adj_run_kernel(c, "calc_u_2_args", args, 6)) != IEQ_OK) return r;
@@ -1260,17 +1279,17 @@ ieq_status ieq_adjoint_steps(ieq_ctx *c, const void *b0, void *lambda, const voi
   // forward sweep: the checkpoints at the start of every segment (the last segment's steps are
   // run by the reverse sweep only)
   using F = AoS<double>;
-  VjpWork<F> vw = vjp_work<F>(c, vf);
-  cudaMemcpyAsync(cur, b0, ab, cudaMemcpyDeviceToDevice, c->stream);
+  VjpWork<F> vw = vjp_work<F>(c, use, vf);
+  cudaMemcpyAsync(cur, b0, vb, cudaMemcpyDeviceToDevice, c->stream);
   for (int s = 0; s < nseg && st == IEQ_OK; ++s) {
-    cudaMemcpyAsync(ck[s], cur, ab, cudaMemcpyDeviceToDevice, c->stream);
+    cudaMemcpyAsync(ck[s], cur, vb, cudaMemcpyDeviceToDevice, c->stream);
     if (s + 1 < nseg) st = advance(cur, t0s[(size_t)s * K], K, nullptr);
   }
   // reverse sweep: recompute a segment from its checkpoint keeping the stage states, then
   // apply the step adjoints backwards
   for (int s = nseg - 1; s >= 0 && st == IEQ_OK; --s) {
     const int n0 = s * K, n1 = std::min(num_steps, n0 + K);
-    cudaMemcpyAsync(cur, ck[s], ab, cudaMemcpyDeviceToDevice, c->stream);
+    cudaMemcpyAsync(cur, ck[s], vb, cudaMemcpyDeviceToDevice, c->stream);
     st = advance(cur, t0s[n0], n1 - n0, seg.data());
     if (st == IEQ_OK) st = reverse(MakeField<F>::of(c, lambda), MakeField<F>::of(c, u), rho, vw, n0, n1);
   }
