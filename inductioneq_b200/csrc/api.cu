@@ -109,6 +109,47 @@ dim3 grid3(int gx, int gy, int gz) {
 }
 
 // ------------------------------------------------------------------------- table upload
+// What the box kernels take of an operator at compile time must cover its rows: they sum ND (NU)
+// list entries a row and look for an x row's points within QX pairs of the node's own, where they
+// read zero beyond the box.
+template <int OP>
+bool rows_covered(const SbpOperator &op) {
+  const int c0 = (op.sw - 1) / 2, WH = op.w_hod, reach = std::max(c0, WH - 1);
+  for (int r = 0; r <= 2 * op.nb; ++r) {
+    int nd = 0, nu = 0;
+    for (int o = -reach; o <= reach; ++o) {
+      const double cD = o >= -c0 && o <= c0 ? op.D.at(r, o + c0) : 0.0;
+      double cH = 0.0;   // (upload_tables' dissipation row, without its sign)
+      for (int s = -WH + 1; s <= 0; ++s)
+        if (o - s >= 0 && o - s < WH) cH += (op.minv[r] * op.DHO.at(r, s + WH - 1)) * op.DHO.at(op.nb, o - s);
+      nd += cD != 0.0;
+      nu += cD != 0.0 || cH != 0.0;
+      if (cD == 0.0) continue;
+      // row r < nb is that of node r, row r > nb that of the node 2 nb - r from the end
+      if ((r < op.nb && r + o < 0) || (r > op.nb && o > 2 * op.nb - r)) return false;
+      // the first (k = 0) or the second node of its pair; either on the interior row
+      for (int k = 0; k < 2; ++k) {
+        if (r < op.nb && k != r % 2) continue;
+        if (r > op.nb && k == (2 * op.nb - r) % 2) continue;   // (an odd row's last pairs reach one further)
+        if (o < -2 * Op<OP>::QX - k || o > 2 * Op<OP>::QX + 1 - k) return false;
+      }
+    }
+    if (nd > Op<OP>::ND || nu > Op<OP>::NU) return false;
+  }
+  return op.nb == Op<OP>::NB && op.sw == Op<OP>::SW && WH == Op<OP>::WH;
+}
+bool rows_covered(const SbpOperator &op, int op_id) {
+  switch (op_id) {
+    case 0: return rows_covered<0>(op);
+    case 1: return rows_covered<1>(op);
+    case 2: return rows_covered<2>(op);
+    case 3: return rows_covered<3>(op);
+    case 4: return rows_covered<4>(op);
+    case 5: return rows_covered<5>(op);
+  }
+  return false;
+}
+
 template <typename R>
 ieq_status upload_tables(ieq_ctx *c) {
   const SbpOperator &op = c->op;
@@ -874,6 +915,11 @@ ieq_status ieq_create(ieq_ctx **out, const char *settings, const char *const *pa
     return IEQ_ERR_SETTINGS;
   }
   c->op_id = (c->s.order / 2 - 1) + (c->s.extended ? 3 : 0);
+  if (!rows_covered(c->op, c->op_id)) {
+    g_create_error = "the operator's rows exceed what the kernels were compiled for";
+    delete c;
+    return IEQ_ERR_SETTINGS;
+  }
   for (int a = 0; a < 3; ++a) {
     if (!c->s.periodic && c->s.nodes[a] < 2 * c->op.nb) {
       g_create_error = "NODES per direction must be at least 2*NUM_BOUNDS = " + std::to_string(2 * c->op.nb);
