@@ -77,6 +77,17 @@ def test_fused_calls_after_a_session(name, fails):
 
 
 @pytest.mark.parametrize("name", sorted(CASES))
+def test_an_end_without_a_session_changes_nothing(name):
+    a, ref = Run(name), Run(name)
+    a.failing_end()
+    with pytest.raises(IeqError):
+        a.end()
+    _same(a.advance(2), ref.advance(2))
+    a.ctx.close()
+    ref.ctx.close()
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
 @pytest.mark.parametrize("before", [False, True])
 def test_fused_calls_within_a_session(name, before):
     # `before`: the graphs exist when the session begins; else the call inside captures them
