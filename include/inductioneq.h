@@ -256,7 +256,8 @@ ieq_status ieq_batch_test_barrier(ieq_batch *batch, int extra_arrivals, long lon
  *     stage the next stage 0 starts a new step) on the context's stream;
  *   ieq_stages_field gives the state field `field` (0: b1, 1: b2, 2: b3 or db of the
  *     three-field schemes) as it stands after the last stage run: the device address of its x
- *     plane, the y and z planes following at component_stride elements (REAL); the fused path
+ *     plane (rows of NODES_X elements, without padding), the y and z planes following at
+ *     component_stride elements (REAL); the fused path
  *     alternates some fields between two buffers, so ask after every stage;
  *   ieq_stages_end copies the state back into the fields.
  * The fields may not be used by other calls on the context between begin and end. */

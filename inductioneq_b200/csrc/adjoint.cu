@@ -9,12 +9,13 @@
 //   step adjoints: lambda_n = (d b_{n+1} / d b_n)^T lambda_{n+1} from the stage states
 //   (SSPRK33; CarpenterKennedy2N54 and ToulorgeDesmet2N84F from the input of every stage),
 //   and the checkpointed sweep over many steps, whose forward passes run the fused stage
-//   kernels of the time stepping with the stage states written out per stage
+//   kernels of the time stepping from one kept stage state to the next
 // The transposes are written out per term (see the notes at k_vjp_pass1); D^T is applied as
 // a gather over the neighbours j = k + p with the coefficient of row(j) at offset -p.
 // The Hall outflow SAT (a switch on the sign of 0.5u - J) is differentiated away from the
 // switch (tv_a = 0); first-order dissipation is linear in b at fixed u; adaptive dissipation
-// (weights that depend on b through a square root and thresholds) has no adjoint.
+// (weights that depend on b through a square root and thresholds) is linearised at b, with
+// kappa's derivative inside its thresholds.
 #include <cmath>
 #include <cstring>
 #include <string>

@@ -184,7 +184,7 @@ bool parse_settings(const char *settings, const char *const *paths, int n_paths,
       s.hodp = std::atoi(val.c_str());
     } else if (key == "IEQ_CG_PASS_A") {
       if (val != "1" && val != "2") {
-        err = "IEQ_CG_PASS_A must be 1 (per-node gather) or 2 (2.5D z march)";
+        err = "IEQ_CG_PASS_A must be 1 (per-node gathers) or 2 (the cooperative loop)";
         return false;
       }
       s.cg_passes = std::atoi(val.c_str());

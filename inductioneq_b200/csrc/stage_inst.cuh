@@ -256,9 +256,11 @@ void launch_stage_col<IEQ_R, IEQ_OP>(const StageArgs<IEQ_R, SoA<IEQ_R>> &a, bool
     // divisions where none of its nodes needs them and the boundary rows where it has none, and
     // a compact warp meets fewer walls and fewer steep places than a row of 32.  From two and a
     // half rounds of blocks on (below, the lanes past rows that are not whole blocks weigh more:
-    // 50^3 0.9-1.05x).  CK2N54, 4 steps, rows of 32 / this, 4th order: Hall periodic 64^3 955 /
-    // 921 us, 112^3 5216 / 4147; rotation 64^3 1737 / 1433, 97^3 6114 / 4940, 112^3 9847 / 5400.
-    // FP32 keeps the rows (0.95-1.3x).
+    // 50^3 0.9-1.05x).  CK2N54, 4 steps, rows of 32 / this, 4th order: rotation 64^3 1458 / 1420
+    // us, 97^3 6527 / 4327, 112^3 7582 / 4651; Hall periodic 72^3 1.14x, 97^3 2557 / 2488, 112^3
+    // 3298 / 3243, but 64^3 595 / 643 and 96^3, 128^3 0.93 where the field is smooth (0.98-1.0
+    // where it is not): rows of whole warps have no idle lanes to gain.  FP32 keeps the rows
+    // (0.95-1.3x).
     const ColShape c = shaped(s1, a.m, 8, 8, 2);
     const dim3 gc = col_grid(c, a.m.nx, a.m.ny, a.m.nz, col_nodes(conv));
     if (2ll * gc.x * gc.y * gc.z > 5ll * kSms * foad_min_blocks<IEQ_OP>()) s1 = c;

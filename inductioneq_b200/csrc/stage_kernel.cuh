@@ -338,7 +338,8 @@ __device__ __forceinline__ bool ad_test(const V3<R> &b1, const V3<R> &u1, const 
 // which rounds alike.
 // (Hall periodic 64^3 with a current sheet, adaptive, 4th order, 20 stages: 2.37 ms with every
 // kappa evaluated from the table rows, 0.92 with the interior points loaded once and thresholds
-// from the host, 0.79 with the axes whose kappas are all zero summed in col_axis.)
+// from the host, 0.79 with the axes whose kappas are all zero summed in col_axis, 0.67 with that
+// and the block shape decided as now.)
 template <typename R, typename F, int OP, bool PER>
 __device__ V3<R> fo_ad_dissipation(const StageArgs<R, F> &a, const int ii[3], const int nn[3],
                                    const Idx<F> st[3], Idx<F> idx, V3<R> Bm, V3<R> um, int skip = 0) {

@@ -18,13 +18,15 @@
 //                   beside the pair kernels launched over the interior x range (XBAND)
 //
 // Each node's sums are formed term by term in the order of the one-node kernels
-// (k_curl_e, k_curl_e_hod, k_stage_col); the results agree with them up to the compiler's
-// choice of fused multiply-adds.
+// (k_curl_e, k_curl_e_hod, k_stage_col), and the stage kernels round what follows the sums alike
+// (stage_kernel.cuh), so they agree bit for bit.
 //
 // A launcher uses these kernels only where every vector load is aligned and stays in one row
-// (nx a multiple of K, each field's component stride a multiple of K, bases aligned to K
-// elements) and where they measured faster (stage_inst.cuh).  Without XBAND, x-boundary rows
-// of a box (and groups whose x window would leave the row) take the one-node code per node.
+// (nx a multiple of K or, on boxes, odd rows at a pitch of nx + 1; each field's component stride
+// a multiple of K, bases aligned to K elements) and where they measured faster (stage_inst.cuh).
+// Without XBAND, the warps of a box that hold the end of a row load the pairs around each node
+// and take every node's own row (col_x_pair_rows); k_stage_hall_x2 and k_curl_e_x2 run the
+// one-node code for the nodes of such warps.
 #pragma once
 #include "stage_col.cuh"
 

@@ -113,3 +113,19 @@ def test_adaptive_dissipation_does_not_depend_on_the_block_shape(order, extended
     for shape in ((8, 8, 2), (128, 1, 1), (1, 128, 1)):
         for got, want in zip(_whole(dict(c, col_block=shape), bh, uh), ref):
             np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("nodes", [(40, 14, 20), (97, 14, 20)])
+@pytest.mark.parametrize("order", [2, 4, 6])
+@pytest.mark.parametrize("make, kw", [(_rotation, {}), (_rotation, dict(uibj=SP, source=CE, ujbi=SP)),
+                                      (_rotation, dict(dissipation="FIRST_ORDER")), (_confined, {}),
+                                      (_hall, dict(dissipation="HIGH_ORDER"))])
+def test_stage_kernels_of_one_and_two_nodes_and_bands_round_alike(make, kw, order, nodes):
+    c = make(nodes, order, **kw)
+    if make is _confined:
+        c["dt"] = 1e-5
+    bh, uh = _start(c, 1e-2, 1.0)
+    ref = _whole(c, bh, uh)
+    for other in (dict(col_pairs=0), dict(xband=0), dict(xband=2)):
+        for got, want in zip(_whole(dict(c, **other), bh, uh), ref):
+            np.testing.assert_array_equal(got, want)
